@@ -32,7 +32,7 @@ struct BatchStepArgs {
     float4 *pos, *vel, *force, *spos, *svel;
     uint32_t *keys_a, *keys_b, *keys_c, *vals_a, *vals_b, *index, *bricks;
     uint16_t* nbr;
-    uint64_t* nbr_meta;
+    uint32_t* nbr_meta;
     uint2* table;
     uint32_t* scratch;
     uint32_t* err;
@@ -42,7 +42,7 @@ struct BatchStepArgs {
 // Dynamic shared memory of k_batch_step: each phase carves its own layout out of one buffer
 // (the force phase's is the largest).
 constexpr size_t STEP_SMEM = FORCE_SMEM;
-static_assert(DENSITY_SMEM + sizeof(SubListCounts) <= STEP_SMEM, "density phase layout");
+static_assert(density_smem(BRICK_WARPS - 1) <= STEP_SMEM, "density phase layout");
 static_assert(onesweep_smem_words(SORT_ITEMS) * 4 <= STEP_SMEM, "sort phase layout");
 static_assert(SORT_MAX_PASSES * SORT_RADIX * 4 <= STEP_SMEM, "hash phase layout");
 
@@ -55,8 +55,7 @@ static_assert(SORT_MAX_PASSES * SORT_RADIX * 4 <= STEP_SMEM, "hash phase layout"
 template <int ITEMS>
 __global__ void __launch_bounds__(BRICK_THREADS, 3) k_batch_step(BatchStepArgs a, KParams kp) {
     extern __shared__ float4 s_dyn[];
-    __shared__ BrickShared S[2];  // the brick phases use the two records in turn
-    __shared__ LaneMap L;
+    __shared__ BrickShared S;
     __shared__ uint32_t s_flag;
     uint32_t* words = reinterpret_cast<uint32_t*>(s_dyn);
     uint32_t* counters = a.scratch + SORT_USER_COUNTER_OFFSET / 4;
@@ -110,17 +109,16 @@ __global__ void __launch_bounds__(BRICK_THREADS, 3) k_batch_step(BatchStepArgs a
                           [&](uint32_t k) { return batch_brick_of(kp, k); }, tile);
     if (!gs.sync(&s_flag)) return;
 
-    SubListCounts& wcnt = *reinterpret_cast<SubListCounts*>(reinterpret_cast<char*>(s_dyn) + DENSITY_SMEM);
-    const bool ok = density_brick_run<3, true>(s_dyn, S, L, wcnt, a.spos, a.svel, a.table, a.bricks, counters, kp,
-                                               a.nbr, a.nbr_meta, a.err);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (ok) mbar_inval(reinterpret_cast<uint64_t*>(&S[0].bar));  // the force phase initialises it again
-        else gs.abort();
+    const bool ok = density_brick_run<3, true>(s_dyn, S, a.spos, a.svel, a.table, a.bricks, counters, kp, a.nbr,
+                                               a.nbr_meta, a.err);
+    if (!__syncthreads_and(ok)) {
+        if (threadIdx.x == 0) gs.abort();
+    } else {
+        brick_fini(S);  // the force phase initialises the barriers again
     }
     if (!gs.sync(&s_flag)) return;
 
-    force_brick_run<3, true, true, true>(s_dyn, S, L, a.spos, a.svel, a.index, a.pos, a.vel, a.force, a.table, a.bricks,
+    force_brick_run<3, true, true, true>(s_dyn, S, a.spos, a.svel, a.index, a.pos, a.vel, a.force, a.table, a.bricks,
                                          counters, kp, a.nbr, a.nbr_meta, a.err);
 }
 
@@ -138,7 +136,7 @@ struct gbsph_batch3d_s {
     uint32_t *keys_a = nullptr, *keys_b = nullptr, *keys_c = nullptr, *vals_a = nullptr, *vals_b = nullptr;
     uint32_t *index = nullptr, *bricks = nullptr;
     uint16_t* nbr = nullptr;
-    uint64_t* nbr_meta = nullptr;
+    uint32_t* nbr_meta = nullptr;
     uint2* table = nullptr;
     bool table_clean = false;
     void* scratch = nullptr;
@@ -215,16 +213,8 @@ KParams make_kp(const B* h) {
     k.kconst = p.kernelConstant;
     k.vlimit = p.velocitylimit;
     k.h2 = p.cellSize * p.cellSize;
-    // smallest float x with sqrtf(x) >= h
-    uint32_t lo = 0, hi = 0x7f800000u;
-    while (hi - lo > 1) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        float f;
-        std::memcpy(&f, &mid, 4);
-        if (std::sqrt(f) >= p.cellSize) hi = mid;
-        else lo = mid;
-    }
-    std::memcpy(&k.r2_thresh, &hi, 4);
+    k.r2_thresh = r2_threshold(p.cellSize);
+    k.v2_thresh = v2_threshold(p.velocitylimit);
     k.gravity = make_float4(p.gravity[0], p.gravity[1], p.gravity[2], p.gravity[3]);
     k.key_mode = GBSPH_KEY_LINEAR_GRID;
     k.dims = 3;
@@ -278,9 +268,9 @@ int enqueue_batch(B* h, const KParams& kp, cudaStream_t s) {
     k_bounds_batch<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, bcounters(h), h->err);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     h->table_clean = true;
-    k_density_brick<3, true><<<h->dens_blocks, BRICK_THREADS, DENSITY_SMEM, s>>>(h->spos, h->svel, h->table, h->bricks,
+    k_density_brick<3, true><<<h->dens_blocks, 32 * DENSITY_CONSUMERS + 32, DENSITY_SMEM, s>>>(h->spos, h->svel, h->table, h->bricks,
                                                                                 bcounters(h), kp, h->nbr, h->nbr_meta, h->err);
-    k_force_brick<3, true, true><<<h->force_blocks, BRICK_THREADS, FORCE_SMEM, s>>>(
+    k_force_brick<3, true, true><<<h->force_blocks, 32 * FORCE_CONSUMERS + 32, FORCE_SMEM, s>>>(
         h->spos, h->svel, h->index, h->pos, h->vel, h->force, h->table, h->bricks, bcounters(h), kp, h->nbr, h->nbr_meta,
         h->err);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
@@ -396,10 +386,10 @@ GBSPH_API int gbsph_batch3d_create(gbsph_batch3d_t* out) {
         const int sms = num_sms();
         if (cudaFuncSetAttribute(k_density_brick<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DENSITY_SMEM) ||
             cudaFuncSetAttribute(k_force_brick<3, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FORCE_SMEM) ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_brick<3, true>, BRICK_THREADS, DENSITY_SMEM))
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_brick<3, true>, 32 * DENSITY_CONSUMERS + 32, DENSITY_SMEM))
             rc = GBSPH_ERR_CUDA;
         h->dens_blocks = std::max(1, nb) * sms;
-        if (!rc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_brick<3, true, true>, BRICK_THREADS, FORCE_SMEM))
+        if (!rc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_brick<3, true, true>, 32 * FORCE_CONSUMERS + 32, FORCE_SMEM))
             rc = GBSPH_ERR_CUDA;
         h->force_blocks = std::max(1, nb) * sms;
         const void* steps[2] = {(const void*)k_batch_step<8>, (const void*)k_batch_step<16>};
@@ -479,7 +469,7 @@ GBSPH_API int gbsph_batch3d_set_scenes(gbsph_batch3d_t h, const gbsph_fluid3d_pa
     h->n = n;
     h->cells = cells;
     const size_t n4 = (n + 63) & ~size_t(63);
-    const size_t bytes = n4 * (5 * 16 + 7 * 4 + NBR_CAP * 2 + 8);
+    const size_t bytes = n4 * (5 * 16 + 7 * 4 + NBR_CAP * 2 + 4);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->block, bytes));
     GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->block, 0, bytes));
     char* p = (char*)h->block;
@@ -495,7 +485,7 @@ GBSPH_API int gbsph_batch3d_set_scenes(gbsph_batch3d_t h, const gbsph_fluid3d_pa
     }
     h->nbr = (uint16_t*)p;
     p += n4 * NBR_CAP * 2;
-    h->nbr_meta = (uint64_t*)p;
+    h->nbr_meta = (uint32_t*)p;
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->table, cells * sizeof(uint2)));
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, onesweep_scratch_bytes((uint32_t)n, SORT_MAX_PASSES)));
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->sdev, n_scenes * sizeof(SceneDev)));

@@ -1,5 +1,7 @@
 // common.cu -- status strings, log sink, version, device helpers shared by the library.
+#include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 
 #include "internal.h"
@@ -35,6 +37,41 @@ int num_sms() {
     if (cudaGetDevice(&dev) != cudaSuccess) return 148;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
     return sms > 0 ? sms : 148;
+}
+
+namespace {
+
+float bits_to_float(uint32_t b) {
+    float f;
+    std::memcpy(&f, &b, 4);
+    return f;
+}
+
+// Smallest float x in (+0, inf] for which pred(sqrtf(x)) holds, pred being false at 0, true at
+// infinity and monotone.
+template <class P>
+float least_square(P pred) {
+    uint32_t lo = 0, hi = 0x7f800000u;
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (pred(std::sqrt(bits_to_float(mid)))) hi = mid;
+        else lo = mid;
+    }
+    return bits_to_float(hi);
+}
+
+}  // namespace
+
+float r2_threshold(float h) {
+    if (!(h > 0.0f)) return 0.0f;  // nothing is nearer than h
+    if (std::isinf(h)) return h;   // every finite distance is
+    return least_square([h](float r) { return r >= h; });
+}
+
+float v2_threshold(float v) {
+    if (std::isnan(v) || v == INFINITY) return NAN;  // nothing exceeds it
+    if (v < 0.0f) return 0.0f;                        // everything does
+    return least_square([v](float r) { return r > v; });
 }
 
 }  // namespace gbsph

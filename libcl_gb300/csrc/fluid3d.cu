@@ -26,26 +26,6 @@ struct DevBuf {
     bool owned = false;
 };
 
-float bits_to_float(uint32_t b) {
-    float f;
-    std::memcpy(&f, &b, 4);
-    return f;
-}
-
-// Smallest float x >= 0 with sqrtf(x) >= h. sqrtf is correctly rounded and monotone, so for
-// every float r2 >= 0: (sqrtf(r2) < h) == (r2 < threshold).
-float r2_threshold(float h) {
-    if (!(h > 0.0f)) return 0.0f;  // nothing is nearer than h
-    if (std::isinf(h)) return h;   // every finite distance is
-    uint32_t lo = 0, hi = 0x7f800000u;  // sqrtf(+0) = 0 < h, sqrtf(inf) = inf >= h
-    while (hi - lo > 1) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        if (std::sqrt(bits_to_float(mid)) >= h) hi = mid;
-        else lo = mid;
-    }
-    return bits_to_float(hi);
-}
-
 int bits_for(uint64_t cells) {  // number of key bits to sort so that every key < cells is covered
     int b = 0;
     while (b < 32 && (1ull << b) < cells) b++;
@@ -67,7 +47,7 @@ struct gbsph_fluid3d_s {
     uint32_t *keys_a = nullptr, *keys_b = nullptr, *keys_c = nullptr;
     uint32_t *vals_a = nullptr, *vals_b = nullptr, *index = nullptr, *bricks = nullptr;
     uint16_t* nbr = nullptr;      // per particle NBR_CAP neighbour slots (density -> forces)
-    uint64_t* nbr_meta = nullptr;  // per particle: sub-list lengths, scan flag (bit 63)
+    uint32_t* nbr_meta = nullptr;  // per particle: list length or scan flag, cell x
     uint32_t* hash_tables = nullptr;  // cell start / end, REF_BUCKETS each
     uint32_t* xlist = nullptr;        // REFERENCE_HASH fused step: XL_CAP neighbours + count per particle
     size_t xlist_n = 0;
@@ -84,7 +64,11 @@ struct gbsph_fluid3d_s {
     uint32_t rec_n4 = 0;
     gbsph_fluid3d_hook_fn hook = nullptr;
     void* hook_user = nullptr;
-    int opt_fused = 1, opt_graph = 1, opt_bw = 16, opt_profile = 0;
+    int opt_fused = 1, opt_graph = 1, opt_profile = 0;
+    // cells per brick: wider ones are cut into units of 8 anyway and leave small scenes fewer
+    // bricks than SMs (65,536 particles: step 95 us at 16, 78 at 8, 77 at 4; from 262,144 on 8
+    // and 16 are alike and 4 is 10% slower)
+    int opt_bw = 8;
     cudaEvent_t ev[6] = {};
     bool ev_valid = false;
     int dens_blocks = 0, force_blocks = 0;
@@ -195,6 +179,7 @@ KParams make_kparams(const H* h) {
     k.vlimit = p.velocitylimit;
     k.h2 = p.cellSize * p.cellSize;
     k.r2_thresh = r2_threshold(p.cellSize);
+    k.v2_thresh = v2_threshold(p.velocitylimit);
     k.gravity = make_float4(p.gravity[0], p.gravity[1], p.gravity[2], p.gravity[3]);
     k.box_min = make_float4(p.boxMin[0], p.boxMin[1], p.boxMin[2], p.boxMin[3]);
     k.box_max = make_float4(p.boxMax[0], p.boxMax[1], p.boxMax[2], p.boxMax[3]);
@@ -250,7 +235,7 @@ void free_particle_arrays(H* h) {
 int alloc_particle_arrays(H* h, size_t n) {
     free_particle_arrays(h);
     const size_t n4 = (n + 63) & ~size_t(63);
-    const size_t bytes = n4 * (2 * 16 + 7 * 4 + NBR_CAP * 2 + 8);
+    const size_t bytes = n4 * (2 * 16 + 7 * 4 + NBR_CAP * 2 + 4);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->pblock, bytes));
     GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->pblock, 0, bytes));
     char* p = (char*)h->pblock;
@@ -265,7 +250,7 @@ int alloc_particle_arrays(H* h, size_t n) {
     }
     h->nbr = (uint16_t*)p;
     p += n4 * NBR_CAP * 2;
-    h->nbr_meta = (uint64_t*)p;
+    h->nbr_meta = (uint32_t*)p;
     h->scratch_bytes = onesweep_scratch_bytes((uint32_t)n, SORT_MAX_PASSES);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, h->scratch_bytes));
     GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->scratch, 0, h->scratch_bytes));
@@ -429,7 +414,7 @@ int st_forces_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false)
 
 int st_density_brick(H* h, const KParams& kp, cudaStream_t s) {
     auto launch = [&](auto kern) {
-        kern<<<h->dens_blocks, BRICK_THREADS, DENSITY_SMEM, s>>>(h->spos, h->svel, h->table, h->bricks, counters(h), kp,
+        kern<<<h->dens_blocks, 32 * DENSITY_CONSUMERS + 32, DENSITY_SMEM, s>>>(h->spos, h->svel, h->table, h->bricks, counters(h), kp,
                                                                  h->nbr, h->nbr_meta, h->err);
     };
     if (kp.dims == 2) launch(k_density_brick<2, false>);
@@ -440,7 +425,7 @@ int st_density_brick(H* h, const KParams& kp, cudaStream_t s) {
 
 int st_force_brick(H* h, const KParams& kp, cudaStream_t s, bool fused) {
     auto launch = [&](auto kern) {
-        kern<<<h->force_blocks, BRICK_THREADS, FORCE_SMEM, s>>>(h->spos, h->svel, h->index, P4(h, 0), P4(h, 1), P4(h, 2),
+        kern<<<h->force_blocks, 32 * FORCE_CONSUMERS + 32, FORCE_SMEM, s>>>(h->spos, h->svel, h->index, P4(h, 0), P4(h, 1), P4(h, 2),
                                                                 h->table, h->bricks, counters(h), kp, h->nbr,
                                                                 h->nbr_meta, h->err);
     };
@@ -614,9 +599,9 @@ int setup_kernels(H* h) {
     GBSPH_CUDA_TRY(&h->last_error, cudaFuncSetAttribute(k_force_brick<3, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
     GBSPH_CUDA_TRY(&h->last_error, cudaFuncSetAttribute(k_force_brick<2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
     GBSPH_CUDA_TRY(&h->last_error, cudaFuncSetAttribute(k_force_brick<2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-    GBSPH_CUDA_TRY(&h->last_error, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_brick<3, false>, BRICK_THREADS, DENSITY_SMEM));
+    GBSPH_CUDA_TRY(&h->last_error, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_brick<3, false>, 32 * DENSITY_CONSUMERS + 32, DENSITY_SMEM));
     h->dens_blocks = std::max(1, nb) * sms;
-    GBSPH_CUDA_TRY(&h->last_error, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_brick<3, true, false>, BRICK_THREADS, FORCE_SMEM));
+    GBSPH_CUDA_TRY(&h->last_error, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_brick<3, true, false>, 32 * FORCE_CONSUMERS + 32, FORCE_SMEM));
     h->force_blocks = std::max(1, nb) * sms;
     return GBSPH_OK;
 }

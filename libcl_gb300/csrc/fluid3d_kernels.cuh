@@ -7,12 +7,11 @@
 //     27 (or 9) neighbour cells in the reference's z, y, x order. In REFERENCE_HASH mode that
 //     includes visiting a bucket twice when two neighbour cells hash to it. They reproduce the
 //     FP32 restatement bit for bit and serve the parity modes.
-//   * "brick" kernels (LINEAR_GRID only) are the fast path. A persistent CTA takes a brick of
-//     W cells along x, loads the cell table of the 9 (or 3) neighbour rows, copies those rows'
-//     contiguous particle ranges into shared memory with cp.async.bulk on one mbarrier, and
-//     each warp evaluates one target cell: lanes = (target, candidate stride) so candidate
-//     loads are shared-memory broadcasts; partial sums are combined with shuffles. FMA and
-//     rsqrt are used, so results agree with the restatement within FP32 tolerance.
+//   * "brick" kernels (LINEAR_GRID only) are the fast path: persistent CTAs stage the particles
+//     around W cells along x in shared memory, a producer warp ahead of the others, and each
+//     warp takes eight pairs of targets; density leaves neighbour lists for forces. FMA and the
+//     approximate reciprocals are used, so results agree with the restatement within FP32
+//     tolerance.
 #pragma once
 
 #include "device.cuh"
@@ -22,10 +21,9 @@ namespace gbsph {
 
 constexpr uint32_t EMPTY = 0xFFFFFFFFu;
 constexpr uint32_t REF_BUCKETS = 262144u;  // BUCKETS, libCL/phys/oclFluid3D.cl:32
-constexpr int BRICK_THREADS = 256;
+constexpr int BRICK_THREADS = 256;  // of the batch's persistent step, whose other phases it fits
 constexpr int BRICK_WARPS = BRICK_THREADS / 32;
 constexpr int BRICK_W_MAX = 16;
-constexpr int BRICK_SLOTS = BRICK_W_MAX + 2;
 
 // One scene of a batch (LINEAR_GRID): its particles, cells and bricks are consecutive ranges
 // of the batch's arrays, and its gas constant, viscosity, box and grid are its own.
@@ -41,6 +39,7 @@ struct KParams {
     float dt, radius, h, mass, p0, rho0, stiff, cvisc, cpress, kconst, vlimit;
     float h2;         // h*h
     float r2_thresh;  // smallest float x with sqrtf(x) >= h, so (sqrtf(r2) < h) == (r2 < r2_thresh)
+    float v2_thresh;  // smallest float x with sqrtf(x) > vlimit (NaN: none), so (sqrtf(f2) > vlimit) == (f2 >= v2_thresh)
     float4 gravity, box_min, box_max, origin;
     int nx, ny, nz;
     int key_mode, dims;
@@ -561,779 +560,748 @@ static __global__ void k_post_fused(const float4* __restrict__ spos, const float
 }
 
 // ---- brick (fast, LINEAR_GRID) neighbour kernels ---------------------------------------------
+//
+// Both passes run as persistent CTAs over the occupied bricks. The last warp of a CTA produces: it
+// takes bricks from a queue, reads the cell ranges of the brick's neighbour rows, cuts the brick
+// into units of at most BRICK_UNIT target cells whose candidates fit the staging, and copies
+// each unit's candidates into one of two buffers. The other warps consume the units: while they
+// compute one, the other buffer is filled, so that the chain queue -> brick -> cell table ->
+// particles does not stand in line with the arithmetic. A unit is handed over through two
+// mbarriers per buffer (full: filled; empty: every consumer is done).
+//
+// The candidates are staged by columns: all cells (y, z = -1..1) of column x, then those of
+// column x + 1. The 27 (or 9) cells around a target are then one contiguous window of the
+// staging, the same for every target of a cell, and a candidate's place in its target's window
+// depends neither on the brick nor on the unit; neighbour lists hold such places, so that the
+// two passes need not cut the bricks alike. Staged by rows, the window is nine short pieces,
+// and the row loop around them cost as many instructions as the candidates themselves.
+//
+// A cell's particles are taken in pairs (two consecutive sorted particles; the last of an odd
+// cell alone), numbered through the unit, and both passes give four lanes to a pair and eight
+// pairs to a warp whatever cells they are in. A lane holds both targets, so a candidate read
+// from shared memory serves two, and the two share one neighbour list: the candidates in range
+// of either (about 46 entries where each has 34).
+//
+// 1,048,576 particles at the start of the block collapse (8 per cell, 216 candidates and 34 in
+// range each): density 137 us (213 us with the rows staged by bulk copies, a warp per cell and
+// lists appended per candidate), forces 150 us (184 us with two lanes per target and the lists
+// staged). Density is bound by instruction issue (79% of cycles; 63 of the 137 us are the
+// candidate loop at 21 instructions for 64 pairs, 20 the lists, 16 the staging), forces by issue
+// and shared-memory wavefronts (55% and 64%).
+// Tried: a bulk copy per cell instead of the 16-byte asynchronous copies (170 / 260 us: the
+// small copies queue), two producers, one per buffer (139 / 178), 3 to 7 consumers at 3 to 6
+// CTAs per SM (density 133-137, forces 150-172).
+constexpr int DENSITY_CONSUMERS = 4, FORCE_CONSUMERS = 5;      // warps beside the producer
+constexpr int DENSITY_CTAS = 5, FORCE_CTAS = 4;                // per SM, by shared memory
+constexpr int BRICK_UNIT = 8;                     // target cells per unit at most
+constexpr int BRICK_CELLS = (BRICK_UNIT + 2) * 9;  // staged cells of a unit
+// Staged candidates per unit (8 lattice cells with their neighbours are 720). Both may cut a
+// brick differently; a target whose window alone exceeds the cap reads global memory.
+constexpr uint32_t DENSITY_CAP = 1024, FORCE_CAP = 768;
+constexpr uint32_t NBR_CAP = 64;                  // neighbour list entries per particle (a pair: twice that)
+constexpr uint32_t TASK_PAIRS = 8;                // pairs a warp takes at once, four lanes each
+constexpr uint32_t LIST_AHEAD = 6;                // 8-entry chunks of a list the force pass loads at once
+constexpr uint32_t LIST_STRIDE = 2 * NBR_CAP + 8;  // halves between a warp's lists (16-byte rows)
+constexpr uint32_t NBR_SCAN = 0xFFFFFFFFu;        // nbr_meta: no list, the force pass scans
+constexpr uint32_t REC_SCAN = 0xFFFFFFFFu;        // rec_cnt: no recorded list for this particle
+
+// One staged unit.
+struct BrickUnit {
+    uint32_t off[BRICK_CELLS + 1];  // staged place of cell (column * R + row); the last entry: all candidates
+    uint2 cell[BRICK_CELLS];        // the cell's first sorted index; staged place | count << 16 (staged units)
+    uint32_t pair[BRICK_UNIT];      // pairs before target cell c (beyond the last cell: npair)
+    uint32_t npair;
+    int ncell;                      // target cells (columns 1 .. ncell); 0: no more units
+    int staged;                     // 0: the candidates did not fit, read them from global memory
+    float stiff, cvisc;             // the scene's parameters (they differ within a batch)
+    float4 box_min, box_max;
+};
 
 struct BrickShared {
-    uint32_t off[9][BRICK_SLOTS + 1];  // lower bounds of each cell inside the row's range
-    uint32_t lo[9];                    // first sorted index of the row's range
-    uint32_t rcnt[9];                  // candidates of the row
-    uint32_t base[9];                  // offset of the row in the staging buffer
-    uint32_t brick;                    // index into the occupied-brick list
-    // the brick's scene: grid, cell-table offset and the parameters that vary per scene
-    int nx, ny, nz, bxn;
-    uint32_t cell_off, lbrick;  // lbrick: the brick's id within its scene
-    float stiff, cvisc;
-    float4 box_min, box_max;
-    unsigned long long bar;
+    BrickUnit unit[2];
+    unsigned long long full[2], empty[2];
 };
 
-// Loads the brick's scene, geometry and neighbour-row ranges into S. A single scene takes its
-// grid and parameters from kp; in a batch (BATCH) the brick id is global and its scene is
-// found in kp.scenes. Returns the brick's first cell x and cell count through x0/ncell.
-template <int DIMS, bool BATCH>
-__device__ __forceinline__ void brick_setup(BrickShared& S, const KParams& kp, uint32_t bid,
-                                            const uint2* __restrict__ table, uint32_t* err, int& x0,
-                                            int& ncell) {
-    constexpr int R = DIMS == 3 ? 9 : 3;
-    const int W = kp.bw;
-    const int t = threadIdx.x;
-    // a single scene's grid comes from kp (no barrier needed); a batch's from its scene
-    // table, through shared memory. The barrier after the table loads publishes S's scene
-    // fields before any warp reads them.
-    if (t == 0) {
-        if (BATCH) {
-            const int sc = scene_of<2>(kp.scenes, kp.n_scenes, bid);
-            const SceneDev& d = kp.scenes[sc];
-            S.nx = d.nx;
-            S.ny = d.ny;
-            S.nz = d.nz;
-            S.bxn = d.bxn;
-            S.cell_off = d.cell_off;
-            S.stiff = d.stiff;
-            S.cvisc = d.cvisc;
-            S.box_min = d.box_min;
-            S.box_max = d.box_max;
-            S.lbrick = bid - d.brick_off;
-        } else {
-            S.nx = kp.nx;
-            S.ny = kp.ny;
-            S.nz = kp.nz;
-            S.bxn = kp.bxn;
-            S.cell_off = 0;
-            S.stiff = kp.stiff;
-            S.cvisc = kp.cvisc;
-            S.box_min = kp.box_min;
-            S.box_max = kp.box_max;
-            S.lbrick = bid;
-        }
-    }
-    if (BATCH) __syncthreads();
-    const uint32_t lb = BATCH ? S.lbrick : bid;
-    const int nx = BATCH ? S.nx : kp.nx, ny = BATCH ? S.ny : kp.ny, nz = BATCH ? S.nz : kp.nz;
-    const uint32_t bxn = BATCH ? (uint32_t)S.bxn : (uint32_t)kp.bxn;
-    const int bx = (int)(lb % bxn);
-    const uint32_t yz = lb / bxn;
-    const int y = (int)(yz % (uint32_t)ny);
-    const int z = (int)(yz / (uint32_t)ny);
-    x0 = bx * W;
-    ncell = min(W, nx - x0);
-    const uint2* tab = BATCH ? table + S.cell_off : table;
-    // a warp per row (warp w takes rows w, w + BRICK_WARPS, ...): lane c reads the range of the
-    // row's column c (cell x0 - 1 + c), a warp scan of the counts gives the columns' offsets
-    // inside the row's range, and the first non-empty column its start
-    const int lane = t & 31;
-    for (int r = t >> 5; r < R; r += BRICK_WARPS) {
-        const int cy = y + (r % 3) - 1;
-        const int cz = DIMS == 3 ? z + (r / 3) - 1 : 0;
-        const int cx = x0 - 1 + lane;
-        uint32_t cnt = 0, st = 0;
-        if (lane < W + 2 && cx >= 0 && cx < nx && cy >= 0 && cy < ny && cz >= 0 && cz < nz) {
-            const uint2 e = tab[(uint32_t)cx + (uint32_t)nx * ((uint32_t)cy + (uint32_t)ny * (uint32_t)cz)];
-            if (e.x != EMPTY) {
-                cnt = e.y - e.x;
-                st = e.x;
-            }
-        }
-        uint32_t inc = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-        const uint32_t nonempty = __ballot_sync(0xffffffffu, cnt != 0u);
-        const uint32_t lo = nonempty ? __shfl_sync(0xffffffffu, st, __ffs(nonempty) - 1) : 0u;
-        const bool bad = (uint64_t)lo + total > kp.n;  // inconsistent table: report, use an empty row
-        // column W + 2 (and beyond) has no count, so its exclusive offset is the row's total
-        if (lane <= W + 2) S.off[r][lane] = bad ? 0u : inc - cnt;
-        if (lane == 0) {
-            S.lo[r] = bad ? 0u : lo;
-            S.rcnt[r] = bad ? 0u : total;
-            if (bad) atomicOr(err, DEV_ERR_KEY_RANGE);
-        }
-    }
-    __syncthreads();
-}
-
-// Warp 0: the rows' bases in the staging buffer (a scan of their counts), then, if the brick
-// fits, lane 0 arms the mbarrier `bar` with the byte count and lane r copies row r. No barrier:
-// the other warps learn whether the brick is staged from brick_total and wait on `bar`
-// (brick_wait's barrier then publishes the bases).
-template <int DIMS, int NARR>
-__device__ __forceinline__ void brick_stage(BrickShared& S, float4* s_buf, uint32_t cap,
-                                            const float4* __restrict__ a0, const float4* __restrict__ a1,
-                                            uint64_t* bar) {
-    constexpr int R = DIMS == 3 ? 9 : 3;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        const uint32_t rc = lane < R ? S.rcnt[lane] : 0u;
-        uint32_t inc = rc;
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        const uint32_t base = inc - rc, total = __shfl_sync(0xffffffffu, inc, R - 1);
-        if (lane < R) S.base[lane] = base;
-        if (total <= cap && total > 0) {
-            if (lane == 0) mbar_arrive_expect_tx(bar, total * 16u * NARR);
-            __syncwarp();
-            if (lane < R && rc) {
-                // this lane's generic-proxy accesses (shared memory, and global memory that an
-                // earlier phase of a persistent kernel wrote) before its bulk copies
-                fence_proxy_async_smem();
-                fence_proxy_async_global();
-                bulk_g2s(s_buf + base, a0 + S.lo[lane], rc * 16u, bar);
-                if (NARR > 1) bulk_g2s(s_buf + cap + base, a1 + S.lo[lane], rc * 16u, bar);
-            }
-        }
-    }
-}
-
-// Candidates the brick stages: the sum of its rows' counts (known to every thread after the
-// set-up's barrier).
-template <int DIMS>
-__device__ __forceinline__ uint32_t brick_total(const BrickShared& S) {
-    constexpr int R = DIMS == 3 ? 9 : 3;
-    uint32_t a = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) a += S.rcnt[r];
-    return a;
-}
-
-// Waits for the staged copies (every thread), then a barrier. Returns false to every thread
-// if any thread's wait hit its limit, after draining the copies still in flight (bounded).
-__device__ __forceinline__ bool brick_wait(uint64_t* bar, uint32_t& phase, uint32_t* err) {
-    bool ok = mbar_wait_bounded(bar, phase);
-    if (!ok) atomicOr(err, DEV_ERR_MBAR_TIMEOUT);
-    ok = __syncthreads_and(ok);
-    phase ^= 1u;
-    if (!ok && threadIdx.x == 0) {
-        // drain the copies still in flight (bounded) before this CTA's shared memory goes away
-        mbar_wait_bounded(bar, phase ^ 1u);
-    }
-    return ok;
-}
-
-// Tree reduction over the Q lanes {q*tg + ti} that share a target.
-__device__ __forceinline__ float reduce_q(float v, uint32_t q, uint32_t Q, uint32_t tg) {
-    for (uint32_t s = 1; s < Q; s <<= 1) {
-        const float o = __shfl_down_sync(0xffffffffu, v, s * tg);
-        if ((q & (2 * s - 1)) == 0 && q + s < Q) v += o;
-    }
-    return v;
-}
-
-// Staged candidates per brick. The density and force kernels use the same value so that they
-// stage (or fall back for) exactly the same bricks: the neighbour lists the density kernel
-// records are indices into that staging.
-constexpr uint32_t BRICK_CAP = 1536;
-constexpr uint32_t NBR_CAP = 64;         // neighbour slots per particle (uint16), split over the Q lanes
-constexpr uint32_t WLIST_STRIDE = NBR_CAP + 8;  // shared-memory stride per target (halves; 16-byte rows)
-constexpr uint32_t LIST_STAGE_MAX = 160;        // targets per brick whose lists the force kernel stages
-constexpr uint32_t GROUP_MAX = 16;              // targets a warp takes at once (both passes)
-constexpr uint32_t NBR_SUBLISTS = 8;            // at most 8 lanes (sub-lists) per target
-constexpr uint64_t NBR_SCAN = 1ull << 63;       // nbr_meta: the force pass scans for this target
-constexpr uint32_t REC_SCAN = 0xFFFFFFFFu;      // rec_cnt: no recorded list for this particle
-
-
-// Dynamic shared memory of the brick kernels.
-constexpr size_t DENSITY_SMEM = (size_t)BRICK_CAP * 16 + (size_t)BRICK_WARPS * GROUP_MAX * WLIST_STRIDE * 2;
-// force: staged positions and velocities, then the lists, list lengths and permutation
-// entries of up to LIST_STAGE_MAX targets (the last two rounded out to 16-byte copies)
-constexpr size_t FORCE_LIST_BYTES = (size_t)LIST_STAGE_MAX * NBR_CAP * 2;
-constexpr size_t FORCE_META_BYTES = (size_t)(LIST_STAGE_MAX + 2) * 8;
-constexpr size_t FORCE_INDEX_BYTES = (size_t)(LIST_STAGE_MAX + 4) * 4;
-constexpr size_t FORCE_SMEM = (size_t)BRICK_CAP * 32 + FORCE_LIST_BYTES + FORCE_META_BYTES + FORCE_INDEX_BYTES;
-
-// Slots of each lane's sub-list when Q lanes share a target: sub-list q holds slots
-// [q * sub, (q + 1) * sub) of the target's NBR_CAP slots.
-__device__ __forceinline__ uint32_t nbr_sub(uint32_t Q) { return NBR_CAP / Q; }
-
-// Lane layout of a group of tg targets (1 <= tg <= GROUP_MAX) on a warp: lane = q * tg + ti
-// serves target ti with stride q of Q = min(32 / tg, NBR_SUBLISTS) (lanes with q >= Q idle).
-// tq packs ti | q << 8;
-// info packs Q | nbr_sub(Q) << 8; group << ti is the mask of the lanes serving target ti.
-// Both neighbour passes use it, so the density pass's sub-lists are the force pass's.
-struct LaneMap {
-    uint16_t tq[GROUP_MAX + 1][32];
-    uint32_t info[GROUP_MAX + 1];
-    uint32_t group[GROUP_MAX + 1];
+// What a lane knows of its pair.
+struct PairTask {
+    bool live, two;         // a pair of this unit (else a stand-in, nothing of which is stored); it has two targets
+    uint32_t gi;            // sorted index of the first target
+    uint32_t self;          // its staged place
+    uint32_t lo, len;       // the window's first staged place and its candidates
+    int c;                  // target cell: column c + 1
 };
 
-__device__ __forceinline__ void lane_map_init(LaneMap& L) {
-    for (uint32_t i = threadIdx.x; i < (GROUP_MAX + 1) * 32; i += blockDim.x) {
-        const uint32_t tg = i / 32, lane = i % 32;
-        if (tg == 0) {
-            L.tq[0][lane] = 0;
-            if (lane == 0) L.info[0] = L.group[0] = 0;
-            continue;
-        }
-        const uint32_t Q = min(32 / tg, NBR_SUBLISTS);
-        L.tq[tg][lane] = (uint16_t)((lane % tg) | ((lane / tg) << 8));
-        if (lane == 0) {
-            uint32_t m = 0;
-            for (uint32_t k = 0; k < Q; ++k) m |= 1u << (k * tg);
-            L.info[tg] = Q | (nbr_sub(Q) << 8);
-            L.group[tg] = m;
-        }
-    }
+template <int R, int RC>
+__device__ __forceinline__ PairTask pair_task(const BrickUnit& U, uint32_t p) {
+    PairTask t;
+    t.live = p < U.npair;
+    p = min(p, U.npair - 1u);
+    t.c = 0;
+#pragma unroll
+    for (int k = 1; k < BRICK_UNIT; ++k) t.c += p >= U.pair[k] ? 1 : 0;
+    const uint32_t k = 2u * (p - U.pair[t.c]), i = (uint32_t)((t.c + 1) * R + RC), o = U.off[i];
+    t.two = k + 1u < U.off[i + 1] - o;
+    t.gi = U.cell[i].x + k;
+    t.self = o + k;
+    t.lo = U.off[t.c * R];
+    t.len = U.off[(t.c + 3) * R] - t.lo;
+    return t;
 }
 
-// Density + pressure for every particle of the occupied bricks (persistent CTAs).
-// Writes sorted position .w = density and sorted velocity .w = pressure, as
-// clCalculateDensity does (libCL/phys/oclFluid3D.cl:189-199). A warp takes a target cell and
-// up to GROUP_MAX of its particles at a time; lanes (target ti, stride q) walk the 9 (or 3)
-// neighbour rows of the cell (3 consecutive cells each, contiguous in the staging buffer),
-// lane q taking candidates q, q + Q, ... of every row, so candidate loads are shared-memory
-// broadcasts. Every target also meets itself (r^2 = 0, term h^6, count 1); that term is
-// removed after the sum instead of testing the index of every candidate. Each lane records
-// its in-range candidates (the target itself included) as staged indices in its own
-// sub-list of nbr[gi][NBR_CAP] (in candidate order); the lists' lengths are the counts the
-// reference's count > 2 test uses and go to nbr_meta[gi] (one byte per sub-list), or
-// nbr_meta[gi] = NBR_SCAN when a sub-list overflowed or the brick could not be staged.
-typedef uint8_t SubListCounts[BRICK_WARPS][GROUP_MAX][NBR_SUBLISTS];  // sub-list lengths per warp group
+// Dynamic shared memory: two staging buffers, then (density) each consumer's neighbour lists.
+constexpr size_t density_smem(int consumers) {
+    return 2 * (size_t)DENSITY_CAP * 16 + (size_t)consumers * TASK_PAIRS * LIST_STRIDE * 2;
+}
+constexpr size_t DENSITY_SMEM = density_smem(DENSITY_CONSUMERS);
+constexpr size_t FORCE_SMEM = 2 * (size_t)FORCE_CAP * 32;
 
-// The body of k_density_brick, on shared memory the caller provides: s_buf (DENSITY_SMEM
-// bytes), S2 (two brick records, used in turn, so that a warp may start the next brick's
-// set-up while others still compute this one), L and wcnt. The batched step's persistent
-// kernel runs it as one of its phases. Returns false if a bulk-copy wait gave up (the CTA left
-// the loop).
-template <int DIMS, bool BATCH>
-__device__ __forceinline__ bool density_brick_run(float4* s_buf, BrickShared* S2, LaneMap& L, SubListCounts& wcnt,
-                                                  float4* __restrict__ spos, float4* __restrict__ svel,
-                                                  const uint2* __restrict__ table, const uint32_t* __restrict__ bricks,
-                                                  uint32_t* counters, const KParams& kp, uint16_t* __restrict__ nbr,
-                                                  uint64_t* __restrict__ nbr_meta, uint32_t* err) {
-    constexpr int R = DIMS == 3 ? 9 : 3;
-    constexpr int RC = DIMS == 3 ? 4 : 1;  // the brick's own row
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    uint16_t* wlist = reinterpret_cast<uint16_t*>(s_buf + BRICK_CAP) + warp * GROUP_MAX * WLIST_STRIDE;
-    lane_map_init(L);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(&S2[0].bar);
-    if (t == 0) {
-        mbar_init(bar, 1);
+__device__ __forceinline__ void brick_init(BrickShared& S) {
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            // the producer's lanes arrive twice each: once for their own writes, once when their
+            // asynchronous copies have landed
+            mbar_init(reinterpret_cast<uint64_t*>(&S.full[i]), 64);
+            mbar_init(reinterpret_cast<uint64_t*>(&S.empty[i]), blockDim.x / 32u - 1u);
+        }
         fence_mbar_init();
     }
-    uint32_t phase = 0;
-    const uint32_t n_bricks = __ldcg(counters);  // written by the bounds pass (an earlier kernel or phase)
-    const float h2 = kp.h2, thr = kp.r2_thresh;
-    const uint32_t buf_a = smem_addr(s_buf);
-    // Brick k uses record S2[k & 1]. Its id was fetched at the start of brick k - 1 and is read
-    // after that brick's barriers; the set-up's barrier of brick k (all warps are done with
-    // brick k - 1) comes before the copies into the staging buffer.
-    if (t == 0) S2[0].brick = atomicAdd(&counters[1], 1u);
     __syncthreads();
-    for (uint32_t it = 0;; it ^= 1u) {
-        BrickShared& S = S2[it];
-        const uint32_t b = S.brick;
-        if (b >= n_bricks) break;
-        if (t == 0) S2[it ^ 1u].brick = atomicAdd(&counters[1], 1u);
-        int x0, ncell;
-        brick_setup<DIMS, BATCH>(S, kp, bricks[b], table, err, x0, ncell);
-        brick_stage<DIMS, 1>(S, s_buf, BRICK_CAP, spos, nullptr, bar);
-        const uint32_t total = brick_total<DIMS>(S);
-        const bool staged = total <= BRICK_CAP && total > 0;
-        if (staged && !brick_wait(bar, phase, err)) return false;
-        for (int c = warp; c < ncell; c += BRICK_WARPS) {
-            const uint32_t t0 = S.off[RC][c + 1], nt = S.off[RC][c + 2] - t0;
-            for (uint32_t g0 = 0; g0 < nt; g0 += GROUP_MAX) {
-                const uint32_t tg = min(GROUP_MAX, nt - g0);
-                const uint32_t e = L.tq[tg][lane], f = L.info[tg];
-                const uint32_t ti = e & 0xFFu, q = e >> 8, Q = f & 0xFFu, sub = f >> 8;
-                const bool active = q < Q;
-                const uint32_t tl = t0 + g0 + ti;
-                const uint32_t gi = S.lo[RC] + tl;
-                const float4 pi = staged ? s_buf[S.base[RC] + tl] : spos[gi];
-                uint16_t* my = wlist + ti * WLIST_STRIDE + q * sub;
-                float acc = 0.0f;
-                uint32_t nk = 0;  // in-range candidates of this lane (the target itself included)
-                if (active && staged) {
-                    // 32-bit shared-memory addresses stepped per candidate: the candidate's
-                    // position (16 bytes) and this lane's next list slot, wa, which stops one
-                    // slot past the sub-list (the next lane's first slot, or the row's padding).
-                    // A lane that gets there has overflowed (nk = sub): its target is then
-                    // scanned by the force pass and none of its sub-lists is read.
-                    const uint32_t my_a = smem_addr(my), w_end = my_a + 2u * sub, step = Q * 16u;
-                    uint32_t wa = my_a;
-#pragma unroll 1
-                    for (int r = 0; r < R; ++r) {
-                        const uint32_t lo = S.off[r][c], len = S.off[r][c + 3] - lo;
-                        uint32_t v = S.base[r] + lo + q;  // staged index of the candidate
-                        uint32_t a = buf_a + v * 16u;
-                        const uint32_t a_end = buf_a + (S.base[r] + lo + len) * 16u;
-#pragma unroll 4
-                        for (; a < a_end; a += step, v += Q) {
-                            const float4 pj = lds_f4(a);
-                            const float dx = pi.x - pj.x, dy = pi.y - pj.y;
-                            float r2 = fmaf(dy, dy, dx * dx);
-                            if (DIMS == 3) {
-                                const float dz = pi.z - pj.z;
-                                r2 = fmaf(dz, dz, r2);
-                            }
-                            const bool in = r2 < thr;
-                            const float tt = in ? h2 - r2 : 0.0f;
-                            acc = fmaf(tt * tt, tt, acc);
-                            // branch-free append: the slot after the last real entry is
-                            // overwritten by the next candidate. The target and coincident
-                            // particles (r^2 = 0) are listed; the force pass skips them.
-                            sts_u16(wa, v);
-                            wa = min(wa + (in ? 2u : 0u), w_end);
-                        }
-                    }
-                    nk = (wa - my_a) >> 1;  // at most sub: an overflowed lane counts sub
-                } else if (active) {  // unstaged brick: candidates from global memory, no lists
-#pragma unroll 1
-                    for (int r = 0; r < R; ++r) {
-                        const uint32_t lo = S.off[r][c], len = S.off[r][c + 3] - lo;
-                        const float4* rp = spos + S.lo[r] + lo;
-                        for (uint32_t k = q; k < len; k += Q) {
-                            const float4 pj = rp[k];
-                            const float dx = pi.x - pj.x, dy = pi.y - pj.y;
-                            float r2 = fmaf(dy, dy, dx * dx);
-                            if (DIMS == 3) {
-                                const float dz = pi.z - pj.z;
-                                r2 = fmaf(dz, dz, r2);
-                            }
-                            const bool in = r2 < thr;
-                            const float tt = in ? h2 - r2 : 0.0f;
-                            acc = fmaf(tt * tt, tt, acc);
-                            nk += in ? 1u : 0u;
-                        }
-                    }
-                }
-                const bool ovf = !staged || nk >= sub;
-                if (kp.rec_nbr) {
-                    // recording (an adjoint's recomputation): the target's sub-lists, concatenated
-                    // in q order, as sorted indices; lane q writes its own entries after those
-                    // of the lanes q' < q of its target
-                    uint32_t before = active ? nk : 0u;
-#pragma unroll
-                    for (uint32_t st = 1; st < NBR_SUBLISTS; st <<= 1) {
-                        const uint32_t v = __shfl_up_sync(0xffffffffu, before, (st * tg) & 31u);
-                        if (q >= st && st < Q) before += v;
-                    }
-                    before -= active ? nk : 0u;  // exclusive
-                    const uint32_t anyovf = __ballot_sync(0xffffffffu, active && ovf) & (L.group[tg] << ti);
-                    if (active && !anyovf) {
-                        const size_t slot = *kp.rec_slot;
-                        uint32_t* out = kp.rec_nbr + (slot * kp.rec_n4 + gi) * NBR_CAP + before;
-                        for (uint32_t e = 0; e < nk; ++e) {
-                            const uint32_t sidx = my[e];
-                            uint32_t g = sidx;
-#pragma unroll
-                            for (int r = 0; r < R; ++r)
-                                if (sidx >= S.base[r]) g = sidx - S.base[r] + S.lo[r];
-                            out[e] = g;
-                        }
-                    }
-                }
-                acc = reduce_q(acc, q, Q, tg);
-                const float cnt = reduce_q((float)nk, q, Q, tg);
-                const uint32_t om = __ballot_sync(0xffffffffu, active && ovf) & (L.group[tg] << ti);
-                // the target's sub-list lengths, one byte each, gathered through shared memory
-                if (active) wcnt[warp][ti][q] = (uint8_t)min(nk, 127u);
-                __syncwarp();
-                if (active && q == 0) {
-                    acc -= h2 * h2 * h2;  // the target's own term
-                    const float count = cnt - 1.0f;
-                    float rho = kp.rho0, p = kp.p0;
-                    if (count > 2.5f) {
-                        rho = fmaxf(1.0f, kp.mass * kp.kconst * acc);
-                        p = kp.p0 + S.stiff * (rho - kp.rho0);
-                    }
-                    spos[gi] = make_float4(pi.x, pi.y, pi.z, rho);
-                    reinterpret_cast<float*>(svel)[4 * (size_t)gi + 3] = p;
-                    const uint64_t lens = *reinterpret_cast<const uint64_t*>(wcnt[warp][ti]);
-                    nbr_meta[gi] = om ? NBR_SCAN : (Q < 8 ? lens & ((1ull << (8 * Q)) - 1ull) : lens);
-                    if (kp.rec_cnt) kp.rec_cnt[(size_t)*kp.rec_slot * kp.rec_n4 + gi] = om ? REC_SCAN : (uint32_t)(cnt + 0.5f);
-                }
-                // copy the group's lists out. A brick's lists fill the brick's targets' rows of
-                // nbr, stored chunk-major: the 16-byte chunk ch (entries 8ch..8ch+7) of the
-                // brick's u-th target is uint4 number ch * ntarg + u (so that the force pass,
-                // one lane per target, reads consecutive chunks); half-warps copy one chunk of
-                // up to 16 consecutive targets each.
-                __syncwarp();
-                if (staged) {
-                    const uint32_t u0 = t0 + g0 - S.off[RC][1], ntarg = S.off[RC][ncell + 1] - S.off[RC][1];
-                    uint4* dst = reinterpret_cast<uint4*>(nbr + (size_t)(S.lo[RC] + S.off[RC][1]) * NBR_CAP);
-                    const uint32_t row = (uint32_t)lane & 15u;
-                    if (row < tg)
-                        for (uint32_t ch = (uint32_t)lane >> 4; ch < NBR_CAP / 8; ch += 2)
-                            dst[(size_t)ch * ntarg + u0 + row] =
-                                *reinterpret_cast<const uint4*>(wlist + row * WLIST_STRIDE + ch * 8u);
-                }
-                __syncwarp();
-            }
+}
+
+// Ends the barriers' life (after a CTA barrier behind the pass), so that a later phase may
+// initialise them again.
+__device__ __forceinline__ void brick_fini(BrickShared& S) {
+    if (threadIdx.x == 0)
+        for (int i = 0; i < 2; ++i) {
+            mbar_inval(reinterpret_cast<uint64_t*>(&S.full[i]));
+            mbar_inval(reinterpret_cast<uint64_t*>(&S.empty[i]));
         }
+}
+
+// The producer warp's loop (see above). `queue` is the pass's brick counter; a0 (and a1 with
+// NARR = 2) the sorted arrays to stage: buffer s holds a0's candidates at s_buf + s * NARR * CAP
+// and a1's CAP entries behind. Returns false if a wait gave up.
+template <int DIMS, bool BATCH, uint32_t CAP, int NARR>
+__device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, const float4* __restrict__ a0,
+                                              const float4* __restrict__ a1, const uint2* __restrict__ table,
+                                              const uint32_t* __restrict__ bricks, uint32_t n_bricks, uint32_t* queue,
+                                              const KParams& kp, uint32_t* err) {
+    constexpr int R = DIMS == 3 ? 9 : 3;
+    constexpr int RC = DIMS == 3 ? 4 : 1;  // the brick's own row
+    const int lane = threadIdx.x & 31;
+    uint32_t fill = 0;  // units handed over
+    // Waits until the buffer of the next unit is free.
+    auto acquire = [&]() -> bool {
+        if (fill < 2) return true;
+        const bool ok = mbar_wait_bounded(reinterpret_cast<uint64_t*>(&S.empty[fill & 1u]), ((fill >> 1) - 1u) & 1u);
+        if (!ok) atomicOr(err, DEV_ERR_MBAR_TIMEOUT);
+        return __all_sync(0xffffffffu, ok);
+    };
+    auto hand_over = [&]() {
+        uint64_t* full = reinterpret_cast<uint64_t*>(&S.full[fill & 1u]);
+        mbar_arrive(full);
+        cp_async_mbar_arrive(full);
+        ++fill;
+    };
+    uint32_t b = 0;
+    if (lane == 0) b = atomicAdd(queue, 1u);
+    b = __shfl_sync(0xffffffffu, b, 0);
+    uint32_t bid = b < n_bricks ? bricks[b] : 0u;
+    while (b < n_bricks) {
+        uint32_t nb = 0;  // the next brick's ticket, asked for early
+        if (lane == 0) nb = atomicAdd(queue, 1u);
+        const SceneDev* sc = BATCH ? kp.scenes + scene_of<2>(kp.scenes, kp.n_scenes, bid) : nullptr;
+        const int nx = BATCH ? sc->nx : kp.nx, ny = BATCH ? sc->ny : kp.ny, nz = BATCH ? sc->nz : kp.nz;
+        const uint32_t bxn = BATCH ? (uint32_t)sc->bxn : (uint32_t)kp.bxn;
+        const uint32_t lb = BATCH ? bid - sc->brick_off : bid;
+        const uint2* tab = BATCH ? table + sc->cell_off : table;
+        const int bx = (int)(lb % bxn);
+        const uint32_t yz = lb / bxn;
+        const int y = (int)(yz % (uint32_t)ny), z = (int)(yz / (uint32_t)ny);
+        const int xb = bx * kp.bw, ncell = min(kp.bw, nx - xb);
+        // lane c holds column c (cell xb - 1 + c): start and count of its R cells
+        const int cx = xb - 1 + lane;
+        const bool col = lane < ncell + 2 && cx >= 0 && cx < nx;
+        uint32_t st[R], cn[R], tot = 0;
+        bool bad = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int cy = y + (r % 3) - 1, cz = DIMS == 3 ? z + (r / 3) - 1 : 0;
+            uint2 e = make_uint2(EMPTY, 0u);
+            if (col && cy >= 0 && cy < ny && cz >= 0 && cz < nz)
+                e = tab[(uint32_t)cx + (uint32_t)nx * ((uint32_t)cy + (uint32_t)ny * (uint32_t)cz)];
+            const bool some = e.x != EMPTY, in = e.x <= e.y && e.y <= kp.n;
+            bad |= some && !in;  // inconsistent table: report, use an empty cell
+            cn[r] = some && in ? e.y - e.x : 0u;
+            st[r] = some && in ? e.x : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) tot += cn[r];
+        if (bad) atomicOr(err, DEV_ERR_KEY_RANGE);
+        nb = __shfl_sync(0xffffffffu, nb, 0);
+        const uint32_t nbid = nb < n_bricks ? bricks[nb] : 0u;
+        uint32_t incl = tot;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const uint32_t excl = incl - tot, incl_next = __shfl_down_sync(0xffffffffu, incl, 1);
+        for (int c0 = 0; c0 < ncell;) {
+            // targets: columns c0 + 1 .. c1, the most that fit the staging with their neighbours
+            const uint32_t e0 = __shfl_sync(0xffffffffu, excl, c0);
+            const uint32_t fits =
+                __ballot_sync(0xffffffffu, lane > c0 && lane <= min(ncell, c0 + BRICK_UNIT) && incl_next - e0 <= CAP);
+            const int c1 = fits ? 31 - __clz((int)fits) : c0 + 1;
+            const uint32_t mine = lane > c0 && lane <= c1 ? cn[RC] : 0u;
+            const uint32_t some = __ballot_sync(0xffffffffu, mine != 0u);
+            if (some) {
+                uint32_t pairs = (mine + 1u) >> 1;  // inclusive count of the pairs up to this column
+                const uint32_t own = pairs;
+#pragma unroll
+                for (int o = 1; o < BRICK_W_MAX + 2; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, pairs, o);
+                    if (lane >= o) pairs += v;
+                }
+                if (!acquire()) {
+                    cp_async_wait_all();
+                    return false;
+                }
+                BrickUnit& U = S.unit[fill & 1u];
+                const int k = lane - c0;
+                if (k >= 0 && k < c1 - c0 + 2) {
+                    uint32_t o = excl - e0;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        U.off[k * R + r] = o;
+                        U.cell[k * R + r] = make_uint2(st[r], o | (cn[r] << 16));
+                        o += cn[r];
+                    }
+                    if (k == c1 - c0 + 1) U.off[(k + 1) * R] = o;
+                }
+                // target cells beyond the unit's last have no pairs: their entry is the total
+                if (lane > c0 && lane <= c0 + BRICK_UNIT) U.pair[lane - c0 - 1] = pairs - own;
+                if (lane == c1) {
+                    U.npair = pairs;
+                    U.ncell = c1 - c0;
+                    U.staged = fits != 0u;
+                    U.stiff = BATCH ? sc->stiff : kp.stiff;
+                    U.cvisc = BATCH ? sc->cvisc : kp.cvisc;
+                    U.box_min = BATCH ? sc->box_min : kp.box_min;
+                    U.box_max = BATCH ? sc->box_max : kp.box_max;
+                }
+                __syncwarp();
+                if (fits) {
+                    // 8 lanes per cell (a cell of eight particles is one line), 4 x 4 cells at a time
+                    const uint32_t e = (uint32_t)lane & 7u;
+                    const uint32_t dst = smem_addr(s_buf + (fill & 1u) * NARR * CAP) + e * 16u;
+                    const float4* const src0 = a0 + e;
+                    const float4* const src1 = NARR > 1 ? a1 + e : nullptr;
+                    const int nc = (c1 - c0 + 2) * R;
+                    for (int i = lane >> 3; i < nc; i += 16) {
+                        uint2 w[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) w[u] = i + u * 4 < nc ? U.cell[i + u * 4] : make_uint2(0u, 0u);
+                        bool more = false;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t n = w[u].y >> 16, d = dst + (w[u].y & 0xFFFFu) * 16u;
+                            if (e < n) {
+                                cp_async16(d, src0 + w[u].x);
+                                if (NARR > 1) cp_async16(d + CAP * 16u, src1 + w[u].x);
+                            }
+                            if (e + 8u < n) {
+                                cp_async16(d + 128u, src0 + w[u].x + 8);
+                                if (NARR > 1) cp_async16(d + 128u + CAP * 16u, src1 + w[u].x + 8);
+                            }
+                            more |= n > 16u;
+                        }
+                        if (more) {
+                            for (int u = 0; u < 4; ++u) {
+                                const uint32_t n = w[u].y >> 16, d = dst + (w[u].y & 0xFFFFu) * 16u;
+                                for (uint32_t p = 16u; e + p < n; p += 8u) {
+                                    cp_async16(d + p * 16u, src0 + w[u].x + p);
+                                    if (NARR > 1) cp_async16(d + (p + CAP) * 16u, src1 + w[u].x + p);
+                                }
+                            }
+                        }
+                    }
+                }
+                hand_over();
+            }
+            c0 = c1;
+        }
+        b = nb;
+        bid = nbid;
+    }
+    if (!acquire()) return false;
+    if (lane == 0) S.unit[fill & 1u].ncell = 0;
+    __syncwarp();
+    hand_over();
+    cp_async_wait_all();
+    return true;
+}
+
+// A consumer warp's wait for unit number `use`; false if it gave up.
+__device__ __forceinline__ bool unit_wait(BrickShared& S, uint32_t use, uint32_t* err) {
+    const bool ok = mbar_wait_bounded(reinterpret_cast<uint64_t*>(&S.full[use & 1u]), (use >> 1) & 1u);
+    if (!ok) atomicOr(err, DEV_ERR_MBAR_TIMEOUT);
+    return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ void unit_release(BrickShared& S, uint32_t use) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(reinterpret_cast<uint64_t*>(&S.empty[use & 1u]));
+}
+
+// min(r^2 - h^2, 0) of a candidate: its sign bit says whether the candidate is in range (a NaN
+// distance is not), minus its cube is the density term. The x and y differences run as a packed
+// pair, which pays for rounding r^2 before h^2 comes off (folding h^2 into the first
+// multiply-add saves the subtraction and loses up to 14% in the pressure's accuracy).
+template <int DIMS>
+__device__ __forceinline__ float density_term(const float4& pi, const float4& pj, float h2) {
+    float dx, dy;
+    f2_unpack(f2_sub(f2_pack(pi.x, pi.y), f2_pack(pj.x, pj.y)), dx, dy);
+    float r2 = fmaf(dy, dy, dx * dx);
+    if (DIMS == 3) {
+        const float dz = pi.z - pj.z;
+        r2 = fmaf(dz, dz, r2);
+    }
+    return fminf(r2 - h2, 0.0f);
+}
+
+// Recording (an adjoint's recomputation): each target's own part of its pair's list, as sorted
+// indices, in the list's order, and its length (REC_SCAN where there is none or it is too long).
+template <int R>
+__device__ __forceinline__ void density_record(const BrickUnit& U, const KParams& kp, const PairTask& t, bool list,
+                                               uint32_t nU, const float4& pA, const float4& pB, const float4* buf,
+                                               const uint16_t* wlist) {
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u, quad = 0xFu << (lane & 28u);
+    const size_t base = (size_t)*kp.rec_slot * kp.rec_n4;
+    uint32_t n[2] = {0u, 0u};
+    const uint32_t rounds = t.live && list ? (nU + 3u) >> 2 : 0u;
+    for (uint32_t k = 0; __any_sync(0xffffffffu, k < rounds); ++k) {
+        const uint32_t e = 4u * k + q;
+        const bool some = k < rounds && e < nU;
+        uint32_t g = 0;
+        float4 pj = pA;
+        if (some) {
+            const uint32_t v = t.lo + (wlist[e] >> 4);
+            pj = buf[v];
+            int a = t.c * R, z = (t.c + 3) * R;  // the last cell that starts at or before v
+            while (z - a > 1) {
+                const int m = (a + z) >> 1;
+                if (U.off[m] <= v) a = m;
+                else z = m;
+            }
+            g = U.cell[a].x + (v - U.off[a]);
+        }
+#pragma unroll
+        for (uint32_t w = 0; w < 2u; ++w) {
+            const bool in = some && (w == 0u || t.two) && density_term<R == 9 ? 3 : 2>(w ? pB : pA, pj, kp.h2) < 0.0f;
+            const uint32_t m = __ballot_sync(0xffffffffu, in) & quad, at = n[w] + (uint32_t)__popc(m & lanemask_lt());
+            if (in && at < NBR_CAP) kp.rec_nbr[(base + t.gi + w) * NBR_CAP + at] = g;
+            n[w] += (uint32_t)__popc(m);
+        }
+    }
+    if (t.live && q < (t.two ? 2u : 1u)) {
+        const uint32_t c = q ? n[1] : n[0];
+        kp.rec_cnt[base + t.gi + q] = list && c <= NBR_CAP ? c : REC_SCAN;
+    }
+}
+
+// Density + pressure for every particle of the occupied bricks, and the pairs' neighbour lists.
+// Writes sorted position .w = density and sorted velocity .w = pressure, as
+// clCalculateDensity does (libCL/phys/oclFluid3D.cl:189-199). A pair's four lanes walk every
+// fourth candidate of its window. Whether a candidate is in range is kept as a bit per target
+// (one funnel shift of the term's sign), and the lists are written from the bits afterwards.
+// Every target meets itself (term h^6, one count); that term is taken off after the sum. A list
+// lies in the 128 (a single: 64) entries of nbr that belong to its particles; entries are places
+// in the window times 16 (bytes). nbr_meta of the pair's first particle: their number, or
+// NBR_SCAN where there are more or the unit was not staged.
+// Returns false if a wait gave up.
+template <int DIMS, bool BATCH>
+__device__ __forceinline__ bool density_brick_run(float4* s_buf, BrickShared& S, float4* __restrict__ spos,
+                                                  float4* __restrict__ svel, const uint2* __restrict__ table,
+                                                  const uint32_t* __restrict__ bricks, uint32_t* counters,
+                                                  const KParams& kp, uint16_t* __restrict__ nbr,
+                                                  uint32_t* __restrict__ nbr_meta, uint32_t* err) {
+    constexpr int R = DIMS == 3 ? 9 : 3;
+    constexpr int RC = DIMS == 3 ? 4 : 1;
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
+    const int warp = threadIdx.x >> 5, consumers = (int)(blockDim.x >> 5) - 1;
+    brick_init(S);
+    const uint32_t n_bricks = __ldcg(counters);  // written by the bounds pass (an earlier kernel or phase)
+    if (warp == consumers) {
+        const bool ok = brick_produce<DIMS, BATCH, DENSITY_CAP, 1>(S, s_buf, spos, nullptr, table, bricks, n_bricks,
+                                                                   &counters[1], kp, err);
+        if (!ok) atomicExch(&counters[3], 1u);
+        return ok;
+    }
+    uint16_t* wlist = reinterpret_cast<uint16_t*>(s_buf + 2 * DENSITY_CAP) + (warp * TASK_PAIRS + (lane >> 2)) * LIST_STRIDE;
+    const uint32_t row = smem_addr(wlist);
+    const float h2 = kp.h2;
+    int turn = warp;  // tasks of eight pairs are dealt to the consumer warps in turn, across units
+    for (uint32_t use = 0;; ++use) {
+        if (!unit_wait(S, use, err)) {
+            atomicExch(&counters[3], 1u);  // no lists for the rest: the force pass leaves them out
+            return false;
+        }
+        const BrickUnit& U = S.unit[use & 1u];
+        if (U.ncell == 0) break;
+        const float4* buf = s_buf + (use & 1u) * DENSITY_CAP;
+        const bool staged = U.staged != 0;
+        const int tasks = (int)((U.npair + TASK_PAIRS - 1u) / TASK_PAIRS);
+        for (; turn < tasks; turn += consumers) {
+            const PairTask t = pair_task<R, RC>(U, (uint32_t)turn * TASK_PAIRS + (lane >> 2));
+            const float4 pA = staged ? buf[t.self] : spos[t.gi];
+            const float4 pB = staged ? buf[t.self + (t.two ? 1u : 0u)] : spos[t.gi + (t.two ? 1u : 0u)];
+            float accA = 0.0f, accB = 0.0f;
+            uint32_t cnt = 0;  // this lane's in-range candidates: A low, B high half
+            uint32_t nU = 0;   // the pair's list entries so far
+            const uint32_t cap = t.two ? 2u * NBR_CAP : NBR_CAP;
+            // terms of one candidate; the signs go to the bits
+            uint32_t mA = 0, mB = 0;
+            auto candidate = [&](const float4& pj) {
+                const float uA = density_term<DIMS>(pA, pj, h2), uB = density_term<DIMS>(pB, pj, h2);
+                const uint64_t u = f2_pack(uA, uB);  // packed: half the issue slots
+                f2_unpack(f2_fma(f2_mul(u, u), u, f2_pack(accA, accB)), accA, accB);
+                mA = __funnelshift_l(__float_as_uint(uA), mA, 1);
+                mB = __funnelshift_l(__float_as_uint(uB), mB, 1);
+            };
+            if (staged) {
+                const uint32_t total = (t.len + 3u - q) >> 2;  // this lane's candidates
+                uint32_t a = smem_addr(buf + t.lo + q), v0 = q * 16u;
+                for (uint32_t i0 = 0; __any_sync(0xffffffffu, i0 < total); i0 += 32u) {
+                    const uint32_t m = i0 < total ? min(32u, total - i0) : 0u;  // at most a word of bits
+                    mA = mB = 0u;
+#pragma unroll 4
+                    for (uint32_t i = 0; i < m; ++i, a += 64u) candidate(lds_f4(a));
+                    if (!t.two) mB = 0u;
+                    cnt += (uint32_t)__popc(mA) + ((uint32_t)__popc(mB) << 16);
+                    uint32_t either = mA | mB;
+                    // places in the list: the counts of the pair's lanes before this one
+                    const uint32_t own = (uint32_t)__popc(either);
+                    uint32_t inc = own;
+                    uint32_t v = __shfl_up_sync(0xffffffffu, inc, 1);
+                    if (q >= 1u) inc += v;
+                    v = __shfl_up_sync(0xffffffffu, inc, 2);
+                    if (q >= 2u) inc += v;
+                    uint32_t w = row + 2u * (nU + inc - own);
+                    nU += __shfl_sync(0xffffffffu, inc, lane | 3u);
+                    if (nU > cap) either = 0u;  // too many: no list
+                    const uint32_t vk = v0 + (m - 1u) * 64u;  // the candidate at bit 0
+                    while (either) {
+                        const uint32_t bit = 31u - (uint32_t)__clz((int)either);
+                        either ^= 1u << bit;
+                        sts_u16(w, vk - bit * 64u);
+                        w += 2u;
+                    }
+                    v0 += 32u * 64u;
+                }
+            } else {  // unstaged unit: candidates from global memory, no lists
+                for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
+                    const uint32_t n = U.off[i + 1] - U.off[i], first = U.cell[i].x;
+                    for (uint32_t k = q; k < n; k += 4u) {
+                        mA = mB = 0u;
+                        candidate(spos[first + k]);
+                        if ((cnt & 0xFFFFu) < 0x1000u) cnt += mA;  // "many" is all that is asked of the counts
+                        if ((cnt >> 16) < 0x1000u) cnt += mB << 16;
+                    }
+                }
+            }
+#pragma unroll
+            for (uint32_t m = 1; m < 4u; m <<= 1) {
+                accA += __shfl_xor_sync(0xffffffffu, accA, m);
+                accB += __shfl_xor_sync(0xffffffffu, accB, m);
+                cnt += __shfl_xor_sync(0xffffffffu, cnt, m);
+            }
+            const bool list = staged && nU <= cap;
+            // lane 0 of the four finishes target A, lane 1 target B
+            if (t.live && (q == 0u || (q == 1u && t.two))) {
+                const uint32_t gi = t.gi + q, n = q ? cnt >> 16 : cnt & 0xFFFFu;
+                const float sum = -(q ? accB : accA) - kp.h2 * kp.h2 * kp.h2;  // without the target's own term
+                const float4 pi = q ? pB : pA;
+                float rho = kp.rho0, p = kp.p0;
+                if (n > 3u) {  // the reference's count > 2 does not count the target
+                    rho = fmaxf(1.0f, kp.mass * kp.kconst * sum);
+                    p = kp.p0 + U.stiff * (rho - kp.rho0);
+                }
+                spos[gi] = make_float4(pi.x, pi.y, pi.z, rho);
+                reinterpret_cast<float*>(svel)[4 * (size_t)gi + 3] = p;
+                if (q == 0u) nbr_meta[gi] = list ? nU : NBR_SCAN;
+            }
+            __syncwarp();
+            if (list && t.live)
+                for (uint32_t ch = q; ch * 8u < nU; ch += 4u)
+                    reinterpret_cast<uint4*>(nbr)[(size_t)t.gi * (NBR_CAP / 8) + ch] =
+                        *reinterpret_cast<const uint4*>(wlist + ch * 8u);
+            if (kp.rec_nbr) density_record<R>(U, kp, t, list, nU, pA, pB, buf, wlist);
+            __syncwarp();
+        }
+        turn -= tasks;
+        unit_release(S, use);
     }
     return true;
 }
 
 template <int DIMS, bool BATCH>
-__global__ void __launch_bounds__(BRICK_THREADS, 4) k_density_brick(float4* __restrict__ spos,
+__global__ void __launch_bounds__(32 * DENSITY_CONSUMERS + 32, DENSITY_CTAS) k_density_brick(float4* __restrict__ spos,
                                                                  float4* __restrict__ svel,
                                                                  const uint2* __restrict__ table,
                                                                  const uint32_t* __restrict__ bricks,
                                                                  uint32_t* counters, KParams kp,
                                                                  uint16_t* __restrict__ nbr,
-                                                                 uint64_t* __restrict__ nbr_meta, uint32_t* err) {
-    extern __shared__ float4 s_buf[];  // [BRICK_CAP] positions, then per-warp neighbour lists
-    __shared__ BrickShared S[2];
-    __shared__ LaneMap L;
-    __shared__ __align__(8) SubListCounts wcnt;
-    density_brick_run<DIMS, BATCH>(s_buf, S, L, wcnt, spos, svel, table, bricks, counters, kp, nbr, nbr_meta, err);
+                                                                 uint32_t* __restrict__ nbr_meta, uint32_t* err) {
+    extern __shared__ float4 s_buf[];
+    __shared__ BrickShared S;
+    density_brick_run<DIMS, BATCH>(s_buf, S, spos, svel, table, bricks, counters, kp, nbr, nbr_meta, err);
 }
 
-// Pressure + viscosity contribution of one in-range neighbour (acc: pressure xyz, viscosity xyz).
-template <int DIMS>
-__device__ __forceinline__ void force_pair(const float4& pi, const float4& vi, float inv_rho_i, const float4& pj,
-                                           const float4& vj, float h, float* acc) {
-    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = DIMS == 3 ? pi.z - pj.z : 0.0f;
-    float r2 = fmaf(dy, dy, dx * dx);
-    if (DIMS == 3) r2 = fmaf(dz, dz, r2);
-    const float inv = rsqrtf(r2);
-    const float vlen = r2 * inv;
-    const float hr = h - vlen;
-    const float dd = inv_rho_i * __frcp_rn(pj.w);  // 1 / (rho_i rho_j)
-    const float sp = (vi.w + vj.w) * dd * hr * hr * inv;
-    acc[0] = fmaf(sp, dx, acc[0]);
-    acc[1] = fmaf(sp, dy, acc[1]);
-    acc[2] = fmaf(sp, dz, acc[2]);
-    const float cv = hr * dd;
-    acc[3] = fmaf(vj.x - vi.x, cv, acc[3]);
-    acc[4] = fmaf(vj.y - vi.y, cv, acc[4]);
-    acc[5] = fmaf(vj.z - vi.z, cv, acc[5]);
-}
-
-// Reciprocal with the approximate (about 1 ulp) hardware instruction.
+// Reciprocal and reciprocal square root with the hardware's approximations (1 and 2 ulp).
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+constexpr uint32_t MIN_NORMAL = 0x00800000u;  // bits of the smallest normal float
 
-// force_pair on the force pass's staged copies. The target's w lanes hold a_i = 1/rho_i
-// (position) and b_i = p_i/rho_i (velocity); the neighbour's hold rho_j and p_j as the density
-// pass wrote them, from which a_j = rcp(rho_j) and b_j = p_j a_j are formed here:
-// (p_i + p_j) / (rho_i rho_j) = b_i a_j + a_i b_j. Skips r = 0 (the target itself, which its
-// list holds, and coincident particles).
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Pressure + viscosity contribution of one candidate (acc: pressure xyz, viscosity xyz), if it is
+// in range. The w lanes hold density (positions) and pressure (velocities); ai = 1 / rho_i, aj =
+// 1 / rho_j. The range test is one unsigned compare of r^2's bits, which also leaves out r = 0
+// (the target itself, which its list holds, and coincident particles) and NaN.
 template <int DIMS>
-__device__ __forceinline__ void force_pair_pre(const float4& pi, const float4& vi, const float4& pj,
-                                               const float4& vj, float h, float* acc) {
+__device__ __forceinline__ void force_pair(const float4& pi, const float4& vi, float ai, const float4& pj,
+                                           const float4& vj, float aj, float h, uint32_t thr, float* acc) {
     const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = DIMS == 3 ? pi.z - pj.z : 0.0f;
     float r2 = fmaf(dy, dy, dx * dx);
     if (DIMS == 3) r2 = fmaf(dz, dz, r2);
-    if (!(r2 > 0.0f)) return;
-    const float inv = rsqrtf(r2);
-    const float hr = h - r2 * inv;
-    const float aj = rcp_approx(pj.w), bj = vj.w * aj;
-    const float dd = pi.w * aj;  // 1 / (rho_i rho_j)
-    const float sp = fmaf(vi.w, aj, pi.w * bj) * (hr * hr * inv);
-    acc[0] = fmaf(sp, dx, acc[0]);
-    acc[1] = fmaf(sp, dy, acc[1]);
-    acc[2] = fmaf(sp, dz, acc[2]);
-    const float cv = hr * dd;
-    acc[3] = fmaf(vj.x - vi.x, cv, acc[3]);
-    acc[4] = fmaf(vj.y - vi.y, cv, acc[4]);
-    acc[5] = fmaf(vj.z - vi.z, cv, acc[5]);
+    const float inv = rsqrt_approx(r2);
+    const float hr = fmaf(-r2, inv, h);               // h - r
+    const float cv = hr * (ai * aj);                   // (h - r) / (rho_i rho_j)
+    const float sp = (vi.w + vj.w) * cv * (hr * inv);  // (p_i + p_j) (h - r)^2 / (rho_i rho_j r)
+    if (__float_as_uint(r2) - MIN_NORMAL < thr) {
+        acc[0] = fmaf(sp, dx, acc[0]);
+        acc[1] = fmaf(sp, dy, acc[1]);
+        if (DIMS == 3) acc[2] = fmaf(sp, dz, acc[2]);
+        acc[3] = fmaf(vj.x - vi.x, cv, acc[3]);
+        acc[4] = fmaf(vj.y - vi.y, cv, acc[4]);
+        acc[5] = fmaf(vj.z - vi.z, cv, acc[5]);
+    }
+}
+
+// clip_box_force with a particle on four lanes, lane l holding component l of its force: the two
+// walls of the lane's axis (none for w, nor for z in 2D), and the sum of the walls' w terms
+// (0 * magnitude) on lane 3. Whole warps; `live` lanes have a particle.
+template <int DIMS>
+__device__ __forceinline__ float clip_box_lane(const KParams& kp, const float4& box_min, const float4& box_max,
+                                               const float4& pos, const float4& vel, float f, uint32_t l, bool live) {
+    const float x = l == 0u ? pos.x : (l == 1u ? pos.y : pos.z);
+    const float lo = l == 0u ? box_min.x : (l == 1u ? box_min.y : box_min.z);
+    const float hi = l == 0u ? box_max.x : (l == 1u ? box_max.y : box_max.z);
+    const float below = __fsub_rn(kp.radius, __fsub_rn(x, lo)), above = __fsub_rn(kp.radius, __fsub_rn(hi, x));
+    const bool axis = live && l < (DIMS == 3 ? 3u : 2u);
+    if (!__any_sync(0xffffffffu, axis && (below > 0.00001f || above > 0.00001f))) return f;
+    const float v = l == 0u ? vel.x : (l == 1u ? vel.y : vel.z);
+    float fw = 0.0f;
+    if (axis) {
+        add_wall(f, fw, 1.0f, below, v);
+        add_wall(f, fw, -1.0f, above, v);
+    }
+    fw += __shfl_xor_sync(0xffffffffu, fw, 1);
+    fw += __shfl_xor_sync(0xffffffffu, fw, 2);
+    return l == 3u ? __fadd_rn(f, fw) : f;
+}
+
+// integrate_force with a particle on four lanes: the lane's component of the new velocity. The
+// clamp's test on the length is made on its square (kp.v2_thresh), so that the root and the
+// division are left to the particles that are clamped.
+__device__ __forceinline__ float integrate_force_lane(const KParams& kp, float v, float f) {
+    const float q = __fmul_rn(f, f);
+    const int g = threadIdx.x & 28;
+    const float f2 = __fadd_rn(__fadd_rn(__fadd_rn(__shfl_sync(0xffffffffu, q, g), __shfl_sync(0xffffffffu, q, g + 1)),
+                                         __shfl_sync(0xffffffffu, q, g + 2)), __shfl_sync(0xffffffffu, q, g + 3));
+    if (f2 >= kp.v2_thresh) f = __fmul_rn(f, __fdiv_rn(kp.vlimit, __fsqrt_rn(f2)));
+    return __fadd_rn(v, __fmul_rn(f, kp.dt));
 }
 
 // Forces (pressure + viscosity) for every particle of the occupied bricks
-// (clCalculateForces, libCL/phys/oclFluid3D.cl:202-255). The brick's rows are staged exactly
-// as in k_density_brick; two lanes take a target and evaluate the in-range pairs that the
-// density kernel recorded in the target's sub-lists. A target whose sub-lists overflowed is
-// scanned over its rows by its whole warp after the list walk; in an unstaged brick both lanes
-// scan the rows in global memory. With FUSED the clip-box, integrate-force, gravity and
-// integrate-velocity stages follow in registers; otherwise the SPH force is added to
-// force[index[i]] (with w = 0) as clCalculateForces does.
-// The body of k_force_brick, on shared memory the caller provides: s_buf (FORCE_SMEM bytes:
-// [BRICK_CAP] positions, [BRICK_CAP] velocities, then the neighbour lists of up to
-// LIST_STAGE_MAX targets), S and L. COH: the sorted state and the lists were written earlier
-// in the same launch, so the direct loads of them go through L2 only. Returns false if a
-// bulk-copy wait gave up (the CTA left the loop).
+// (clCalculateForces, libCL/phys/oclFluid3D.cl:202-255). A pair's lane l evaluates entries 2 l and
+// 2 l + 1 of each 8-entry chunk of the pair's list for both targets; the lists' first LIST_AHEAD
+// chunks are read straight from global memory before anything else, the candidates lie in the
+// staging. Targets without a list in a staged unit are scanned over their window by the whole
+// warp; in an unstaged unit the pair's lanes scan the cells in global memory. With FUSED the
+// clip-box, integrate-force, gravity and integrate-velocity stages follow in registers, a
+// component per lane; otherwise the SPH force is added to force[index[i]] (with w = 0) as
+// clCalculateForces does.
+// COH: the sorted state and the lists were written earlier in the same launch, so the direct
+// loads of them go through L2 only. Returns false if a wait gave up.
 template <int DIMS, bool FUSED, bool BATCH, bool COH = false>
-__device__ __forceinline__ bool force_brick_run(float4* s_buf, BrickShared* S2, LaneMap& L,
-                                                const float4* __restrict__ spos, const float4* __restrict__ svel,
-                                                const uint32_t* __restrict__ index, float4* __restrict__ pos,
-                                                float4* __restrict__ vel, float4* __restrict__ force,
-                                                const uint2* __restrict__ table, const uint32_t* __restrict__ bricks,
-                                                uint32_t* counters, const KParams& kp,
-                                                const uint16_t* __restrict__ nbr,
-                                                const uint64_t* __restrict__ nbr_meta, uint32_t* err) {
+__device__ __forceinline__ bool force_brick_run(float4* s_buf, BrickShared& S, const float4* __restrict__ spos,
+                                                const float4* __restrict__ svel, const uint32_t* __restrict__ index,
+                                                float4* __restrict__ pos, float4* __restrict__ vel,
+                                                float4* __restrict__ force, const uint2* __restrict__ table,
+                                                const uint32_t* __restrict__ bricks, uint32_t* counters,
+                                                const KParams& kp, const uint16_t* __restrict__ nbr,
+                                                const uint32_t* __restrict__ nbr_meta, uint32_t* err) {
     constexpr int R = DIMS == 3 ? 9 : 3;
     constexpr int RC = DIMS == 3 ? 4 : 1;
-    const int t = threadIdx.x, lane = t & 31;
-    lane_map_init(L);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(&S2[0].bar);
-    if (t == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    uint32_t phase = 0;
-    const uint32_t n_bricks = __ldcg(counters);  // written by the bounds pass (an earlier kernel or phase)
-    const float4* s_pos = s_buf;
-    const float4* s_vel = s_buf + BRICK_CAP;
-    uint16_t* s_lists = reinterpret_cast<uint16_t*>(s_buf + 2 * BRICK_CAP);
-    uint64_t* s_meta = reinterpret_cast<uint64_t*>(reinterpret_cast<char*>(s_lists) + FORCE_LIST_BYTES);
-    uint32_t* s_index = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(s_meta) + FORCE_META_BYTES);
-    // records used in turn, as in density_brick_run
-    if (t == 0) S2[0].brick = atomicAdd(&counters[2], 1u);
-    __syncthreads();
-    for (uint32_t it = 0;; it ^= 1u) {
-        BrickShared& S = S2[it];
-        const uint32_t b = S.brick;
-        if (b >= n_bricks) break;
-        if (t == 0) S2[it ^ 1u].brick = atomicAdd(&counters[2], 1u);
-        int x0, ncell;
-        brick_setup<DIMS, BATCH>(S, kp, bricks[b], table, err, x0, ncell);
-        // the brick's targets are consecutive particles: stage their lists with the rows
-        const uint32_t tfirst = S.lo[RC] + S.off[RC][1];
-        const uint32_t ntarg = S.off[RC][ncell + 1] - S.off[RC][1];
-        const bool lists_staged = ntarg <= LIST_STAGE_MAX && S.rcnt[RC] > 0;
-        // warp 0: row bases (a scan of the rows' counts); if the brick fits, lane 0 arms the
-        // mbarrier with the byte count, lane r copies row r's positions and velocities, and lanes
-        // R .. R + 2 the targets' lists, list lengths and permutation entries
-        if (t < 32) {
-            const uint32_t rc = lane < R ? S.rcnt[lane] : 0u;
-            uint32_t inc = rc;
+    const uint32_t lane = threadIdx.x & 31u, l = lane & 3u;
+    const int warp = threadIdx.x >> 5, consumers = (int)(blockDim.x >> 5) - 1;
+    brick_init(S);
+    // written by the bounds pass (an earlier kernel or phase); nothing to do where the density
+    // pass gave up, which leaves particles without a list
+    const uint32_t n_bricks = __ldcg(counters + 3) ? 0u : __ldcg(counters);
+    if (warp == consumers)
+        return brick_produce<DIMS, BATCH, FORCE_CAP, 2>(S, s_buf, spos, svel, table, bricks, n_bricks, &counters[2], kp,
+                                                        err);
+    const uint32_t thr = max(__float_as_uint(kp.r2_thresh), MIN_NORMAL) - MIN_NORMAL;
+    int turn = warp;  // tasks of eight pairs are dealt to the consumer warps in turn, across units
+    for (uint32_t use = 0;; ++use) {
+        if (!unit_wait(S, use, err)) return false;
+        const BrickUnit& U = S.unit[use & 1u];
+        if (U.ncell == 0) break;
+        const float4* s_pos = s_buf + (use & 1u) * 2u * FORCE_CAP;
+        const float4* s_vel = s_pos + FORCE_CAP;
+        const bool staged = U.staged != 0;
+        const float cvisc = U.cvisc;
+        const int tasks = (int)((U.npair + TASK_PAIRS - 1u) / TASK_PAIRS);
+        for (; turn < tasks; turn += consumers) {
+            const PairTask t = pair_task<R, RC>(U, (uint32_t)turn * TASK_PAIRS + (lane >> 2));
+            const uint32_t two = t.two ? 1u : 0u;
+            // everything from global memory at once: the list's length and first chunks (whatever
+            // its length), the targets' particles and, with those known, the lane's component of
+            // their force, velocity and position
+            const uint32_t meta = ld_phase<COH>(nbr_meta + t.gi);
+            const uint32_t oA = ld_phase<COH>(index + t.gi), oB = ld_phase<COH>(index + t.gi + two);
+            const uint32_t* list = reinterpret_cast<const uint32_t*>(nbr) + (size_t)t.gi * (NBR_CAP / 2) + l;
+            uint32_t ch[LIST_AHEAD];
 #pragma unroll
-            for (int o = 1; o < 16; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += v;
+            for (uint32_t k = 0; k < LIST_AHEAD; ++k) ch[k] = ld_phase<COH>(list + 4u * k);
+            const float f_A = reinterpret_cast<const float*>(force + oA)[l], f_B = reinterpret_cast<const float*>(force + oB)[l];
+            float v_A = 0.f, v_B = 0.f, p_A = 0.f, p_B = 0.f;
+            if (FUSED) {
+                v_A = reinterpret_cast<const float*>(vel + oA)[l];
+                v_B = reinterpret_cast<const float*>(vel + oB)[l];
+                p_A = reinterpret_cast<const float*>(pos + oA)[l];
+                p_B = reinterpret_cast<const float*>(pos + oB)[l];
             }
-            const uint32_t base = inc - rc, total = __shfl_sync(0xffffffffu, inc, R - 1);
-            if (lane < R) S.base[lane] = base;
-            if (total <= BRICK_CAP && total > 0) {
-                const uint32_t lbytes = lists_staged ? ntarg * NBR_CAP * 2 : 0u;
-                // list lengths and permutation entries of the targets, from 16-byte boundaries
-                const uint32_t mbytes = lists_staged ? (((tfirst + ntarg + 1u) & ~1u) - (tfirst & ~1u)) * 8u : 0u;
-                const uint32_t ibytes = lists_staged ? (((tfirst + ntarg + 3u) & ~3u) - (tfirst & ~3u)) * 4u : 0u;
-                if (lane == 0) mbar_arrive_expect_tx(bar, total * 32u + lbytes + mbytes + ibytes);
-                __syncwarp();
-                if (lane < R && rc) {
-                    fence_proxy_async_smem();  // as in brick_stage
-                    fence_proxy_async_global();
-                    bulk_g2s(s_buf + base, spos + S.lo[lane], rc * 16u, bar);
-                    bulk_g2s(s_buf + BRICK_CAP + base, svel + S.lo[lane], rc * 16u, bar);
-                }
-                if (lbytes && lane >= R && lane < R + 3) {
-                    fence_proxy_async_smem();
-                    fence_proxy_async_global();
-                    if (lane == R) bulk_g2s(s_lists, nbr + (size_t)tfirst * NBR_CAP, lbytes, bar);
-                    else if (lane == R + 1) bulk_g2s(s_meta, nbr_meta + (tfirst & ~1u), mbytes, bar);
-                    else bulk_g2s(s_index, index + (tfirst & ~3u), ibytes, bar);
-                }
+            float4 pA, pB, vA, vB;
+            if (staged) {
+                pA = s_pos[t.self];
+                pB = s_pos[t.self + two];
+                vA = s_vel[t.self];
+                vB = s_vel[t.self + two];
+            } else {
+                pA = ld_phase<COH>(spos + t.gi);
+                pB = ld_phase<COH>(spos + t.gi + two);
+                vA = ld_phase<COH>(svel + t.gi);
+                vB = ld_phase<COH>(svel + t.gi + two);
             }
-        }
-        const uint32_t total = brick_total<DIMS>(S);
-        const bool staged = total <= BRICK_CAP && total > 0;
-        if (staged && !brick_wait(bar, phase, err)) return false;
-        // P = 2 lanes per target: the brick's targets are consecutive in the centre row, so the
-        // CTA takes 128 of them at a time whatever cell they are in; the two lanes of a target
-        // split its list (or, in an unstaged brick, take alternate candidates of each row) and
-        // their partial sums are added with a shuffle. The summation order depends on neither
-        // the brick width nor the brick's target count, as long as the brick is staged.
-        const uint32_t tbeg = S.off[RC][1];
-        constexpr uint32_t lp = 1u, P = 1u << lp;
-        for (uint32_t u0 = 0; u0 < ntarg; u0 += BRICK_THREADS >> lp) {
-            const uint32_t u = u0 + ((uint32_t)t >> lp), p = (uint32_t)t & (P - 1u);
-            const bool active = u < ntarg;
-            const uint32_t tl = tbeg + u;
-            const uint32_t gi = S.lo[RC] + tl;
-            float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), vi = pi, f_o = pi, v_o = pi, p_o = pi;
-            uint32_t o = 0, Q = 0, sub = 0, c = 0;
-            uint64_t meta = NBR_SCAN;
-            if (active) {
-                // the target's cell and its place in the density pass's groups (its sub-lists)
-                while (c + 1 < (uint32_t)ncell && S.off[RC][c + 2] <= tl) ++c;
-                const uint32_t c0 = S.off[RC][c + 1], nt = S.off[RC][c + 2] - c0;
-                const uint32_t g0 = (tl - c0) & ~(GROUP_MAX - 1u);
-                const uint32_t f = L.info[min(GROUP_MAX, nt - g0)];
-                Q = f & 0xFFu;
-                sub = f >> 8;
-                pi = staged ? s_pos[S.base[RC] + tl] : ld_phase<COH>(spos + gi);
-                vi = staged ? s_vel[S.base[RC] + tl] : ld_phase<COH>(svel + gi);
-                if (staged) {  // the target's w lanes: 1/rho and p/rho (force_pair_pre)
-                    pi.w = rcp_approx(pi.w);
-                    vi.w *= pi.w;
-                }
-                if (p == 0) {  // prefetch what the integration needs
-                    o = (staged && lists_staged) ? s_index[gi - (tfirst & ~3u)] : ld_phase<COH>(index + gi);
-                    f_o = force[o];
-                    if (FUSED) {
-                        v_o = vel[o];
-                        p_o = pos[o];
-                    }
-                }
-                meta = !staged ? NBR_SCAN : (lists_staged ? s_meta[gi - (tfirst & ~1u)] : ld_phase<COH>(nbr_meta + gi));
-            }
-            const bool scan = (meta & NBR_SCAN) != 0;
-            // Sub-lists that start on 16-byte chunks and pair up (Q = 2, 4, 8) can be walked a
-            // chunk at a time; a warp whose listed targets are all of that kind does so. Any
-            // other warp walks every listed target in one flat loop (the same loop for every
-            // layout, so that its lanes stay together). Both visit a target's entries in the
-            // same order, which depends on the target's own sub-lists only: with Q even lane p
-            // takes sub-lists p, p + 2, ... whole, otherwise entries p, p + 2, ... of the
-            // concatenated sub-lists.
-            const bool whole = (Q % P) == 0 && (sub & 7u) == 0;
-            const bool chunked = __all_sync(0xffffffffu, scan || whole);
-            if (active) {
-                const float inv_rho_i = staged ? pi.w : 1.0f / pi.w;
-                if (!scan) {
-                    // slot s of the target's list sits at chunk-major position
-                    // ((s >> 3) * ntarg + u) * 8 + (s & 7)
-                    const uint16_t* lst = (lists_staged ? s_lists : nbr + (size_t)tfirst * NBR_CAP) + (gi - tfirst) * 8u;
-                    const uint32_t n8 = ntarg * 8u;
-                    if (!chunked) {
-                        // (q, k): the next entry's sub-list and place in it; m: the lane's count
-                        const bool pairs = (Q % P) == 0;
-                        const uint32_t dq = pairs ? P : 1u, dk = pairs ? 1u : P;
-                        uint32_t q = pairs ? p : 0u, k = pairs ? 0u : p, m;
-                        if (pairs) {  // bytes p, p + 2, ... of meta
-                            m = (uint32_t)(((meta & (0x00FF00FF00FF00FFull << (8 * p))) * 0x0101010101010101ull) >> 56);
-                        } else {
-                            const uint32_t n = (uint32_t)((meta * 0x0101010101010101ull) >> 56);
-                            m = n > p ? (n - p + P - 1u) / P : 0u;
-                        }
-                        uint32_t nq = (uint32_t)(meta >> (8 * q)) & 127u;
-                        auto settle = [&]() {
-                            while (k >= nq && q + dq < Q) {
-                                k -= nq;
-                                q += dq;
-                                nq = (uint32_t)(meta >> (8 * q)) & 127u;
-                            }
-                        };
-                        settle();
-#pragma unroll 1
-                        for (uint32_t i = 0; i < m; ++i) {
-                            const uint32_t s = q * sub + k;
-                            const uint32_t li = (s >> 3) * n8 + (s & 7u);
-                            // staged lists are in shared memory, the others in global memory
-                            const uint32_t i0 = lists_staged ? lst[li] : ld_phase<COH>(lst + li);
-                            force_pair_pre<DIMS>(pi, vi, s_pos[i0], s_vel[i0], kp.h, acc);
-                            k += dk;
-                            settle();
-                        }
-                    } else {
-#pragma unroll 1
-                        for (uint32_t q = p; q < Q; q += P) {
-                            const uint32_t n = (uint32_t)(meta >> (8 * q)) & 127u;
-                            const uint4* l4 = reinterpret_cast<const uint4*>(lst);
-                            for (uint32_t k0 = 0; k0 < n; k0 += 8) {
-                                const size_t li = (size_t)((q * sub + k0) >> 3) * ntarg;
-                                const uint4 v = lists_staged ? l4[li] : ld_phase<COH>(l4 + li);
-                                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-                                const uint32_t m = min(8u, n - k0);
+            const float aA = rcp_approx(pA.w), aB = rcp_approx(pB.w);
+            float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            auto both = [&](const float4& pj, const float4& vj) {
+                const float aj = rcp_approx(pj.w);
+                force_pair<DIMS>(pA, vA, aA, pj, vj, aj, kp.h, thr, accA);
+                force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
+            };
+            const bool scan = meta == NBR_SCAN;
+            if (staged) {
+                const uint32_t n = scan ? 0u : meta, win = smem_addr(s_pos + t.lo);
+                auto entry = [&](uint32_t v) { both(lds_f4(win + v), lds_f4(win + v + FORCE_CAP * 16u)); };
+                for (uint32_t k0 = 2u * l; k0 < n; k0 += 8u * LIST_AHEAD) {
+                    if (k0 >= 8u * LIST_AHEAD) {
 #pragma unroll
-                                for (uint32_t e = 0; e < 8; ++e) {
-                                    if (e >= m) break;
-                                    const uint32_t idx = (w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
-                                    force_pair_pre<DIMS>(pi, vi, s_pos[idx], s_vel[idx], kp.h, acc);
-                                }
-                            }
-                        }
+                        for (uint32_t k = 0; k < LIST_AHEAD; ++k)
+                            if (k0 + 8u * k < n) ch[k] = ld_phase<COH>(list + 4u * k + ((k0 >> 3) << 2));
                     }
-                } else if (!staged) {  // unstaged brick: both lanes scan the rows in global memory
-#pragma unroll 1
-                    for (int r = 0; r < R; ++r) {
-                        const float4* rp = spos + S.lo[r];
-                        const float4* rv = svel + S.lo[r];
-                        const uint32_t hi = S.off[r][c + 3];
-                        for (uint32_t j = S.off[r][c] + p; j < hi; j += P) {
-                            const float4 pj = ld_phase<COH>(rp + j);
-                            const float dx = pi.x - pj.x, dy = pi.y - pj.y;
-                            float r2 = fmaf(dy, dy, dx * dx);
-                            if (DIMS == 3) {
-                                const float dz = pi.z - pj.z;
-                                r2 = fmaf(dz, dz, r2);
-                            }
-                            if (r2 < kp.r2_thresh && r2 > 0.0f)
-                                force_pair<DIMS>(pi, vi, inv_rho_i, pj, ld_phase<COH>(rv + j), kp.h, acc);
-                        }
+#pragma unroll
+                    for (uint32_t k = 0; k < LIST_AHEAD; ++k) {
+                        if (k0 + 8u * k >= n) break;
+                        entry(ch[k] & 0xFFFFu);
+                        if (k0 + 8u * k + 1u < n) entry(ch[k] >> 16);
                     }
+                }
+            } else {
+                for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
+                    const uint32_t cnt = U.off[i + 1] - U.off[i], first = U.cell[i].x;
+                    for (uint32_t j = l; j < cnt; j += 4u) both(ld_phase<COH>(spos + first + j), ld_phase<COH>(svel + first + j));
+                }
+            }
+            // pressure and viscosity terms together, then the sums over the pair's lanes
+            float f[2][3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                f[0][k] = fmaf(kp.cpress, accA[k], cvisc * accA[3 + k]);
+                f[1][k] = fmaf(kp.cpress, accB[k], cvisc * accB[3 + k]);
+#pragma unroll
+                for (uint32_t m = 1; m < 4u; m <<= 1) {
+                    f[0][k] += __shfl_xor_sync(0xffffffffu, f[0][k], m);
+                    f[1][k] += __shfl_xor_sync(0xffffffffu, f[1][k], m);
                 }
             }
             if (staged) {
-                // Targets of a staged brick whose sub-lists overflowed: the whole warp scans
-                // each one's rows in turn (lane l takes candidates l, l + 32, ... of every
-                // row) and the sum goes to the target's first lane.
-                uint32_t pend = __ballot_sync(0xffffffffu, active && scan && p == 0);
+                // pairs without a list: the whole warp scans each one's window in turn
+                uint32_t pend = __ballot_sync(0xffffffffu, t.live && scan && l == 0u);
                 while (pend) {
-                    const int src = __ffs(pend) - 1;
+                    const int src = __ffs((int)pend) - 1;
                     pend &= pend - 1u;
-                    const float4 ps = make_float4(__shfl_sync(0xffffffffu, pi.x, src), __shfl_sync(0xffffffffu, pi.y, src),
-                                                  __shfl_sync(0xffffffffu, pi.z, src), __shfl_sync(0xffffffffu, pi.w, src));
-                    const float4 vs = make_float4(__shfl_sync(0xffffffffu, vi.x, src), __shfl_sync(0xffffffffu, vi.y, src),
-                                                  __shfl_sync(0xffffffffu, vi.z, src), __shfl_sync(0xffffffffu, vi.w, src));
-                    const uint32_t cs = __shfl_sync(0xffffffffu, c, src);
-                    float a[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    const uint32_t self = __shfl_sync(0xffffffffu, t.self, src), lo = __shfl_sync(0xffffffffu, t.lo, src),
+                                   len = __shfl_sync(0xffffffffu, t.len, src), more = __shfl_sync(0xffffffffu, two, src);
 #pragma unroll 1
-                    for (int r = 0; r < R; ++r) {
-                        const float4* rp = s_pos + S.base[r];
-                        const float4* rv = s_vel + S.base[r];
-                        const uint32_t hi = S.off[r][cs + 3];
-                        for (uint32_t j = S.off[r][cs] + (uint32_t)lane; j < hi; j += 32) {
-                            const float4 pj = rp[j];
-                            const float dx = ps.x - pj.x, dy = ps.y - pj.y;
-                            float r2 = fmaf(dy, dy, dx * dx);
-                            if (DIMS == 3) {
-                                const float dz = ps.z - pj.z;
-                                r2 = fmaf(dz, dz, r2);
+                    for (uint32_t w = 0; w <= more; ++w) {
+                        const float4 ps = s_pos[self + w], vs = s_vel[self + w];
+                        const float as = rcp_approx(ps.w);
+                        float a[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                        for (uint32_t j = lo + lane; j < lo + len; j += 32u)
+                            force_pair<DIMS>(ps, vs, as, s_pos[j], s_vel[j], rcp_approx(s_pos[j].w), kp.h, thr, a);
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            float x = fmaf(kp.cpress, a[k], cvisc * a[3 + k]);
+                            for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+                            if ((lane >> 2) == (uint32_t)src >> 2) {
+                                if (w) f[1][k] = x;
+                                else f[0][k] = x;
                             }
-                            if (r2 < kp.r2_thresh) force_pair_pre<DIMS>(ps, vs, pj, rv[j], kp.h, a);
                         }
-                    }
-                    for (int m = 16; m > 0; m >>= 1) {
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) a[k] += __shfl_xor_sync(0xffffffffu, a[k], m);
-                    }
-                    if (lane == src) {
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) acc[k] = a[k];
                     }
                 }
             }
-            for (uint32_t m = P >> 1; m > 0; m >>= 1) {
+            // lane l takes component l, target A and then target B
+            const float g = l == 0u ? kp.gravity.x : (l == 1u ? kp.gravity.y : (l == 2u ? kp.gravity.z : kp.gravity.w));
 #pragma unroll
-                for (int k = 0; k < 6; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], m);
-            }
-            if (active && p == 0) {
-                float4 fs = f_o;
-                const float cvisc = S.cvisc;
-                fs.x = __fadd_rn(fs.x, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, acc[0]), __fmul_rn(cvisc, acc[3])), kp.mass));
-                fs.y = __fadd_rn(fs.y, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, acc[1]), __fmul_rn(cvisc, acc[4])), kp.mass));
-                fs.z = __fadd_rn(fs.z, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, acc[2]), __fmul_rn(cvisc, acc[5])), kp.mass));
-                fs.w = 0.0f;
+            for (int w = 0; w < 2; ++w) {
+                const bool live = t.live && (w == 0 || t.two);
+                const uint32_t o = w ? oB : oA;
+                const float add = l == 0u ? f[w][0] : (l == 1u ? f[w][1] : f[w][2]);
+                float F = l == 3u ? 0.0f : __fadd_rn(w ? f_B : f_A, __fmul_rn(add, kp.mass));
                 if (FUSED) {
-                    fs = clip_box_force(kp, S.box_min, S.box_max, pi, vi, fs);
-                    if (kp.rec_force) kp.rec_force[o] = fs;
-                    const float4 v = integrate_force(kp, v_o, fs);
-                    vel[o] = v;
-                    force[o] = kp.gravity;
-                    pos[o] = integrate_velocity(kp, p_o, v);
-                } else {
-                    force[o] = fs;
+                    F = clip_box_lane<DIMS>(kp, U.box_min, U.box_max, w ? pB : pA, w ? vB : vA, F, l, live);
+                    if (kp.rec_force && live) reinterpret_cast<float*>(kp.rec_force + o)[l] = F;
+                    const float v = integrate_force_lane(kp, w ? v_B : v_A, F);
+                    if (live) {
+                        reinterpret_cast<float*>(vel + o)[l] = v;
+                        reinterpret_cast<float*>(force + o)[l] = g;
+                        reinterpret_cast<float*>(pos + o)[l] = __fadd_rn(w ? p_B : p_A, __fmul_rn(v, kp.dt));
+                    }
+                } else if (live) {
+                    reinterpret_cast<float*>(force + o)[l] = F;
                 }
             }
         }
-        __syncthreads();  // every warp is done with the brick before the next one's set-up
+        turn -= tasks;
+        unit_release(S, use);
     }
     return true;
 }
 
 template <int DIMS, bool FUSED, bool BATCH>
-__global__ void __launch_bounds__(BRICK_THREADS, 3) k_force_brick(const float4* __restrict__ spos,
+__global__ void __launch_bounds__(32 * FORCE_CONSUMERS + 32, FORCE_CTAS) k_force_brick(const float4* __restrict__ spos,
                                                                const float4* __restrict__ svel,
                                                                const uint32_t* __restrict__ index,
                                                                float4* __restrict__ pos,
@@ -1343,13 +1311,12 @@ __global__ void __launch_bounds__(BRICK_THREADS, 3) k_force_brick(const float4* 
                                                                const uint32_t* __restrict__ bricks,
                                                                uint32_t* counters, KParams kp,
                                                                const uint16_t* __restrict__ nbr,
-                                                               const uint64_t* __restrict__ nbr_meta,
+                                                               const uint32_t* __restrict__ nbr_meta,
                                                                uint32_t* err) {
     extern __shared__ float4 s_buf[];
-    __shared__ BrickShared S[2];
-    __shared__ LaneMap L;
-    force_brick_run<DIMS, FUSED, BATCH>(s_buf, S, L, spos, svel, index, pos, vel, force, table, bricks, counters, kp,
-                                        nbr, nbr_meta, err);
+    __shared__ BrickShared S;
+    force_brick_run<DIMS, FUSED, BATCH>(s_buf, S, spos, svel, index, pos, vel, force, table, bricks, counters, kp, nbr,
+                                        nbr_meta, err);
 }
 
 }  // namespace gbsph

@@ -110,4 +110,11 @@ cudaError_t cell_bounds_launch(const uint32_t* sorted_keys, uint32_t n, uint32_t
 
 int num_sms();
 
+// Smallest float x >= 0 with sqrtf(x) >= h (common.cu). sqrtf is correctly rounded and monotone, so
+// for every float r2 >= 0: (sqrtf(r2) < h) == (r2 < r2_threshold(h)).
+float r2_threshold(float h);
+// Smallest float x >= 0 with sqrtf(x) > v, or NaN where there is none: (sqrtf(f2) > v) ==
+// (f2 >= v2_threshold(v)) for every float f2 >= 0 and for NaN.
+float v2_threshold(float v);
+
 }  // namespace gbsph
