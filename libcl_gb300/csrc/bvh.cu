@@ -2,8 +2,8 @@
 // (libCL/geom/oclBvhTrimesh.h:20-84, libCL/geom/oclBvhTrimesh.cpp:56-143,
 // libCL/geom/oclBvhTrimesh.cl:33-298), the reference's second user of the radix sort; and its
 // 2D sibling over line segments, the oclBvhLines replacement (libCL/geom/oclBvhLines.h:20-77,
-// libCL/geom/oclBvhLines.cpp:48-115, libCL/geom/oclBvhLines.cl:27-245), which shares the node
-// creation, linking, leaves and parent links (templated on the node type).
+// libCL/geom/oclBvhLines.cpp:48-115, libCL/geom/oclBvhLines.cl:27-245), which shares the tree
+// kernel (templated on the node type).
 //
 // One build, in the reference's order:
 //   global bounding box (accumulated into the handle's box, which starts at zero and is never
@@ -12,11 +12,12 @@
 //   gets the highest bit (29..0) where keys i and i+1 differ -> each internal node links to
 //   the nearer of its nearest left / right nodes with a higher bit (the one with the lower
 //   bit; the root has neither) -> leaves take the free child slots -> boxes bottom-up.
-// The reference finds the higher-bit neighbours by a linear scan per node and computes the
-// boxes by one root-to-leaf descent per triangle with a visit flag per node. Here the scans
-// skip 64- and 4096-node blocks by their maximum bit (same answer, bounded work) and the
-// boxes are refitted bottom-up from parent links with a visit counter per node; min and max
-// are evaluated with the reference's operand order, so every box is bit-identical.
+// The reference makes a pass of each of the last three, finds the higher-bit neighbours by a
+// linear scan per node and computes the boxes by one root-to-leaf descent per triangle with a
+// visit flag per node. Here one kernel (k_bvh_tree) climbs from the leaves: a subtree that
+// covers the sorted leaves [a, b] hangs on node a - 1 or node b, whichever has the lower bit, so
+// links, boxes and records are written once, without any search; min and max are evaluated with
+// the reference's operand order, so every box is bit-identical.
 #include <algorithm>
 #include <cfloat>
 #include <string>
@@ -29,7 +30,6 @@ using namespace gbsph;
 namespace {
 
 constexpr int BVH_THREADS = 256;
-constexpr uint32_t BLK = 64, SBLK = 4096;  // scan-skipping block sizes (SBLK = BLK * BLK)
 
 // OpenCL's min / max of floats: min(x, y) = y < x ? y : x, max(x, y) = x < y ? y : x.
 __device__ __forceinline__ float cl_min(float x, float y) { return y < x ? y : x; }
@@ -59,17 +59,74 @@ __device__ __forceinline__ uint32_t spread16(uint32_t x) {
     return x;
 }
 
-// Empty boxes of clCreateNodes: +-MAXFLOAT in the coordinate lanes (w = 0 for triangles).
-__device__ __forceinline__ void box_init(gbsph_bvh_node& nd) {
-    nd.bbMin[0] = nd.bbMin[1] = nd.bbMin[2] = FLT_MAX;
-    nd.bbMin[3] = 0.f;
-    nd.bbMax[0] = nd.bbMax[1] = nd.bbMax[2] = -FLT_MAX;
-    nd.bbMax[3] = 0.f;
-}
-__device__ __forceinline__ void box_init(gbsph_bvh2d_node& nd) {
-    nd.bbMin[0] = nd.bbMin[1] = FLT_MAX;
-    nd.bbMax[0] = nd.bbMax[1] = -FLT_MAX;
-}
+// What the tree kernel needs of a node type: its box, its records and its leaves.
+struct TriTree {  // oclBvhTrimesh: 48-byte nodes
+    using Node = gbsph_bvh_node;
+    struct Box {
+        float4 lo, hi;
+    };
+    struct Prims {
+        const uint32_t* index;
+        const float4* vertex;
+        uint32_t nv;
+    };
+    static constexpr uint32_t MASK = (1u << 30) - 1u;  // key bits that make nodes
+    static constexpr uint32_t TRAV = 2;                 // internal nodes' final flag
+    // +-MAXFLOAT in the coordinate lanes (clCreateNodes), w = 0
+    static __device__ __forceinline__ Box empty() {
+        return {make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f)};
+    }
+    static __device__ __forceinline__ Box leaf(const Prims& p, uint32_t tri) {
+        Box b = empty();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float4 v = p.vertex[min(p.index[3 * tri + k], p.nv - 1)];
+            b.lo = cl_min4(b.lo, v);
+            b.hi = cl_max4(b.hi, v);
+        }
+        return b;
+    }
+    static __device__ __forceinline__ Box merge(const Box& l, const Box& r) {
+        return {cl_min4(l.lo, r.lo), cl_max4(l.hi, r.hi)};
+    }
+    static __device__ __forceinline__ Box load(const Node* n) {  // written by another CTA: through L2
+        const float4* f = reinterpret_cast<const float4*>(n);
+        return {__ldcg(f), __ldcg(f + 1)};
+    }
+    static __device__ __forceinline__ void store(Node* n, const Box& b, int left, int right, uint32_t bit, uint32_t trav) {
+        float4* f = reinterpret_cast<float4*>(n);
+        f[0] = b.lo;
+        f[1] = b.hi;
+        reinterpret_cast<int4*>(n)[2] = make_int4(left, right, (int)bit, (int)trav);
+    }
+};
+struct SegTree {  // oclBvhLines: 32-byte nodes
+    using Node = gbsph_bvh2d_node;
+    struct Box {
+        float4 b;  // min xy, max xy
+    };
+    struct Prims {
+        const float2* vertex;
+    };
+    static constexpr uint32_t MASK = 0xFFFFFFFFu;
+    // In the reference the first visitor of a node leaves trav = 2 and the second swaps it for 3
+    // before computing the box (libCL/geom/oclBvhLines.cl:186-245).
+    static constexpr uint32_t TRAV = 3;
+    static __device__ __forceinline__ Box empty() { return {make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX)}; }
+    static __device__ __forceinline__ Box leaf(const Prims& p, uint32_t seg) {
+        const float2 v0 = p.vertex[2 * seg], v1 = p.vertex[2 * seg + 1];
+        return {make_float4(cl_min(cl_min(FLT_MAX, v0.x), v1.x), cl_min(cl_min(FLT_MAX, v0.y), v1.y),
+                            cl_max(cl_max(-FLT_MAX, v0.x), v1.x), cl_max(cl_max(-FLT_MAX, v0.y), v1.y))};
+    }
+    static __device__ __forceinline__ Box merge(const Box& l, const Box& r) {
+        return {make_float4(cl_min(l.b.x, r.b.x), cl_min(l.b.y, r.b.y), cl_max(l.b.z, r.b.z), cl_max(l.b.w, r.b.w))};
+    }
+    static __device__ __forceinline__ Box load(const Node* n) { return {__ldcg(reinterpret_cast<const float4*>(n))}; }
+    static __device__ __forceinline__ void store(Node* n, const Box& b, int left, int right, uint32_t bit, uint32_t trav) {
+        reinterpret_cast<float4*>(n)[0] = b.b;
+        reinterpret_cast<int4*>(n)[1] = make_int4(left, right, (int)bit, (int)trav);
+    }
+};
 
 // Per-block min / max of the vertices (all four lanes), combined with the handle's box by the
 // last block to finish (clAABB, libCL/geom/oclBvhTrimesh.cl:33-76).
@@ -101,18 +158,29 @@ __global__ void __launch_bounds__(BVH_THREADS) k_bvh_box(const float4* __restric
         last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        const volatile float4* vp = part;  // written by other blocks: read past L1
-        float4 a = box[0], b = box[1];
-        for (uint32_t k = 0; k < gridDim.x; ++k) {
-            const float4 lo = make_float4(vp[2 * k].x, vp[2 * k].y, vp[2 * k].z, vp[2 * k].w);
-            const float4 hi = make_float4(vp[2 * k + 1].x, vp[2 * k + 1].y, vp[2 * k + 1].z, vp[2 * k + 1].w);
-            a = cl_min4(a, lo);
-            b = cl_max4(b, hi);
+    if (!last) return;
+    // the partial boxes by all threads of the last block (min and max of numbers do not depend on
+    // the order); one thread reading 257 of them in turn took 40 of the kernel's 48 us
+    __threadfence();
+    mn = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f);
+    mx = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
+    for (uint32_t k = threadIdx.x; k < gridDim.x; k += BVH_THREADS) {  // written by other blocks: past L1
+        mn = cl_min4(mn, __ldcg(part + 2 * k));
+        mx = cl_max4(mx, __ldcg(part + 2 * k + 1));
+    }
+    smin[threadIdx.x] = mn;
+    smax[threadIdx.x] = mx;
+    __syncthreads();
+    for (int s = BVH_THREADS / 2; s > 0; s >>= 1) {
+        if ((int)threadIdx.x < s) {
+            smin[threadIdx.x] = cl_min4(smin[threadIdx.x], smin[threadIdx.x + s]);
+            smax[threadIdx.x] = cl_max4(smax[threadIdx.x], smax[threadIdx.x + s]);
         }
-        box[0] = a;
-        box[1] = b;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        box[0] = cl_min4(box[0], smin[0]);
+        box[1] = cl_max4(box[1], smax[0]);
         *done = 0;
     }
 }
@@ -153,212 +221,147 @@ __global__ void __launch_bounds__(BVH_THREADS) k_bvh_morton_lines(const float2* 
     val[g] = g;
 }
 
-// clCreateNodes (libCL/geom/oclBvhTrimesh.cl:119-143, libCL/geom/oclBvhLines.cl:71-95): the
-// highest bit, of bits [0, TOP], where sorted keys i and i + 1 differ; and the block maxima of
-// the bits.
-template <class Node, int TOP>
-__global__ void __launch_bounds__(BVH_THREADS) k_bvh_nodes(const uint32_t* __restrict__ key, uint32_t m,
-                                                           Node* __restrict__ node,
-                                                           uint8_t* __restrict__ bits, uint8_t* __restrict__ bmax) {
-    constexpr uint32_t MASK = TOP == 31 ? 0xFFFFFFFFu : (1u << (TOP + 1)) - 1u;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t bit = 0;
-    if (i < m) {
-        const uint32_t d = (key[i] ^ key[i + 1]) & MASK;
-        bit = d ? 31u - (uint32_t)__clz(d) : 0u;
-        Node nd;
-        box_init(nd);
-        nd.left = nd.right = -1;
-        nd.bit = bit;
-        nd.trav = 0;
-        node[i] = nd;
-        bits[i] = (uint8_t)bit;
+__device__ __forceinline__ unsigned long long exch_acq_rel(unsigned long long* p, unsigned long long v) {
+    unsigned long long o;
+    asm volatile("atom.acq_rel.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(o) : "l"(p), "l"(v) : "memory");
+    return o;
+}
+
+// Nodes, links, leaves and boxes (clCreateNodes, clLinkNodes, clCreateLeaves, clComputeAABBs:
+// libCL/geom/oclBvhTrimesh.cl:119-298, libCL/geom/oclBvhLines.cl:71-245) in one climb. A thread
+// starts with sorted leaf g; a subtree over the leaves [a, b] is the right child of node a - 1 or
+// the left child of node b, whichever has the lower bit (node b at equal bits); the first of a
+// node's two children to arrive leaves its box, its far end and its id and stops, the second
+// writes the node's record and goes on with the two ranges joined. The subtree over all leaves
+// is the root.
+//
+// Bits above 0 cannot tie (between two nodes with the same highest differing bit the keys must
+// fall back, which makes a higher one). Bit 0 ties where keys repeat: of a run of nodes with
+// bit 0, all of which claim the same slot in the reference, the last one holds it (as in a
+// sequential run of the reference's work-items) and the others keep their left leaf, an empty
+// box and no parent; the last one's subtree then stands in for the whole run, whose first leaf is
+// the first key of the same value above bit 0.
+//
+// Nodes of the CTA's own range meet in shared memory; a child whose sibling did not come there,
+// and subtrees that leave the range, go on through one 64-bit exchange per node in `link` (all
+// ones before the launch). 1.05M triangles: 130 us, of which about 40 are the last subtrees'
+// climb through the top levels, an exchange and a box at a time (16,640 triangles: 30 us); 64 to
+// 256 leaves per CTA are alike, 512 and 1024 slower. Six kernels did this before (node records with
+// empty boxes, block maxima, a neighbour search per node, leaves, parent links, a climb with a
+// counter, two fences and 24 scalar loads per node): 415 us.
+constexpr int TREE_THREADS = 128;
+
+template <class T>
+__global__ void __launch_bounds__(TREE_THREADS) k_bvh_tree(const uint32_t* __restrict__ key, const uint32_t* __restrict__ val,
+                                                          uint32_t n, typename T::Prims prims, typename T::Node* node,
+                                                          unsigned long long* link, uint32_t* __restrict__ root) {
+    using Box = typename T::Box;
+    __shared__ uint32_t s_key[TREE_THREADS + 2];  // keys base - 1 ... base + 256
+    __shared__ Box s_box[2][TREE_THREADS];         // a node's left and right child
+    __shared__ uint2 s_end[2][TREE_THREADS];       // their far ends and ids
+    __shared__ uint32_t s_came[TREE_THREADS];      // bit 0: left, bit 1: right
+    const uint32_t t = threadIdx.x, base = blockIdx.x * TREE_THREADS, g = base + t, ls = n - 1u;
+    for (uint32_t k = t; k < TREE_THREADS + 2; k += TREE_THREADS) {
+        const uint32_t i = base + k - 1u;  // wraps for the first key of the first CTA
+        s_key[k] = i < n ? key[i] : 0u;
     }
-    // maximum bit of each 64-node block (blocks of 256 threads hold 4 of them)
-    uint32_t v = i < m ? bit : 0u;
-    for (int s = 16; s > 0; s >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, s));
-    __shared__ uint32_t w[BVH_THREADS / 32];
-    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = v;
+    s_came[t] = 0u;
     __syncthreads();
-    if (threadIdx.x < BVH_THREADS / BLK) {
-        const uint32_t b = (blockIdx.x * BVH_THREADS) / BLK + threadIdx.x;
-        if (b * BLK < m) bmax[b] = (uint8_t)max(w[2 * threadIdx.x], w[2 * threadIdx.x + 1]);
-    }
-}
-
-// Maximum bit of each 4096-node super-block.
-__global__ void k_bvh_smax(const uint8_t* __restrict__ bmax, uint32_t nb, uint8_t* __restrict__ smax) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s * (SBLK / BLK) >= nb) return;
-    uint8_t v = 0;
-    for (uint32_t b = s * (SBLK / BLK); b < min(nb, (s + 1) * (SBLK / BLK)); ++b) v = max(v, bmax[b]);
-    smax[s] = v;
-}
-
-// Nearest node left of i (dir < 0) or right of i (dir > 0) whose bit exceeds `bit`, or -1:
-// element steps inside a block, block steps inside a super-block, then super-block steps.
-__device__ int nearest_higher(const uint8_t* __restrict__ bits, const uint8_t* __restrict__ bmax,
-                              const uint8_t* __restrict__ smax, int m, int i, int dir, uint32_t bit) {
-    int j = i + dir;
-    while (j >= 0 && j < m) {
-        if ((j % (int)BLK) == (dir > 0 ? 0 : (int)BLK - 1) && bmax[j / BLK] <= bit) {
-            // skip this block; at a super-block boundary, skip super-blocks too
-            if ((j % (int)SBLK) == (dir > 0 ? 0 : (int)SBLK - 1)) {
-                int sb = j / (int)SBLK;
-                while (sb >= 0 && sb * (int)SBLK < m && smax[sb] <= bit) sb += dir;
-                if (sb < 0 || sb * (int)SBLK >= m) return -1;
-                j = dir > 0 ? sb * (int)SBLK : min(m - 1, sb * (int)SBLK + (int)SBLK - 1);
-                if ((j % (int)BLK) != (dir > 0 ? 0 : (int)BLK - 1) || bmax[j / BLK] > bit) continue;
-            }
-            j += dir * (int)BLK;
-            continue;
+    auto key_at = [&](uint32_t i) -> uint32_t {
+        const uint32_t k = i - base + 1u;
+        return (k < TREE_THREADS + 2 ? s_key[k] : __ldg(key + i)) & T::MASK;
+    };
+    // Highest bit in which keys i and i + 1 differ; NO_NODE before the first and after the last leaf.
+    constexpr uint32_t NO_NODE = 64u;
+    auto bit_of = [&](uint32_t i) -> uint32_t {
+        if (i >= ls) return NO_NODE;
+        const uint32_t d = key_at(i) ^ key_at(i + 1u);
+        return d ? 31u - (uint32_t)__clz((int)d) : 0u;
+    };
+    // A subtree: its leaves [a, b], its node c, the bits of the nodes a - 1 and b beside it.
+    uint32_t a = g, b = g, c = ls + g, bl = NO_NODE, br = NO_NODE;
+    Box box{};
+    // Joins this thread's subtree with its sibling (node oc, far end oe, box ob) under node p; side:
+    // the thread's is the right child. Writes p's record; false: p is the root.
+    auto join = [&](uint32_t p, uint32_t side, uint32_t oc, uint32_t oe, const Box& ob) -> bool {
+        const uint32_t bit = side ? bl : br;
+        const uint32_t far = bit_of(side ? oe - 1u : oe);
+        box = side ? T::merge(ob, box) : T::merge(box, ob);
+        T::store(node + p, box, (int)(side ? oc : c), (int)(side ? c : oc), bit, T::TRAV);
+        c = p;
+        if (side) {
+            a = oe;
+            bl = far;
+        } else {
+            b = oe;
+            br = far;
         }
-        if (bits[j] > bit) return j;
-        j += dir;
-    }
-    return -1;
-}
+        if (bit == 0u && bl == 0u) {  // a run of repeated keys: its first leaf
+            const uint32_t k = key_at(p) >> 1;
+            uint32_t lo = 0u, hi = a - 1u;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (key_at(mid) >> 1 < k) lo = mid + 1u;
+                else hi = mid;
+            }
+            a = lo;
+            bl = bit_of(a - 1u);
+        }
+        if (bl == NO_NODE && br == NO_NODE) {
+            *root = p;
+            return false;
+        }
+        return true;
+    };
 
-// clLinkNodes (libCL/geom/oclBvhTrimesh.cl:145-199, libCL/geom/oclBvhLines.cl:97-151).
-// Several nodes can only claim the same slot (or the root) when sorted keys repeat (their
-// bits are then 0); the largest claimant wins here, as in a sequential run of the
-// reference's work-items.
-template <class Node>
-__global__ void __launch_bounds__(BVH_THREADS) k_bvh_link(const uint8_t* __restrict__ bits,
-                                                          const uint8_t* __restrict__ bmax,
-                                                          const uint8_t* __restrict__ smax, int m,
-                                                          Node* __restrict__ node,
-                                                          uint32_t* __restrict__ root) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const uint32_t bit = bits[i];
-    const int l = nearest_higher(bits, bmax, smax, m, i, -1, bit);
-    const int r = nearest_higher(bits, bmax, smax, m, i, +1, bit);
-    if (l < 0 && r < 0) {
-        atomicMax(root, (uint32_t)i);  // one root unless keys repeat; then the last, as a sequential run
-    } else if (r < 0 || (l >= 0 && bits[l] < bits[r])) {
-        atomicMax(&node[l].right, i);
-    } else {
-        atomicMax(&node[r].left, i);
+    bool carry = g < n;
+    if (carry) {
+        const uint32_t prim = val[g];
+        bl = bit_of(g - 1u);
+        br = bit_of(g);
+        box = T::leaf(prims, prim);
+        T::store(node + c, box, 0, 0, prim, 0u);
+        // a node that lost its slot to the last of its run
+        if (br == 0u && bit_of(g + 1u) == 0u) T::store(node + g, T::empty(), (int)c, -1, 0u, 0u);
+        for (;;) {
+            const uint32_t side = bl < br ? 1u : 0u, p = side ? a - 1u : b, i = p - base;
+            if (i >= TREE_THREADS) break;  // not a node of this CTA
+            s_box[side][i] = box;
+            s_end[side][i] = make_uint2(side ? b : a, c);
+            __threadfence_block();
+            carry = atomicOr(&s_came[i], 1u << side) != 0u;
+            if (!carry) break;
+            __threadfence_block();
+            const uint2 o = s_end[side ^ 1u][i];
+            carry = join(p, side, o.y, o.x, s_box[side ^ 1u][i]);
+            if (!carry) break;
+        }
     }
-}
-
-// clCreateLeaves (libCL/geom/oclBvhTrimesh.cl:201-234, libCL/geom/oclBvhLines.cl:153-184):
-// leaf n-1+g holds primitive val[g] in .bit and takes the free slot between internal nodes
-// g-1 and g. (The leaf's box is written by the box pass.)
-template <class Node>
-__global__ void __launch_bounds__(BVH_THREADS) k_bvh_leaves(const uint32_t* __restrict__ val, uint32_t n,
-                                                            Node* __restrict__ node) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    const uint32_t ls = n - 1, L = ls + g;
-    Node nd;
-    box_init(nd);
-    nd.left = nd.right = 0;
-    nd.bit = val[g];
-    nd.trav = 0;
-    node[L] = nd;
-    if (g == 0) {
-        node[0].left = (int32_t)L;
-    } else if (g == ls) {
-        node[ls - 1].right = (int32_t)L;
-    } else if (node[g].left == -1) {
-        node[g].left = (int32_t)L;
-    } else if (node[g - 1].right == -1) {
-        node[g - 1].right = (int32_t)L;
-    }
-}
-
-// Parent links from the child slots, and the visit counters cleared.
-template <class Node>
-__global__ void __launch_bounds__(BVH_THREADS) k_bvh_parents(const Node* __restrict__ node, uint32_t m,
-                                                             int32_t* __restrict__ parent,
-                                                             uint32_t* __restrict__ visits) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int32_t l = node[i].left, r = node[i].right;
-    if (l >= 0) parent[l] = (int32_t)i;
-    if (r >= 0) parent[r] = (int32_t)i;
-    visits[i] = 0;
-}
-
-// Boxes (clComputeAABBs, libCL/geom/oclBvhTrimesh.cl:236-298): each leaf's box from its
-// triangle; the second of a node's two children to arrive computes the node's box as
-// min(left, right) / max(left, right) and goes on up; internal nodes end with trav = 2.
-__global__ void __launch_bounds__(BVH_THREADS) k_bvh_refit(const uint32_t* __restrict__ index,
-                                                           const float4* __restrict__ vertex, uint32_t n, uint32_t nv,
-                                                           gbsph_bvh_node* node, const int32_t* __restrict__ parent,
-                                                           uint32_t* visits, const uint32_t* __restrict__ root) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    const uint32_t L = n - 1 + g;
-    const uint32_t tri = node[L].bit;
-    float4 mn = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), mx = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
-    for (int k = 0; k < 3; ++k) {
-        const float4 v = vertex[min(index[3 * tri + k], nv - 1)];
-        mn = cl_min4(mn, v);
-        mx = cl_max4(mx, v);
-    }
-    *reinterpret_cast<float4*>(node[L].bbMin) = mn;
-    *reinterpret_cast<float4*>(node[L].bbMax) = mx;
-    const uint32_t rt = *root;
-    int32_t c = (int32_t)L;
-    for (uint32_t depth = 0; depth < 2 * n && (uint32_t)c != rt; ++depth) {
-        const int32_t p = parent[c];
-        if (p < 0) return;  // not reachable from the root (repeated keys)
-        __threadfence();
-        if (atomicAdd(&visits[p], 1u) == 0) return;  // the other child is not done yet
-        __threadfence();
-        const volatile gbsph_bvh_node* vn = node;
-        const int32_t l = vn[p].left, r = vn[p].right;
-        float4 a, b;
-        a.x = cl_min(vn[l].bbMin[0], vn[r].bbMin[0]);
-        a.y = cl_min(vn[l].bbMin[1], vn[r].bbMin[1]);
-        a.z = cl_min(vn[l].bbMin[2], vn[r].bbMin[2]);
-        a.w = cl_min(vn[l].bbMin[3], vn[r].bbMin[3]);
-        b.x = cl_max(vn[l].bbMax[0], vn[r].bbMax[0]);
-        b.y = cl_max(vn[l].bbMax[1], vn[r].bbMax[1]);
-        b.z = cl_max(vn[l].bbMax[2], vn[r].bbMax[2]);
-        b.w = cl_max(vn[l].bbMax[3], vn[r].bbMax[3]);
-        *reinterpret_cast<float4*>(node[p].bbMin) = a;
-        *reinterpret_cast<float4*>(node[p].bbMax) = b;
-        node[p].trav = 2;
-        c = p;
-    }
-}
-
-// Boxes of oclBvhLines (clComputeAABBs, libCL/geom/oclBvhLines.cl:186-245): each leaf's box
-// from its segment's two vertices; the second of a node's two children to arrive computes
-// min(left, right) / max(left, right) and goes on up. In the reference the first visitor
-// leaves trav = 2 and the second swaps it for 3 before computing, so internal nodes end with
-// trav = 3.
-__global__ void __launch_bounds__(BVH_THREADS) k_bvh_refit_lines(const float2* __restrict__ vertex, uint32_t n,
-                                                                 gbsph_bvh2d_node* node,
-                                                                 const int32_t* __restrict__ parent,
-                                                                 uint32_t* visits, const uint32_t* __restrict__ root) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    const uint32_t L = n - 1 + g;
-    const uint32_t seg = node[L].bit;
-    const float2 v0 = vertex[2 * seg], v1 = vertex[2 * seg + 1];
-    const float2 mn = make_float2(cl_min(cl_min(FLT_MAX, v0.x), v1.x), cl_min(cl_min(FLT_MAX, v0.y), v1.y));
-    const float2 mx = make_float2(cl_max(cl_max(-FLT_MAX, v0.x), v1.x), cl_max(cl_max(-FLT_MAX, v0.y), v1.y));
-    *reinterpret_cast<float4*>(node[L].bbMin) = make_float4(mn.x, mn.y, mx.x, mx.y);
-    const uint32_t rt = *root;
-    int32_t c = (int32_t)L;
-    for (uint32_t depth = 0; depth < 2 * n && (uint32_t)c != rt; ++depth) {
-        const int32_t p = parent[c];
-        if (p < 0) return;  // not reachable from the root (repeated keys)
-        __threadfence();
-        if (atomicAdd(&visits[p], 1u) == 0) return;  // the other child is not done yet
-        __threadfence();
-        const volatile gbsph_bvh2d_node* vn = node;
-        const int32_t l = vn[p].left, r = vn[p].right;
-        const float4 box = make_float4(cl_min(vn[l].bbMin[0], vn[r].bbMin[0]), cl_min(vn[l].bbMin[1], vn[r].bbMin[1]),
-                                       cl_max(vn[l].bbMax[0], vn[r].bbMax[0]), cl_max(vn[l].bbMax[1], vn[r].bbMax[1]));
-        *reinterpret_cast<float4*>(node[p].bbMin) = box;
-        node[p].trav = 3;
-        c = p;
+    __syncthreads();
+    // Subtrees go on through global memory: this thread's own, then the lone child of its node.
+    const uint32_t lone = s_came[t];
+    for (int round = 0; round < 2; ++round) {
+        if (round == 1) {
+            carry = lone == 1u || lone == 2u;
+            if (carry) {
+                const uint32_t side = lone >> 1;
+                const uint2 e = s_end[side][t];
+                box = s_box[side][t];
+                c = e.y;
+                a = side ? g + 1u : e.x;
+                b = side ? e.x : g;
+                bl = bit_of(a - 1u);
+                br = bit_of(b);
+            }
+        }
+        while (carry) {
+            const uint32_t side = bl < br ? 1u : 0u, p = side ? a - 1u : b;
+            // the exchange releases the subtree's records (also those that other threads of the CTA
+            // wrote before the barrier) and acquires its sibling's
+            const unsigned long long o = exch_acq_rel(link + p, (unsigned long long)(side ? b : a) << 32 | c);
+            if (o == ~0ull) break;  // the sibling is not there yet
+            carry = join(p, side, (uint32_t)o, (uint32_t)(o >> 32), T::load(node + (uint32_t)o));
+        }
     }
 }
 
@@ -373,9 +376,8 @@ struct gbsph_bvh_s {
     uint32_t n = 0;    // triangles of the last build
     void* block = nullptr;
     gbsph_bvh_node* node = nullptr;
-    uint32_t *key = nullptr, *val = nullptr, *visits = nullptr, *root = nullptr, *err = nullptr, *done = nullptr;
-    int32_t* parent = nullptr;
-    uint8_t *bits = nullptr, *bmax = nullptr, *smax = nullptr;
+    uint32_t *key = nullptr, *val = nullptr, *root = nullptr, *err = nullptr, *done = nullptr;
+    unsigned long long* link = nullptr;  // per internal node: the first child to arrive
     float4* box = nullptr;   // [min, max], persists across builds
     float4* part = nullptr;  // per-block partial boxes
     std::string last_error;
@@ -390,9 +392,8 @@ int ensure(gbsph_bvh_s* h, uint32_t n) {
     if (h->block) cudaFree(h->block);
     h->block = nullptr;
     const size_t nn = 2 * (size_t)n, m = n;
-    const size_t nb = (m + BLK - 1) / BLK, ns = (m + SBLK - 1) / SBLK;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t bytes = al(nn * sizeof(gbsph_bvh_node)) + 3 * al(m * 4) + al(nn * 4) + al(m) + al(nb) + al(ns) + 256;
+    const size_t bytes = al(nn * sizeof(gbsph_bvh_node)) + 2 * al(m * 4) + al(m * 8);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->block, bytes));
     char* p = (char*)h->block;
     h->node = (gbsph_bvh_node*)p;
@@ -401,15 +402,7 @@ int ensure(gbsph_bvh_s* h, uint32_t n) {
     p += al(m * 4);
     h->val = (uint32_t*)p;
     p += al(m * 4);
-    h->visits = (uint32_t*)p;
-    p += al(m * 4);
-    h->parent = (int32_t*)p;
-    p += al(nn * 4);
-    h->bits = (uint8_t*)p;
-    p += al(m);
-    h->bmax = (uint8_t*)p;
-    p += al(nb);
-    h->smax = (uint8_t*)p;
+    h->link = (unsigned long long*)p;
     h->cap = n;
     return GBSPH_OK;
 }
@@ -478,15 +471,8 @@ GBSPH_API int gbsph_bvh_compute(gbsph_bvh_t h, const float* vertex, size_t n_ver
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     rc = gbsph_radix_sort_compute(h->sort, h->key, h->val, n, n, 0, 32, stream);
     if (rc) return fail(&h->last_error, rc, std::string("sort: ") + gbsph_radix_sort_last_error(h->sort));
-    const uint32_t nb = (m + BLK - 1) / BLK;
-    k_bvh_nodes<gbsph_bvh_node, 29><<<grid(m), BVH_THREADS, 0, s>>>(h->key, m, h->node, h->bits, h->bmax);
-    k_bvh_smax<<<(unsigned)((nb + 255) / 256 / (SBLK / BLK) + 1), 256, 0, s>>>(h->bmax, nb, h->smax);
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->root, 0, 4, s));
-    k_bvh_link<gbsph_bvh_node><<<grid(m), BVH_THREADS, 0, s>>>(h->bits, h->bmax, h->smax, (int)m, h->node, h->root);
-    k_bvh_leaves<gbsph_bvh_node><<<grid(n), BVH_THREADS, 0, s>>>(h->val, n, h->node);
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->parent, 0xFF, (2 * (size_t)n - 1) * 4, s));
-    k_bvh_parents<gbsph_bvh_node><<<grid(m), BVH_THREADS, 0, s>>>(h->node, m, h->parent, h->visits);
-    k_bvh_refit<<<grid(n), BVH_THREADS, 0, s>>>(index, v4, n, nv, h->node, h->parent, h->visits, h->root);
+    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->link, 0xFF, (size_t)m * 8, s));
+    k_bvh_tree<TriTree><<<(n + TREE_THREADS - 1) / TREE_THREADS, TREE_THREADS, 0, s>>>(h->key, h->val, n, TriTree::Prims{index, v4, nv}, h->node, h->link, h->root);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     h->n = n;
     return GBSPH_OK;
@@ -725,9 +711,8 @@ struct gbsph_bvh_lines_s {
     uint32_t n = 0;    // segments of the last build
     void* block = nullptr;
     gbsph_bvh2d_node* node = nullptr;
-    uint32_t *key = nullptr, *val = nullptr, *visits = nullptr, *root = nullptr;
-    int32_t* parent = nullptr;
-    uint8_t *bits = nullptr, *bmax = nullptr, *smax = nullptr;
+    uint32_t *key = nullptr, *val = nullptr, *root = nullptr;
+    unsigned long long* link = nullptr;
     std::string last_error;
 };
 
@@ -739,9 +724,8 @@ int ensure_lines(gbsph_bvh_lines_s* h, uint32_t n) {
     h->block = nullptr;
     h->cap = 0;
     const size_t nn = 2 * (size_t)n, m = n;
-    const size_t nb = (m + BLK - 1) / BLK, ns = (m + SBLK - 1) / SBLK;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t bytes = al(nn * sizeof(gbsph_bvh2d_node)) + 3 * al(m * 4) + al(nn * 4) + al(m) + al(nb) + al(ns) + 256;
+    const size_t bytes = al(nn * sizeof(gbsph_bvh2d_node)) + 2 * al(m * 4) + al(m * 8) + 256;
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->block, bytes));
     char* p = (char*)h->block;
     h->node = (gbsph_bvh2d_node*)p;
@@ -750,16 +734,8 @@ int ensure_lines(gbsph_bvh_lines_s* h, uint32_t n) {
     p += al(m * 4);
     h->val = (uint32_t*)p;
     p += al(m * 4);
-    h->visits = (uint32_t*)p;
-    p += al(m * 4);
-    h->parent = (int32_t*)p;
-    p += al(nn * 4);
-    h->bits = (uint8_t*)p;
-    p += al(m);
-    h->bmax = (uint8_t*)p;
-    p += al(nb);
-    h->smax = (uint8_t*)p;
-    p += al(ns);
+    h->link = (unsigned long long*)p;
+    p += al(m * 8);
     h->root = (uint32_t*)p;
     h->cap = n;
     return GBSPH_OK;
@@ -810,15 +786,8 @@ GBSPH_API int gbsph_bvh_lines_compute(gbsph_bvh_lines_t h, const float* vertex, 
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     rc = gbsph_radix_sort_compute(h->sort, h->key, h->val, n, n, 0, 32, stream);
     if (rc) return fail(&h->last_error, rc, std::string("sort: ") + gbsph_radix_sort_last_error(h->sort));
-    const uint32_t nb = (m + BLK - 1) / BLK;
-    k_bvh_nodes<gbsph_bvh2d_node, 31><<<grid(m), BVH_THREADS, 0, s>>>(h->key, m, h->node, h->bits, h->bmax);
-    k_bvh_smax<<<(unsigned)((nb + 255) / 256 / (SBLK / BLK) + 1), 256, 0, s>>>(h->bmax, nb, h->smax);
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->root, 0, 4, s));
-    k_bvh_link<gbsph_bvh2d_node><<<grid(m), BVH_THREADS, 0, s>>>(h->bits, h->bmax, h->smax, (int)m, h->node, h->root);
-    k_bvh_leaves<gbsph_bvh2d_node><<<grid(n), BVH_THREADS, 0, s>>>(h->val, n, h->node);
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->parent, 0xFF, (2 * (size_t)n - 1) * 4, s));
-    k_bvh_parents<gbsph_bvh2d_node><<<grid(m), BVH_THREADS, 0, s>>>(h->node, m, h->parent, h->visits);
-    k_bvh_refit_lines<<<grid(n), BVH_THREADS, 0, s>>>(v2, n, h->node, h->parent, h->visits, h->root);
+    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->link, 0xFF, (size_t)m * 8, s));
+    k_bvh_tree<SegTree><<<(n + TREE_THREADS - 1) / TREE_THREADS, TREE_THREADS, 0, s>>>(h->key, h->val, n, SegTree::Prims{v2}, h->node, h->link, h->root);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     h->n = n;
     return GBSPH_OK;
