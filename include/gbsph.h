@@ -482,8 +482,8 @@ GBSPH_API const char* gbsph_bvh_last_error(gbsph_bvh_t h);
  * first triangle the particle's next displacement crosses within particleRadius; that
  * particle's position, velocity and force (device float4[n_particles]) are then updated as
  * the reference does. Uses deltaTime, particleRadius, pressureConstant, density, cellSize and
- * mass of `params`; `vertex` / `index` are the mesh the BVH was built from. Reads the root
- * back (synchronises `stream` once), then runs asynchronously. */
+ * mass of `params`; `vertex` / `index` are the mesh the BVH was built from. Asynchronous on
+ * `stream`. */
 GBSPH_API int gbsph_bvh_collide(gbsph_bvh_t h, const gbsph_fluid3d_params* params, float* position,
                                 float* velocity, float* force, size_t n_particles, const float* vertex,
                                 size_t n_vertices, const uint32_t* index, void* stream);
