@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "count_sort.cuh"
 #include "fluid3d_kernels.cuh"
 #include "grid_sync.cuh"
 #include "onesweep.cuh"
@@ -138,6 +139,8 @@ struct gbsph_batch3d_s {
     uint16_t* nbr = nullptr;
     uint32_t* nbr_meta = nullptr;
     uint2* table = nullptr;
+    uint32_t* count = nullptr;  // the counting sort's cell counts (staged step, where it fits), zero between steps
+    bool count_clean = false;
     bool table_clean = false;
     void* scratch = nullptr;
     uint32_t* err = nullptr;
@@ -165,13 +168,14 @@ void binvalidate(B* h) {
 }
 
 void bfree(B* h) {
-    void* ptrs[5] = {h->block, h->table, h->scratch, h->sdev, nullptr};
+    void* ptrs[5] = {h->block, h->table, h->scratch, h->sdev, h->count};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     h->block = nullptr;
     h->table = nullptr;
     h->scratch = nullptr;
     h->sdev = nullptr;
+    h->count = nullptr;
     h->n = h->cells = 0;
 }
 
@@ -238,35 +242,59 @@ int enqueue_batch(B* h, const KParams& kp, cudaStream_t s) {
     const bool clear = h->table_clean;
     if (!clear) GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->table, 0xFF, h->cells * sizeof(uint2), s));
     h->table_clean = false;
-    GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, kp.n, sort_passes(0, kp.end_bit, kp.digit_bits), s));
-    const int blocks = std::max(1, std::min((int)((kp.n + 255) / 256), num_sms() * 8));
-    if (clear)
-        k_hash_batch<true><<<blocks, 256, 0, s>>>(h->pos, kp, h->keys_a, (uint32_t*)h->scratch, h->keys_c, h->table);
-    else
-        k_hash_batch<false><<<blocks, 256, 0, s>>>(h->pos, kp, h->keys_a, (uint32_t*)h->scratch, nullptr, nullptr);
-    GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
-    OnesweepArgs a;
-    a.keys_in = h->keys_a;
-    a.keys_out = h->keys_c;
-    a.vals_out = h->index;
-    a.tmp_keys[0] = h->keys_b;
-    a.tmp_vals[0] = h->vals_b;
-    a.tmp_keys[1] = h->keys_a;
-    a.tmp_vals[1] = h->vals_a;
-    a.n = kp.n;
-    a.end_bit = kp.end_bit;
-    a.digit_bits = kp.digit_bits;
-    a.items = h->sort_items;
-    a.scratch = h->scratch;
-    a.err = h->err;
-    a.gather.n_gather = 2;
-    a.gather.src[0] = h->pos;
-    a.gather.src[1] = h->vel;
-    a.gather.dst[0] = h->spos;
-    a.gather.dst[1] = h->svel;
-    GBSPH_CUDA_TRY(&h->last_error, onesweep_passes(a, s));
-    k_bounds_batch<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, bcounters(h), h->err);
-    GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+    if (h->count) {
+        if (!h->count_clean) GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, count_words(kp.table_cells) * 4, s));
+        h->count_clean = false;
+        CountSort c;
+        c.pos = h->pos;
+        c.vel = h->vel;
+        c.spos = h->spos;
+        c.svel = h->svel;
+        c.keys_in = h->keys_a;
+        c.places = h->keys_b;
+        c.slots = reinterpret_cast<uint2*>(h->vals_a);  // and vals_b behind it
+        c.keys = h->keys_c;
+        c.index = h->index;
+        c.bricks = h->bricks;
+        c.count = h->count;
+        c.table = h->table;
+        c.scratch = h->scratch;
+        c.err = h->err;
+        c.clear = clear;
+        c.full = false;
+        GBSPH_CUDA_TRY(&h->last_error, count_sort<true>(c, kp, s));
+        h->count_clean = true;
+    } else {
+        GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, kp.n, sort_passes(0, kp.end_bit, kp.digit_bits), s));
+        const int blocks = std::max(1, std::min((int)((kp.n + 255) / 256), num_sms() * 8));
+        if (clear)
+            k_hash_batch<true><<<blocks, 256, 0, s>>>(h->pos, kp, h->keys_a, (uint32_t*)h->scratch, h->keys_c, h->table);
+        else
+            k_hash_batch<false><<<blocks, 256, 0, s>>>(h->pos, kp, h->keys_a, (uint32_t*)h->scratch, nullptr, nullptr);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+        OnesweepArgs a;
+        a.keys_in = h->keys_a;
+        a.keys_out = h->keys_c;
+        a.vals_out = h->index;
+        a.tmp_keys[0] = h->keys_b;
+        a.tmp_vals[0] = h->vals_b;
+        a.tmp_keys[1] = h->keys_a;
+        a.tmp_vals[1] = h->vals_a;
+        a.n = kp.n;
+        a.end_bit = kp.end_bit;
+        a.digit_bits = kp.digit_bits;
+        a.items = h->sort_items;
+        a.scratch = h->scratch;
+        a.err = h->err;
+        a.gather.n_gather = 2;
+        a.gather.src[0] = h->pos;
+        a.gather.src[1] = h->vel;
+        a.gather.dst[0] = h->spos;
+        a.gather.dst[1] = h->svel;
+        GBSPH_CUDA_TRY(&h->last_error, onesweep_passes(a, s));
+        k_bounds_batch<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, bcounters(h), h->err);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+    }
     h->table_clean = true;
     k_density_brick<3, true><<<h->dens_blocks, 32 * DENSITY_CONSUMERS + 32, DENSITY_SMEM, s>>>(h->spos, h->svel, h->table, h->bricks,
                                                                                 bcounters(h), kp, h->nbr, h->nbr_meta, h->err);
@@ -324,9 +352,9 @@ int bcompute(B* h, cudaStream_t s, bool allow_graph) {
                     std::to_string(kp.digit_bits) + "-bit digits need more than four passes over " +
                         std::to_string(kp.end_bit) + "-bit keys");
     auto enqueue = [&](cudaStream_t st) { return h->persistent ? enqueue_persistent(h, kp, st) : enqueue_batch(h, kp, st); };
-    if (!h->use_graph || !allow_graph || !h->table_clean || (h->persistent && !h->persistent_graph_ok)) {
+    if (!h->use_graph || !allow_graph || !h->table_clean || (h->count && !h->count_clean && !h->persistent) || (h->persistent && !h->persistent_graph_ok)) {
         const int rc = enqueue(s);
-        if (rc) h->table_clean = false;
+        if (rc) h->table_clean = h->count_clean = false;
         return rc;
     }
     std::vector<char> key(sizeof(KParams));
@@ -342,14 +370,14 @@ int bcompute(B* h, cudaStream_t s, bool allow_graph) {
         if (g) cudaGraphDestroy(g);
         if (rc || ce != cudaSuccess || ie != cudaSuccess) {
             h->gexec = nullptr;
-            h->table_clean = false;
+            h->table_clean = h->count_clean = false;
             if (h->persistent) {  // a cooperative launch that this driver cannot capture: run it eagerly
                 cudaGetLastError();
                 h->persistent_graph_ok = false;
                 h->last_error = std::string("the persistent step could not be captured (") +
                                 cudaGetErrorString(ce != cudaSuccess ? ce : ie) + "); it runs eagerly";
                 const int rc2 = enqueue(s);
-                if (rc2) h->table_clean = false;
+                if (rc2) h->table_clean = h->count_clean = false;
                 return rc2;
             }
             if (rc) return rc;
@@ -361,7 +389,7 @@ int bcompute(B* h, cudaStream_t s, bool allow_graph) {
     }
     const cudaError_t le = cudaGraphLaunch(h->gexec, s);
     if (le != cudaSuccess) {
-        h->table_clean = false;
+        h->table_clean = h->count_clean = false;
         return fail(&h->last_error, GBSPH_ERR_CUDA, std::string("graph launch: ") + cudaGetErrorString(le));
     }
     h->table_clean = true;
@@ -487,8 +515,11 @@ GBSPH_API int gbsph_batch3d_set_scenes(gbsph_batch3d_t h, const gbsph_fluid3d_pa
     p += n4 * NBR_CAP * 2;
     h->nbr_meta = (uint32_t*)p;
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->table, cells * sizeof(uint2)));
-    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, onesweep_scratch_bytes((uint32_t)n, SORT_MAX_PASSES)));
+    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, sort_scratch_bytes((uint32_t)n)));
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->sdev, n_scenes * sizeof(SceneDev)));
+    if (count_sort_fits((uint32_t)cells, (uint32_t)n))
+        GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->count, count_words((uint32_t)cells) * 4));
+    h->count_clean = false;
     h->sdev_bw = -1;
     h->table_clean = false;
     return upload_scenes(h);
@@ -627,7 +658,7 @@ GBSPH_API int gbsph_batch3d_sync_status(gbsph_batch3d_t h, void* stream) {
     GBSPH_CUDA_TRY(&h->last_error, cudaMemcpy(&bits, h->err, 4, cudaMemcpyDeviceToHost));
     if (bits) {
         GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->err, 0, 4));
-        h->table_clean = false;
+        h->table_clean = h->count_clean = false;
         return fail(&h->last_error, dev_err_to_status(bits), "device error word 0x" + std::to_string(bits));
     }
     return GBSPH_OK;

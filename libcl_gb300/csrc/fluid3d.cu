@@ -13,6 +13,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "count_sort.cuh"
 #include "fluid3d_access.h"
 
 using namespace gbsph;
@@ -48,7 +49,10 @@ struct gbsph_fluid3d_s {
     uint32_t *vals_a = nullptr, *vals_b = nullptr, *index = nullptr, *bricks = nullptr;
     uint16_t* nbr = nullptr;      // per particle NBR_CAP neighbour slots (density -> forces)
     uint32_t* nbr_meta = nullptr;  // per particle: list length or scan flag, cell x
-    uint32_t* hash_tables = nullptr;  // cell start / end, REF_BUCKETS each
+    uint2* hash_table = nullptr;      // REFERENCE_HASH: start, end of each bucket
+    uint32_t* count = nullptr;        // the counting sort's cell counts, zero between steps
+    size_t count_words = 0;
+    bool count_clean = false;
     uint32_t* xlist = nullptr;        // REFERENCE_HASH fused step: XL_CAP neighbours + count per particle
     size_t xlist_n = 0;
     uint2* table = nullptr;           // LINEAR_GRID interleaved table
@@ -251,7 +255,7 @@ int alloc_particle_arrays(H* h, size_t n) {
     h->nbr = (uint16_t*)p;
     p += n4 * NBR_CAP * 2;
     h->nbr_meta = (uint32_t*)p;
-    h->scratch_bytes = onesweep_scratch_bytes((uint32_t)n, SORT_MAX_PASSES);
+    h->scratch_bytes = sort_scratch_bytes((uint32_t)n);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, h->scratch_bytes));
     GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->scratch, 0, h->scratch_bytes));
     h->n_alloc = n;
@@ -285,9 +289,9 @@ int ensure_tables(H* h) {
             invalidate_graph(h);
         }
     } else {
-        if (!h->hash_tables) {
-            GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->hash_tables, 2 * (size_t)REF_BUCKETS * 4));
-            GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->hash_tables, 0xFF, 2 * (size_t)REF_BUCKETS * 4));
+        if (!h->hash_table) {
+            GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->hash_table, (size_t)REF_BUCKETS * sizeof(uint2)));
+            GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->hash_table, 0xFF, (size_t)REF_BUCKETS * sizeof(uint2)));
         }
         if (h->xlist_n != h->n_alloc) {  // the fused step's neighbour lists
             if (h->xlist) cudaFree(h->xlist);
@@ -297,6 +301,17 @@ int ensure_tables(H* h) {
             h->xlist_n = h->n_alloc;
             invalidate_graph(h);
         }
+    }
+    // the counting sort's counts, only where it is used
+    const size_t cells = h->params.keyMode == GBSPH_KEY_LINEAR_GRID ? h->table_cells : (size_t)REF_BUCKETS;
+    if (h->opt_fused && count_sort_fits((uint32_t)cells, (uint32_t)h->n) && count_words((uint32_t)cells) > h->count_words) {
+        if (h->count) cudaFree(h->count);
+        h->count = nullptr;
+        h->count_words = 0;
+        GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->count, count_words((uint32_t)cells) * 4));
+        h->count_words = count_words((uint32_t)cells);
+        h->count_clean = false;
+        invalidate_graph(h);
     }
     return GBSPH_OK;
 }
@@ -349,6 +364,33 @@ int st_sort(H* h, const KParams& kp, cudaStream_t s, bool gather, cudaEvent_t be
     return GBSPH_OK;
 }
 
+bool use_count_sort(const H* h, const KParams& kp) {
+    return h->count && count_sort_fits(kp.table_cells, kp.n) && count_words(kp.table_cells) <= h->count_words;
+}
+
+int st_count_sort(H* h, const KParams& kp, cudaStream_t s, bool clear, bool gather_vel) {
+    const bool linear = kp.key_mode == GBSPH_KEY_LINEAR_GRID;
+    CountSort a;
+    a.pos = P4(h, 0);
+    a.vel = gather_vel ? P4(h, 1) : nullptr;
+    a.spos = h->spos;
+    a.svel = h->svel;
+    a.keys_in = h->keys_a;
+    a.places = h->keys_b;
+    a.slots = reinterpret_cast<uint2*>(h->vals_a);  // and vals_b behind it
+    a.keys = h->keys_c;
+    a.index = h->index;
+    a.bricks = h->bricks;
+    a.count = h->count;
+    a.table = linear ? h->table : h->hash_table;
+    a.scratch = h->scratch;
+    a.err = h->err;
+    a.clear = clear;
+    a.full = !linear;
+    GBSPH_CUDA_TRY(&h->last_error, count_sort<false>(a, kp, s));
+    return GBSPH_OK;
+}
+
 // Sorted velocities gathered on their own (when the velocity upload is still in flight while
 // the sort runs).
 __global__ void k_gather_velocity(const uint32_t* __restrict__ index, const float4* __restrict__ vel,
@@ -370,8 +412,9 @@ int st_bounds(H* h, const KParams& kp, cudaStream_t s, bool full_clear) {
         k_bounds_linear<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, counters(h), h->err);
         GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     } else {
-        GBSPH_CUDA_TRY(&h->last_error, cell_bounds_launch(h->keys_c, kp.n, h->hash_tables,
-                                                          h->hash_tables + REF_BUCKETS, REF_BUCKETS, h->err, s));
+        GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->hash_table, 0xFF, (size_t)REF_BUCKETS * sizeof(uint2), s));
+        k_bounds_hash<<<grid1(kp.n), 256, 0, s>>>(h->keys_c, kp.n, h->hash_table, REF_BUCKETS, h->err);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     }
     return GBSPH_OK;
 }
@@ -383,14 +426,14 @@ int st_density_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false
     uint32_t* xl = h->xlist;
     uint32_t* xc = h->xlist ? h->xlist + (size_t)h->xlist_n * XL_CAP : nullptr;
     if (kp.key_mode == GBSPH_KEY_LINEAR_GRID)
-        k_density_exact<GBSPH_KEY_LINEAR_GRID, PairTable, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, PairTable{h->table}, kp, nullptr, nullptr);
+        k_density_exact<GBSPH_KEY_LINEAR_GRID, false><<<grid1(kp.n), 256, 0, s>>>(
+            h->spos, h->svel, h->table, kp, nullptr, nullptr);
     else if (lists && xl)
-        k_density_exact<GBSPH_KEY_REFERENCE_HASH, SplitTable, true><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, SplitTable{h->hash_tables, h->hash_tables + REF_BUCKETS}, kp, xl, xc);
+        k_density_exact<GBSPH_KEY_REFERENCE_HASH, true><<<grid1(kp.n), 256, 0, s>>>(
+            h->spos, h->svel, h->hash_table, kp, xl, xc);
     else
-        k_density_exact<GBSPH_KEY_REFERENCE_HASH, SplitTable, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, SplitTable{h->hash_tables, h->hash_tables + REF_BUCKETS}, kp, nullptr, nullptr);
+        k_density_exact<GBSPH_KEY_REFERENCE_HASH, false><<<grid1(kp.n), 256, 0, s>>>(
+            h->spos, h->svel, h->hash_table, kp, nullptr, nullptr);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
@@ -399,14 +442,14 @@ int st_forces_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false)
     const uint32_t* xl = h->xlist;
     const uint32_t* xc = h->xlist ? h->xlist + (size_t)h->xlist_n * XL_CAP : nullptr;
     if (kp.key_mode == GBSPH_KEY_LINEAR_GRID)
-        k_forces_exact<GBSPH_KEY_LINEAR_GRID, PairTable, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, P4(h, 2), h->index, PairTable{h->table}, kp, nullptr, nullptr);
+        k_forces_exact<GBSPH_KEY_LINEAR_GRID, false><<<grid1(kp.n), 256, 0, s>>>(
+            h->spos, h->svel, P4(h, 2), h->index, h->table, kp, nullptr, nullptr);
     else if (lists && xl)
-        k_forces_exact<GBSPH_KEY_REFERENCE_HASH, SplitTable, true><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, P4(h, 2), h->index, SplitTable{h->hash_tables, h->hash_tables + REF_BUCKETS}, kp, xl, xc);
+        k_forces_exact<GBSPH_KEY_REFERENCE_HASH, true><<<grid1(kp.n), 256, 0, s>>>(
+            h->spos, h->svel, P4(h, 2), h->index, h->hash_table, kp, xl, xc);
     else
-        k_forces_exact<GBSPH_KEY_REFERENCE_HASH, SplitTable, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, P4(h, 2), h->index, SplitTable{h->hash_tables, h->hash_tables + REF_BUCKETS}, kp,
+        k_forces_exact<GBSPH_KEY_REFERENCE_HASH, false><<<grid1(kp.n), 256, 0, s>>>(
+            h->spos, h->svel, P4(h, 2), h->index, h->hash_table, kp,
             nullptr, nullptr);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
@@ -527,11 +570,19 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
         GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->table, 0xFF, h->table_cells * sizeof(uint2), s));
     h->table_clean = false;
     if (io) GBSPH_CUDA_TRY(&h->last_error, cudaStreamWaitEvent(s, h->io_ev[1], 0));
-    RC(st_hash(h, kp, s, clear));
-    RC(mark(h, 1, s));
     // with host input the sort does not wait for the velocity upload: the sorted velocities
-    // are gathered after the cell bounds (before the density pass, which writes their w)
-    RC(st_sort(h, kp, s, true, nullptr, io == nullptr));
+    // are gathered after it (before the density pass, which writes their w)
+    const bool counting = use_count_sort(h, kp);
+    if (counting) {
+        if (!h->count_clean) GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, h->count_words * 4, s));
+        h->count_clean = false;
+        RC(mark(h, 1, s));
+        RC(st_count_sort(h, kp, s, clear, io == nullptr));
+    } else {
+        RC(st_hash(h, kp, s, clear));
+        RC(mark(h, 1, s));
+        RC(st_sort(h, kp, s, true, nullptr, io == nullptr));
+    }
     auto gather_velocity = [&]() -> int {
         if (!io) return GBSPH_OK;
         GBSPH_CUDA_TRY(&h->last_error, cudaStreamWaitEvent(s, h->io_ev[2], 0));
@@ -541,9 +592,11 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
     };
     RC(mark(h, 2, s));
     if (linear) {
-        // counters were zeroed with the sort scratch in st_hash
-        k_bounds_linear<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, counters(h), h->err);
-        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+        if (!counting) {
+            // counters were zeroed with the sort scratch in st_hash
+            k_bounds_linear<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, counters(h), h->err);
+            GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+        }
         h->table_clean = true;
         RC(gather_velocity());
         RC(mark(h, 3, s));
@@ -552,7 +605,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
         if (io) GBSPH_CUDA_TRY(&h->last_error, cudaStreamWaitEvent(s, h->io_ev[3], 0));
         RC(st_force_brick(h, kp, s, h->hook == nullptr));
     } else {
-        RC(st_bounds(h, kp, s, true));
+        if (!counting) RC(st_bounds(h, kp, s, true));
         RC(gather_velocity());
         RC(mark(h, 3, s));
         RC(st_density_exact(h, kp, s, true));
@@ -564,6 +617,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
             GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
         }
     }
+    h->count_clean = h->count_clean || counting;
     RC(mark(h, 5, s));
     h->ev_valid = h->opt_profile != 0;
     if (h->hook) RC(run_hook(h, s));
@@ -576,7 +630,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
 }
 
 std::vector<char> graph_key(const H* h, const KParams& kp) {
-    std::vector<char> k(sizeof(KParams) + 3 * sizeof(void*) + 4 * sizeof(int));
+    std::vector<char> k(sizeof(KParams) + 3 * sizeof(void*) + 4 * sizeof(int));  // the library's own buffers: invalidate_graph
     char* p = k.data();
     std::memcpy(p, &kp, sizeof(KParams));
     p += sizeof(KParams);
@@ -698,7 +752,8 @@ GBSPH_API int gbsph_fluid3d_destroy(gbsph_fluid3d_t h) {
     for (auto& b : h->buf)
         if (b.owned && b.ptr) cudaFree(b.ptr);
     free_particle_arrays(h);
-    if (h->hash_tables) cudaFree(h->hash_tables);
+    if (h->hash_table) cudaFree(h->hash_table);
+    if (h->count) cudaFree(h->count);
     if (h->xlist) cudaFree(h->xlist);
     if (h->table) cudaFree(h->table);
     if (h->err) cudaFree(h->err);
@@ -850,10 +905,10 @@ int compute_impl(H* h, cudaStream_t s, const HostIO* io, bool io_graph) {
                 GBSPH_CUDA_TRY(&h->last_error, cudaMemcpyAsync(io->out[w], P4(h, w), bytes, cudaMemcpyDeviceToHost, s));
         return GBSPH_OK;
     }
-    const bool steady = kp.key_mode != GBSPH_KEY_LINEAR_GRID || h->table_clean;
+    const bool steady = (kp.key_mode != GBSPH_KEY_LINEAR_GRID || h->table_clean) && (h->count_clean || !use_count_sort(h, kp));
     if (h->hook || !h->opt_graph || !steady || h->opt_profile || (io && !io_graph)) {
         const int rc = enqueue_fused(h, kp, s, io);
-        if (rc) h->table_clean = false;
+        if (rc) h->table_clean = h->count_clean = false;
         return rc;
     }
     std::vector<char> key = graph_key(h, kp);
@@ -875,24 +930,27 @@ int compute_impl(H* h, cudaStream_t s, const HostIO* io, bool io_graph) {
         const cudaError_t ce = cudaStreamEndCapture(h->cap_stream, &g);
         if (rc || ce != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
-            h->table_clean = false;
+            h->table_clean = h->count_clean = false;
             return rc ? rc : fail(&h->last_error, GBSPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
         }
         const cudaError_t ie = cudaGraphInstantiate(&gexec, g, 0);
         cudaGraphDestroy(g);
         if (ie != cudaSuccess) {
             gexec = nullptr;
-            h->table_clean = false;
+            h->table_clean = h->count_clean = false;
             return fail(&h->last_error, GBSPH_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
         }
         gkey = key;
     }
     const cudaError_t le = cudaGraphLaunch(gexec, s);
     if (le != cudaSuccess) {
-        h->table_clean = false;
+        h->table_clean = h->count_clean = false;
         return fail(&h->last_error, GBSPH_ERR_CUDA, std::string("graph launch: ") + cudaGetErrorString(le));
     }
-    h->table_clean = true;
+    // a step on hashed keys leaves the grid's table as an earlier step wrote it, but no longer that
+    // step's sorted keys to clear it by
+    h->table_clean = kp.key_mode == GBSPH_KEY_LINEAR_GRID;
+    h->count_clean = h->count_clean || use_count_sort(h, kp);
     return GBSPH_OK;
 }
 
@@ -987,10 +1045,10 @@ GBSPH_API int gbsph_fluid3d_get_cell_bounds(gbsph_fluid3d_t h, uint32_t* cell_st
         k_table_split<<<(unsigned)((n_cells + 255) / 256), 256, 0, s>>>(h->table, (uint32_t)n_cells, cell_start, cell_end);
         GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     } else {
-        if (n_cells != REF_BUCKETS || !h->hash_tables)
+        if (n_cells != REF_BUCKETS || !h->hash_table)
             return fail(&h->last_error, GBSPH_ERR_SIZE_MISMATCH, "n_cells must be 262144");
-        GBSPH_CUDA_TRY(&h->last_error, cudaMemcpyAsync(cell_start, h->hash_tables, REF_BUCKETS * 4ull, cudaMemcpyDeviceToDevice, s));
-        GBSPH_CUDA_TRY(&h->last_error, cudaMemcpyAsync(cell_end, h->hash_tables + REF_BUCKETS, REF_BUCKETS * 4ull, cudaMemcpyDeviceToDevice, s));
+        k_table_split<<<REF_BUCKETS / 256, 256, 0, s>>>(h->hash_table, REF_BUCKETS, cell_start, cell_end);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     }
     return GBSPH_OK;
 }
@@ -1003,7 +1061,7 @@ GBSPH_API int gbsph_fluid3d_sync_status(gbsph_fluid3d_t h, void* stream) {
     GBSPH_CUDA_TRY(&h->last_error, cudaMemcpy(&bits, h->err, 4, cudaMemcpyDeviceToHost));
     if (bits) {
         GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->err, 0, 4));
-        h->table_clean = false;
+        h->table_clean = h->count_clean = false;
         return fail(&h->last_error, dev_err_to_status(bits), "device error word 0x" + std::to_string(bits));
     }
     return GBSPH_OK;

@@ -208,8 +208,17 @@ static __global__ void __launch_bounds__(256) k_bounds_linear(const uint32_t* __
                 [=](uint32_t k) { return (k % nx) / bw + bxn * (k / nx); }, blockIdx.x);
 }
 
-// Batch version of k_hash: each particle keys into its own scene's grid; the key is the
-// scene's cell offset plus the local linear key. The body takes the block's histogram
+// A batch's key: the scene's cell offset plus the linear key in the scene's own grid.
+__device__ __forceinline__ uint32_t batch_key(const KParams& kp, uint32_t i, float4 p) {
+    const SceneDev& d = kp.scenes[scene_of<0>(kp.scenes, kp.n_scenes, i)];
+    const int gx = (int)floorf(__fdiv_rn(__fsub_rn(p.x, d.origin.x), kp.h));
+    const int gy = (int)floorf(__fdiv_rn(__fsub_rn(p.y, d.origin.y), kp.h));
+    const int gz = (int)floorf(__fdiv_rn(__fsub_rn(p.z, d.origin.z), kp.h));
+    return d.cell_off + (uint32_t)clampi(gx, 0, d.nx - 1) +
+           (uint32_t)d.nx * ((uint32_t)clampi(gy, 0, d.ny - 1) + (uint32_t)d.ny * (uint32_t)clampi(gz, 0, d.nz - 1));
+}
+
+// Batch version of k_hash: each particle keys into its own scene's grid. The body takes the block's histogram
 // buffer (SORT_MAX_PASSES * SORT_RADIX words of shared memory) from the caller.
 template <bool CLEAR>
 __device__ __forceinline__ void hash_batch_run(uint32_t* s_h, const float4* __restrict__ pos, const KParams& kp,
@@ -219,13 +228,7 @@ __device__ __forceinline__ void hash_batch_run(uint32_t* s_h, const float4* __re
     __syncthreads();
     const int passes = sort_passes(0, kp.end_bit, kp.digit_bits);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kp.n; i += gridDim.x * blockDim.x) {
-        const SceneDev& d = kp.scenes[scene_of<0>(kp.scenes, kp.n_scenes, i)];
-        const float4 p = pos[i];
-        const int gx = (int)floorf(__fdiv_rn(__fsub_rn(p.x, d.origin.x), kp.h));
-        const int gy = (int)floorf(__fdiv_rn(__fsub_rn(p.y, d.origin.y), kp.h));
-        const int gz = (int)floorf(__fdiv_rn(__fsub_rn(p.z, d.origin.z), kp.h));
-        const uint32_t k = d.cell_off + (uint32_t)clampi(gx, 0, d.nx - 1) +
-                           (uint32_t)d.nx * ((uint32_t)clampi(gy, 0, d.ny - 1) + (uint32_t)d.ny * (uint32_t)clampi(gz, 0, d.nz - 1));
+        const uint32_t k = batch_key(kp, i, pos[i]);
         keys[i] = k;
         for (int q = 0; q < passes; ++q) {
             const int shift = q * kp.digit_bits;
@@ -264,6 +267,20 @@ static __global__ void __launch_bounds__(256) k_bounds_batch(const uint32_t* __r
     bounds_tile(keys, kp, table, bricks, n_bricks, err, [&](uint32_t k) { return batch_brick_of(kp, k); }, blockIdx.x);
 }
 
+// Cell bounds of sorted keys alone (REFERENCE_HASH, per-stage calls): the cells' first index and end.
+static __global__ void __launch_bounds__(256) k_bounds_hash(const uint32_t* __restrict__ keys, uint32_t n,
+                                                            uint2* __restrict__ table, uint32_t cells, uint32_t* err) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t k = keys[i];
+    if (k >= cells) {
+        atomicOr(err, DEV_ERR_KEY_RANGE);
+        return;
+    }
+    if (i == 0 || keys[i - 1] != k) table[k].x = i;
+    if (i + 1 == n || keys[i + 1] != k) table[k].y = i + 1;
+}
+
 // Splits the interleaved table into two arrays (for inspection through the ABI).
 static __global__ void k_table_split(const uint2* __restrict__ table, uint32_t cells,
                               uint32_t* __restrict__ cs, uint32_t* __restrict__ ce) {
@@ -276,19 +293,9 @@ static __global__ void k_table_split(const uint2* __restrict__ table, uint32_t c
 
 // ---- exact (reference-order) neighbour kernels ---------------------------------------------
 
-struct SplitTable {  // REFERENCE_HASH: bfCellStart / bfCellEnd
-    const uint32_t* cs;
-    const uint32_t* ce;
-    __device__ __forceinline__ uint2 get(uint32_t k) const { return make_uint2(cs[k], ce[k]); }
-};
-struct PairTable {  // LINEAR_GRID: interleaved
-    const uint2* t;
-    __device__ __forceinline__ uint2 get(uint32_t k) const { return t[k]; }
-};
-
 // Calls f(start, end) for each non-empty neighbour cell in the reference's visiting order.
-template <int MODE, class Table, class F>
-__device__ __forceinline__ void for_each_neighbour_cell(const KParams& kp, const Table& tab, float4 p, F&& f) {
+template <int MODE, class F>
+__device__ __forceinline__ void for_each_neighbour_cell(const KParams& kp, const uint2* __restrict__ tab, float4 p, F&& f) {
     int gx, gy, gz;
     grid_position(kp, p, gx, gy, gz);
     const int zr = kp.dims == 2 ? 0 : 1;
@@ -308,7 +315,7 @@ __device__ __forceinline__ void for_each_neighbour_cell(const KParams& kp, const
                 } else {
                     cell = hash_key(gx + x, gy + y, gz + z);
                 }
-                const uint2 e = tab.get(cell);
+                const uint2 e = tab[cell];
                 if (e.x == EMPTY) continue;
                 f(e.x, e.y);
             }
@@ -330,9 +337,9 @@ constexpr uint32_t XL_CAP = 64;
 // j (visiting order, repeats of a bucket visited twice included) go to xl[k * n + particle]
 // (entry-major, so that the force kernel's threads, stepping through their lists together,
 // read consecutive words) and their number to xc[particle].
-template <int MODE, class Table, bool RECORD>
+template <int MODE, bool RECORD>
 __global__ void __launch_bounds__(256) k_density_exact(float4* __restrict__ spos, float4* __restrict__ svel,
-                                                       Table tab, KParams kp, uint32_t* __restrict__ xl,
+                                                       const uint2* __restrict__ tab, KParams kp, uint32_t* __restrict__ xl,
                                                        uint32_t* __restrict__ xc) {
     const uint32_t particle = blockIdx.x * blockDim.x + threadIdx.x;
     if (particle >= kp.n) return;
@@ -375,12 +382,12 @@ __global__ void __launch_bounds__(256) k_density_exact(float4* __restrict__ spos
 // takes them from its list, in the same visiting order, instead of scanning the buckets again:
 // the same pairs in the same order, so the same sums, but the warp's threads step through
 // their pairs together rather than each meeting its in-range candidates at different steps.
-template <int MODE, class Table, bool LISTED>
+template <int MODE, bool LISTED>
 __global__ void __launch_bounds__(256) k_forces_exact(const float4* __restrict__ spos,
                                                       const float4* __restrict__ svel,
                                                       float4* __restrict__ force,
                                                       const uint32_t* __restrict__ index,
-                                                      Table tab, KParams kp, const uint32_t* __restrict__ xl,
+                                                      const uint2* __restrict__ tab, KParams kp, const uint32_t* __restrict__ xl,
                                                       const uint32_t* __restrict__ xc) {
     const uint32_t particle = blockIdx.x * blockDim.x + threadIdx.x;
     if (particle >= kp.n) return;
