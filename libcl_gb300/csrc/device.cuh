@@ -164,6 +164,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return true;
 }
 
+// Least and greatest value over the warp's 32 lanes (NaNs are left out while another lane has a number).
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+__device__ __forceinline__ uint32_t warp_max(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+
 // ---- packed FP32 (f32x2, sm_100 and later): two lanes of FP32 per 64-bit register ----------
 __device__ __forceinline__ uint64_t f2_pack(float a, float b) {
     uint64_t r;

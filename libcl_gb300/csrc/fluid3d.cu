@@ -419,38 +419,49 @@ int st_bounds(H* h, const KParams& kp, cudaStream_t s, bool full_clear) {
     return GBSPH_OK;
 }
 
+// Targets per warp of the exact density kernel. Few targets leave each warp a short chain and
+// spread a small scene over the chip; many share the search for their cells' candidates. Us
+// with 2 / 4 / 8 / 16: 4,096 particles 9.6 / 11.6 / 13.8 / 19.9, 16,384 17.8 / 13.7 / 13.8 / 19.9,
+// 32,768 26.0 / 19.8 / 17.9 / 21.2, 65,536 46.5 / 30.4 / 28.1 / 26.0, 1,048,576: 8 463, 16 377, 32 426.
+constexpr uint32_t EXACT_FEW = 8192, EXACT_SOME = 49152;
+
 // Exact (reference-order) density and forces. With lists (the fused REFERENCE_HASH step, where
 // the two run back to back on the same sorted state) the density kernel records each
 // particle's in-range neighbours and the force kernel walks them instead of the buckets.
 int st_density_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false) {
     uint32_t* xl = h->xlist;
     uint32_t* xc = h->xlist ? h->xlist + (size_t)h->xlist_n * XL_CAP : nullptr;
-    if (kp.key_mode == GBSPH_KEY_LINEAR_GRID)
-        k_density_exact<GBSPH_KEY_LINEAR_GRID, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, h->table, kp, nullptr, nullptr);
-    else if (lists && xl)
-        k_density_exact<GBSPH_KEY_REFERENCE_HASH, true><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, h->hash_table, kp, xl, xc);
+    auto launch = [&](auto kern, uint32_t targets, const uint2* table, uint32_t* l, uint32_t* c) {
+        const uint32_t per = targets * EXACT_WARPS;
+        kern<<<(kp.n + per - 1) / per, 32 * EXACT_WARPS, 0, s>>>(h->spos, h->svel, table, kp, l, c);
+    };
+    auto pick = [&](auto k2, auto k8, auto k16, const uint2* table, uint32_t* l, uint32_t* c) {
+        if (kp.n <= EXACT_FEW) launch(k2, 2, table, l, c);
+        else if (kp.n <= EXACT_SOME) launch(k8, 8, table, l, c);
+        else launch(k16, 16, table, l, c);
+    };
+    constexpr int LIN = GBSPH_KEY_LINEAR_GRID, HASH = GBSPH_KEY_REFERENCE_HASH;
+    if (kp.key_mode == LIN)
+        pick(k_density_exact<LIN, false, 2>, k_density_exact<LIN, false, 8>, k_density_exact<LIN, false, 16>, h->table, nullptr, nullptr);
+    else if (lists)
+        pick(k_density_exact<HASH, true, 2>, k_density_exact<HASH, true, 8>, k_density_exact<HASH, true, 16>, h->hash_table, xl, xc);
     else
-        k_density_exact<GBSPH_KEY_REFERENCE_HASH, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, h->hash_table, kp, nullptr, nullptr);
+        pick(k_density_exact<HASH, false, 2>, k_density_exact<HASH, false, 8>, k_density_exact<HASH, false, 16>, h->hash_table, nullptr, nullptr);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
 
-int st_forces_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false) {
+int st_forces_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false, bool post = false) {
     const uint32_t* xl = h->xlist;
     const uint32_t* xc = h->xlist ? h->xlist + (size_t)h->xlist_n * XL_CAP : nullptr;
-    if (kp.key_mode == GBSPH_KEY_LINEAR_GRID)
-        k_forces_exact<GBSPH_KEY_LINEAR_GRID, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, P4(h, 2), h->index, h->table, kp, nullptr, nullptr);
-    else if (lists && xl)
-        k_forces_exact<GBSPH_KEY_REFERENCE_HASH, true><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, P4(h, 2), h->index, h->hash_table, kp, xl, xc);
-    else
-        k_forces_exact<GBSPH_KEY_REFERENCE_HASH, false><<<grid1(kp.n), 256, 0, s>>>(
-            h->spos, h->svel, P4(h, 2), h->index, h->hash_table, kp,
-            nullptr, nullptr);
+    auto launch = [&](auto kern, const uint2* table) {
+        kern<<<grid1(kp.n), 256, 0, s>>>(h->spos, h->svel, P4(h, 2), h->index, table, kp, xl, xc, P4(h, 0), P4(h, 1));
+    };
+    constexpr int LIN = GBSPH_KEY_LINEAR_GRID, HASH = GBSPH_KEY_REFERENCE_HASH;
+    if (kp.key_mode == LIN) launch(k_forces_exact<LIN, false, false>, h->table);
+    else if (lists && post) launch(k_forces_exact<HASH, true, true>, h->hash_table);
+    else if (lists) launch(k_forces_exact<HASH, true, false>, h->hash_table);
+    else launch(k_forces_exact<HASH, false, false>, h->hash_table);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
@@ -611,11 +622,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
         RC(st_density_exact(h, kp, s, true));
         RC(mark(h, 4, s));
         if (io) GBSPH_CUDA_TRY(&h->last_error, cudaStreamWaitEvent(s, h->io_ev[3], 0));
-        RC(st_forces_exact(h, kp, s, true));
-        if (!h->hook) {
-            k_post_fused<<<grid1(kp.n), 256, 0, s>>>(h->spos, h->svel, h->index, P4(h, 0), P4(h, 1), P4(h, 2), kp);
-            GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
-        }
+        RC(st_forces_exact(h, kp, s, true, h->hook == nullptr));
     }
     h->count_clean = h->count_clean || counting;
     RC(mark(h, 5, s));

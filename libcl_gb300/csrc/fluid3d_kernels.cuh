@@ -293,28 +293,40 @@ static __global__ void k_table_split(const uint2* __restrict__ table, uint32_t c
 
 // ---- exact (reference-order) neighbour kernels ---------------------------------------------
 
-// Calls f(start, end) for each non-empty neighbour cell in the reference's visiting order.
-template <int MODE, class F>
-__device__ __forceinline__ void for_each_neighbour_cell(const KParams& kp, const uint2* __restrict__ tab, float4 p, F&& f) {
-    int gx, gy, gz;
+// The cell a particle's neighbours are counted from.
+template <int MODE>
+__device__ __forceinline__ void neighbour_centre(const KParams& kp, float4 p, int& gx, int& gy, int& gz) {
     grid_position(kp, p, gx, gy, gz);
-    const int zr = kp.dims == 2 ? 0 : 1;
     if (MODE == GBSPH_KEY_LINEAR_GRID) {
         gx = clampi(gx, 0, kp.nx - 1);
         gy = clampi(gy, 0, kp.ny - 1);
         gz = kp.dims == 2 ? 0 : clampi(gz, 0, kp.nz - 1);
     }
+}
+
+// The table entry of cell (x, y, z); false outside the grid.
+template <int MODE>
+__device__ __forceinline__ bool neighbour_cell(const KParams& kp, int x, int y, int z, uint32_t& cell) {
+    if (MODE == GBSPH_KEY_LINEAR_GRID) {
+        if (x < 0 || y < 0 || z < 0 || x >= kp.nx || y >= kp.ny || z >= kp.nz) return false;
+        cell = (uint32_t)x + (uint32_t)kp.nx * ((uint32_t)y + (uint32_t)kp.ny * (uint32_t)z);
+    } else {
+        cell = hash_key(x, y, z);
+    }
+    return true;
+}
+
+// Calls f(start, end) for each non-empty neighbour cell in the reference's visiting order.
+template <int MODE, class F>
+__device__ __forceinline__ void for_each_neighbour_cell(const KParams& kp, const uint2* __restrict__ tab, float4 p, F&& f) {
+    int gx, gy, gz;
+    neighbour_centre<MODE>(kp, p, gx, gy, gz);
+    const int zr = kp.dims == 2 ? 0 : 1;
     for (int z = -zr; z <= zr; z++)
         for (int y = -1; y <= 1; y++)
             for (int x = -1; x <= 1; x++) {
                 uint32_t cell;
-                if (MODE == GBSPH_KEY_LINEAR_GRID) {
-                    const int cx = gx + x, cy = gy + y, cz = gz + z;
-                    if (cx < 0 || cy < 0 || cz < 0 || cx >= kp.nx || cy >= kp.ny || cz >= kp.nz) continue;
-                    cell = (uint32_t)cx + (uint32_t)kp.nx * ((uint32_t)cy + (uint32_t)kp.ny * (uint32_t)cz);
-                } else {
-                    cell = hash_key(gx + x, gy + y, gz + z);
-                }
+                if (!neighbour_cell<MODE>(kp, gx + x, gy + y, gz + z, cell)) continue;
                 const uint2 e = tab[cell];
                 if (e.x == EMPTY) continue;
                 f(e.x, e.y);
@@ -332,36 +344,209 @@ __device__ __forceinline__ float exact_r2(float vx, float vy, float vz) {
 // In-range neighbours the exact density kernel records per particle for the exact force
 // kernel (sorted indices in visiting order); a particle with more is scanned again.
 constexpr uint32_t XL_CAP = 64;
+constexpr int EXACT_WARPS = 2;         // per CTA of the density kernel
+constexpr uint32_t EXACT_HELD = 128;   // candidates a warp holds before it pairs them, a multiple of 64
+
+// A warp's shared memory in the exact density kernel, for T targets per warp.
+template <int T>
+struct ExactWarp {
+    float4 a[EXACT_HELD / 64][32];  // candidate 64 p + l and candidate 64 p + 32 + l: x, x, y, y
+    float4 b[EXACT_HELD / 64][32];  // z, z, sorted index, sorted index
+    uint32_t base[32];              // non-empty neighbour cells in visiting order: first index - candidates before
+    float list[XL_CAP * (T + 1)];   // r2 of the in-range candidates: entry k of target t at k * (T + 1) + t
+};
 
 // clCalculateDensity, libCL/phys/oclFluid3D.cl:150-200. With RECORD, the in-range neighbours
-// j (visiting order, repeats of a bucket visited twice included) go to xl[k * n + particle]
-// (entry-major, so that the force kernel's threads, stepping through their lists together,
-// read consecutive words) and their number to xc[particle].
-template <int MODE, bool RECORD>
-__global__ void __launch_bounds__(256) k_density_exact(float4* __restrict__ spos, float4* __restrict__ svel,
-                                                       const uint2* __restrict__ tab, KParams kp, uint32_t* __restrict__ xl,
-                                                       uint32_t* __restrict__ xc) {
-    const uint32_t particle = blockIdx.x * blockDim.x + threadIdx.x;
-    if (particle >= kp.n) return;
-    const float4 posI = spos[particle];
-    float density = 0.0f;
-    int count = 0;
-    uint32_t* mine = RECORD ? xl + particle : nullptr;
-    for_each_neighbour_cell<MODE>(kp, tab, posI, [&](uint32_t start, uint32_t end) {
-        for (uint32_t j = start; j < end; j++) {
-            if (j == particle) continue;
-            const float4 pj = spos[j];
-            const float r2 = exact_r2(__fsub_rn(posI.x, pj.x), __fsub_rn(posI.y, pj.y), __fsub_rn(posI.z, pj.z));
-            if (r2 < kp.r2_thresh) {  // fast_length < h
-                const float vlen = __fsqrt_rn(r2);
-                const float t = __fsub_rn(__fmul_rn(kp.h, kp.h), __fmul_rn(vlen, vlen));
-                density = __fadd_rn(density, __fmul_rn(__fmul_rn(t, t), t));
-                if (RECORD && (uint32_t)count < XL_CAP) mine[(size_t)count * kp.n] = j;
-                count++;
+// j (visiting order, repeats of a bucket visited twice included) go to xl[particle * XL_CAP + k]
+// and their number to xc[particle].
+//
+// The sum of a particle runs in the reference's order, so it is one thread's; what leads to
+// it need not be. A warp takes T consecutive sorted particles and, for each cell among them,
+//  - reads the neighbour cells' ranges at once, a lane each;
+//  - goes through the candidates 32 at a time, in visiting order, and holds those within h of
+//    the box around the cell's targets. For a target inside the box and each axis,
+//    fl(target - candidate) is at least the rounded distance to the box in magnitude
+//    (rounding is monotone), and exact_r2 grows with each: none that is left out is in range;
+//  - for each target tests the held candidates, two to a lane, and appends r2 of those in
+//    range to the target's list.
+// Then a thread sums its target's list. A thread that scans its 27 buckets by itself (12 of
+// the 32 lanes at work, and the root and the sum executed for nearly every candidate because
+// some lane is in range) took 522 us for 1,048,576 particles, 324 candidates and 34 in range
+// each, and 23.6 us for 256, all of it the chain of table reads; this takes 377 and 7.7 us.
+// Bound by instruction issue (76% of cycles). Tried: 64 and 192 candidates held (388 / 391), 32
+// targets per warp (426), the two candidates of a lane next to each other (397).
+template <int MODE, bool RECORD, int T>
+__global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __restrict__ spos, float4* __restrict__ svel,
+                                                                    const uint2* __restrict__ tab, KParams kp,
+                                                                    uint32_t* __restrict__ xl, uint32_t* __restrict__ xc) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    __shared__ ExactWarp<T> shared[EXACT_WARPS];
+    ExactWarp<T>& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
+    const uint32_t first = (blockIdx.x * EXACT_WARPS + (threadIdx.x >> 5)) * T, particle = first + lane;
+    const bool live = lane < T && particle < kp.n;
+    uint32_t left = __ballot_sync(FULL, live);
+    if (!left) return;
+    const float4 posI = live ? spos[particle] : make_float4(0.f, 0.f, 0.f, 0.f);
+    int gx, gy, gz;
+    neighbour_centre<MODE>(kp, posI, gx, gy, gz);
+    const int l = (int)lane, ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = kp.dims == 2 ? 0 : l / 9 - 1;  // place in the visiting order
+    uint32_t count = 0;
+    while (left) {
+        const int lead = __ffs(left) - 1;
+        const int cx = __shfl_sync(FULL, gx, lead), cy = __shfl_sync(FULL, gy, lead), cz = __shfl_sync(FULL, gz, lead);
+        const uint32_t group = __ballot_sync(FULL, live && gx == cx && gy == cy && gz == cz);
+        left &= ~group;
+
+        // the neighbour cells' ranges, lane = place in the visiting order
+        uint2 e = make_uint2(EMPTY, EMPTY);
+        uint32_t cell;
+        if (l < (kp.dims == 2 ? 9 : 27) &&
+            neighbour_cell<MODE>(kp, cx + ox, cy + oy, cz + oz, cell))
+            e = tab[cell];
+        const uint32_t n = e.x == EMPTY ? 0u : e.y - e.x;
+        uint32_t off = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(FULL, off, d);
+            if (l >= d) off += o;
+        }
+        const uint32_t total = __shfl_sync(FULL, off, 31);
+        off -= n;
+        const uint32_t some = __ballot_sync(FULL, n != 0);
+        if (n) S.base[__popc(some & lt)] = e.x - off;
+
+        // the box around the group's targets
+        const bool in = (group >> lane) & 1u;
+        float lo[3], hi[3];
+        {
+            const float x0 = __shfl_sync(FULL, posI.x, lead), y0 = __shfl_sync(FULL, posI.y, lead), z0 = __shfl_sync(FULL, posI.z, lead);
+            const float v[3] = {in ? posI.x : x0, in ? posI.y : y0, in ? posI.z : z0};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = warp_min(v[a]);
+                hi[a] = warp_max(v[a]);
             }
         }
-    });
-    if (RECORD) xc[particle] = (uint32_t)count;
+        __syncwarp();
+
+        uint32_t seen = 0, held = 0;
+        // candidate base + lane: its index (EMPTY beyond the last) and position
+        auto fetch = [&](uint32_t base, float4& p) -> uint32_t {
+            const uint32_t heads = __reduce_or_sync(FULL, n && off - base < 32u ? 1u << (off - base) : 0u);
+            const uint32_t r = seen + (uint32_t)__popc(heads & (lt | 1u << lane)) - 1u;
+            seen += (uint32_t)__popc(heads);
+            if (base + lane >= total) return EMPTY;
+            const uint32_t j = base + lane + S.base[r];
+            p = spos[j];
+            return j;
+        };
+        // pairs the held candidates with the group's targets
+        auto pair = [&]() {
+            for (uint32_t s = held + lane; s < (held + 63u & ~63u); s += 32)  // never in range
+                reinterpret_cast<float*>(&S.a[s >> 6][s & 31])[s >> 5 & 1] = INFINITY;
+            __syncwarp();
+            const uint32_t np = (held + 63u) >> 6;
+            for (uint32_t g = group; g; g &= g - 1) {
+                const int t = __ffs(g) - 1;
+                const float x = __shfl_sync(FULL, posI.x, t), y = __shfl_sync(FULL, posI.y, t), z = __shfl_sync(FULL, posI.z, t);
+                const uint64_t x2 = f2_pack(x, x), y2 = f2_pack(y, y), z2 = f2_pack(z, z);
+                const uint32_t self = first + (uint32_t)t;
+                uint32_t c = __shfl_sync(FULL, count, t);
+                float* list = S.list + t;
+                uint32_t* rec = RECORD ? xl + (size_t)self * XL_CAP : nullptr;
+                for (uint32_t p = 0; p < np; ++p) {
+                    const float4 a = S.a[p][lane], b = S.b[p][lane];
+                    const uint64_t vx = f2_sub(x2, f2_pack(a.x, a.y)), vy = f2_sub(y2, f2_pack(a.z, a.w)),
+                                   vz = f2_sub(z2, f2_pack(b.x, b.y));
+                    // summed one by one: a packed square and a packed sum are joined into an fma, which rounds once
+                    float x0, x1, y0, y1, z0, z1;
+                    f2_unpack(f2_mul(vx, vx), x0, x1);
+                    f2_unpack(f2_mul(vy, vy), y0, y1);
+                    f2_unpack(f2_mul(vz, vz), z0, z1);
+                    const float r0 = __fadd_rn(__fadd_rn(x0, y0), z0), r1 = __fadd_rn(__fadd_rn(x1, y1), z1);
+                    const uint32_t j0 = __float_as_uint(b.z), j1 = __float_as_uint(b.w);
+                    const bool in0 = r0 < kp.r2_thresh && j0 != self, in1 = r1 < kp.r2_thresh && j1 != self;  // fast_length < h
+                    const uint32_t m0 = __ballot_sync(FULL, in0), m1 = __ballot_sync(FULL, in1);
+                    const uint32_t k0 = c + (uint32_t)__popc(m0 & lt);
+                    c += (uint32_t)__popc(m0);
+                    const uint32_t k1 = c + (uint32_t)__popc(m1 & lt);
+                    c += (uint32_t)__popc(m1);
+                    if (in0 && k0 < XL_CAP) {
+                        list[k0 * (T + 1)] = r0;
+                        if (RECORD) rec[k0] = j0;
+                    }
+                    if (in1 && k1 < XL_CAP) {
+                        list[k1 * (T + 1)] = r1;
+                        if (RECORD) rec[k1] = j1;
+                    }
+                }
+                if (l == t) count = c;
+            }
+            __syncwarp();
+            held = 0;
+        };
+        float4 p, ahead;
+        uint32_t j = fetch(0, p), next = EMPTY;
+        for (uint32_t base = 0; base < total; base += 32, j = next, p = ahead) {
+            if (base + 32 < total) next = fetch(base + 32, ahead);
+            bool keep = false;
+            if (j != EMPTY)
+                keep = exact_r2(fmaxf(fmaxf(__fsub_rn(lo[0], p.x), __fsub_rn(p.x, hi[0])), 0.f),
+                                fmaxf(fmaxf(__fsub_rn(lo[1], p.y), __fsub_rn(p.y, hi[1])), 0.f),
+                                fmaxf(fmaxf(__fsub_rn(lo[2], p.z), __fsub_rn(p.z, hi[2])), 0.f)) < kp.r2_thresh;
+            const uint32_t m = __ballot_sync(FULL, keep);
+            if (keep) {
+                const uint32_t s = held + (uint32_t)__popc(m & lt), half = s >> 5 & 1;
+                float* a = reinterpret_cast<float*>(&S.a[s >> 6][s & 31]) + half;
+                float* b = reinterpret_cast<float*>(&S.b[s >> 6][s & 31]) + half;
+                a[0] = p.x;
+                a[2] = p.y;
+                b[0] = p.z;
+                b[2] = __uint_as_float(j);
+            }
+            held += (uint32_t)__popc(m);
+            if (held > EXACT_HELD - 32) pair();
+        }
+        if (held) pair();
+    }
+    __syncwarp();
+    // 32 / T lanes share a target: each computes every (32 / T)-th term, all add them in order
+    auto term = [&](float r2) {
+        const float vlen = __fsqrt_rn(r2);
+        const float t = __fsub_rn(__fmul_rn(kp.h, kp.h), __fmul_rn(vlen, vlen));
+        return __fmul_rn(__fmul_rn(t, t), t);
+    };
+    float density = 0.0f;
+    {
+        constexpr uint32_t SHARE = 32 / T;
+        const int t = l / (int)SHARE, first_lane = l - l % (int)SHARE;
+        const uint32_t mine = __shfl_sync(FULL, count, t), most = warp_max(mine <= XL_CAP ? mine : 0u);
+        float d = 0.0f;
+        for (uint32_t k = 0; k < most; k += SHARE) {
+            const uint32_t at = k + lane % SHARE;
+            const float v = at < mine ? term(S.list[at * (T + 1) + (uint32_t)t]) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < (int)SHARE; ++i) {
+                const float o = __shfl_sync(FULL, v, first_lane + i);
+                if (k + i < mine) d = __fadd_rn(d, o);
+            }
+        }
+        density = __shfl_sync(FULL, d, (l * (int)SHARE) & 31);
+    }
+    if (!live) return;
+    if (count > XL_CAP) {  // more than the list holds: through the buckets again
+        density = 0.0f;
+        for_each_neighbour_cell<MODE>(kp, tab, posI, [&](uint32_t start, uint32_t end) {
+            for (uint32_t j = start; j < end; j++) {
+                if (j == particle) continue;
+                const float4 pj = spos[j];
+                const float r2 = exact_r2(__fsub_rn(posI.x, pj.x), __fsub_rn(posI.y, pj.y), __fsub_rn(posI.z, pj.z));
+                if (r2 < kp.r2_thresh) density = __fadd_rn(density, term(r2));
+            }
+        });
+    }
+    if (RECORD) xc[particle] = count;
     // The reference writes .w in place while other work-items read .xyz only. Here the
     // candidates' positions are loaded as whole float4s, so a load may race with another
     // thread's write of that particle's .w; the loaded .w is never used (the sums take .xyz
@@ -375,79 +560,6 @@ __global__ void __launch_bounds__(256) k_density_exact(float4* __restrict__ spos
         reinterpret_cast<float*>(spos)[4 * (size_t)particle + 3] = kp.rho0;
         reinterpret_cast<float*>(svel)[4 * (size_t)particle + 3] = kp.p0;
     }
-}
-
-// clCalculateForces, libCL/phys/oclFluid3D.cl:202-255: force[index[i]] += SPH force, w = 0.
-// With LISTED, a particle whose in-range neighbours the density kernel recorded (xc <= XL_CAP)
-// takes them from its list, in the same visiting order, instead of scanning the buckets again:
-// the same pairs in the same order, so the same sums, but the warp's threads step through
-// their pairs together rather than each meeting its in-range candidates at different steps.
-template <int MODE, bool LISTED>
-__global__ void __launch_bounds__(256) k_forces_exact(const float4* __restrict__ spos,
-                                                      const float4* __restrict__ svel,
-                                                      float4* __restrict__ force,
-                                                      const uint32_t* __restrict__ index,
-                                                      const uint2* __restrict__ tab, KParams kp, const uint32_t* __restrict__ xl,
-                                                      const uint32_t* __restrict__ xc) {
-    const uint32_t particle = blockIdx.x * blockDim.x + threadIdx.x;
-    if (particle >= kp.n) return;
-    const float4 posI = spos[particle], velI = svel[particle];
-    float px = 0.f, py = 0.f, pz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
-    // one pair with the neighbour's position and velocity at hand
-    auto pair_at = [&](const float4& posJ, const float4& velJ) {
-        const float vx = __fsub_rn(posI.x, posJ.x), vy = __fsub_rn(posI.y, posJ.y), vz = __fsub_rn(posI.z, posJ.z);
-        const float r2 = exact_r2(vx, vy, vz);
-        if (r2 < kp.r2_thresh) {  // fast_length < h
-            const float vlen = __fsqrt_rn(r2);
-            const float density2 = __fmul_rn(posI.w, posJ.w);
-            const float s = __fdiv_rn(__fadd_rn(velI.w, velJ.w), density2);
-            const float hr = __fsub_rn(kp.h, vlen);
-            px = __fadd_rn(px, __fmul_rn(s, __fmul_rn(__fmul_rn(__fdiv_rn(vx, vlen), hr), hr)));
-            py = __fadd_rn(py, __fmul_rn(s, __fmul_rn(__fmul_rn(__fdiv_rn(vy, vlen), hr), hr)));
-            pz = __fadd_rn(pz, __fmul_rn(s, __fmul_rn(__fmul_rn(__fdiv_rn(vz, vlen), hr), hr)));
-            qx = __fadd_rn(qx, __fmul_rn(__fdiv_rn(__fsub_rn(velJ.x, velI.x), density2), hr));
-            qy = __fadd_rn(qy, __fmul_rn(__fdiv_rn(__fsub_rn(velJ.y, velI.y), density2), hr));
-            qz = __fadd_rn(qz, __fmul_rn(__fdiv_rn(__fsub_rn(velJ.z, velI.z), density2), hr));
-        }
-    };
-    auto pair = [&](uint32_t j) {
-        const float4 posJ = spos[j];
-        const float vx = __fsub_rn(posI.x, posJ.x), vy = __fsub_rn(posI.y, posJ.y), vz = __fsub_rn(posI.z, posJ.z);
-        if (exact_r2(vx, vy, vz) < kp.r2_thresh) pair_at(posJ, svel[j]);
-    };
-    const uint32_t nl = LISTED ? xc[particle] : EMPTY;
-    if (LISTED && nl <= XL_CAP) {
-        // the recorded neighbours in their order; the next one's index, position and velocity
-        // are loaded while the current pair is computed
-        const uint32_t* mine = xl + particle;
-        float4 pn = posI, vn = velI;
-        if (nl) {
-            const uint32_t j0 = mine[0];
-            pn = spos[j0];
-            vn = svel[j0];
-        }
-        for (uint32_t k = 0; k < nl; ++k) {
-            const float4 posJ = pn, velJ = vn;
-            if (k + 1 < nl) {
-                const uint32_t jn = mine[(size_t)(k + 1) * kp.n];
-                pn = spos[jn];
-                vn = svel[jn];
-            }
-            pair_at(posJ, velJ);
-        }
-    } else {
-        for_each_neighbour_cell<MODE>(kp, tab, posI, [&](uint32_t start, uint32_t end) {
-            for (uint32_t j = start; j < end; j++)
-                if (j != particle) pair(j);
-        });
-    }
-    const uint32_t o = index[particle];
-    float4 f = force[o];
-    f.x = __fadd_rn(f.x, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, px), __fmul_rn(kp.cvisc, qx)), kp.mass));
-    f.y = __fadd_rn(f.y, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, py), __fmul_rn(kp.cvisc, qy)), kp.mass));
-    f.z = __fadd_rn(f.z, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, pz), __fmul_rn(kp.cvisc, qz)), kp.mass));
-    f.w = 0.0f;
-    force[o] = f;
 }
 
 // ---- post stages ---------------------------------------------------------------------------
@@ -504,6 +616,123 @@ __device__ __forceinline__ float4 integrate_velocity(const KParams& kp, float4 p
                        __fadd_rn(p.z, __fmul_rn(v.z, kp.dt)), __fadd_rn(p.w, __fmul_rn(v.w, kp.dt)));
 }
 
+constexpr uint32_t XL_BLOCK = 16;  // list entries the exact force kernel stages at once
+
+// clCalculateForces, libCL/phys/oclFluid3D.cl:202-255: force[index[i]] += SPH force, w = 0.
+// With LISTED, a particle whose in-range neighbours the density kernel recorded (xc <= XL_CAP)
+// takes them from its list, in the same visiting order, instead of scanning the buckets again:
+// the same pairs in the same order, so the same sums, but the warp's threads step through
+// their pairs together rather than each meeting its in-range candidates at different steps.
+// A warp copies its particles' lists through shared memory, XL_BLOCK entries at a time; threads
+// that read their own rows took 269 us where this takes 190 (1,048,576 particles), and lists
+// laid out entry by entry, which they read in 224, cost the density kernel 43 us in scattered
+// stores. With POST (the fused step without a hook) the particle is also clipped and integrated
+// here: 217 us for both, and a launch less (224 and 30 in kernels of their own at first). Bound by the
+// latency of the gathers. Loading two, four or eight neighbours at once takes more registers
+// and is slower (238 / 256 / 322).
+template <int MODE, bool LISTED, bool POST>
+__global__ void __launch_bounds__(256) k_forces_exact(const float4* __restrict__ spos,
+                                                      const float4* __restrict__ svel,
+                                                      float4* __restrict__ force,
+                                                      const uint32_t* __restrict__ index,
+                                                      const uint2* __restrict__ tab, KParams kp, const uint32_t* __restrict__ xl,
+                                                      const uint32_t* __restrict__ xc, float4* __restrict__ pos,
+                                                      float4* __restrict__ vel) {
+    const uint32_t particle = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = particle < kp.n;
+    if (!LISTED && !live) return;
+    const float4 posI = spos[live ? particle : 0], velI = svel[live ? particle : 0];
+    float px = 0.f, py = 0.f, pz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
+    // one pair with the neighbour's position and velocity at hand
+    auto pair_at = [&](const float4& posJ, const float4& velJ) {
+        const float vx = __fsub_rn(posI.x, posJ.x), vy = __fsub_rn(posI.y, posJ.y), vz = __fsub_rn(posI.z, posJ.z);
+        const float r2 = exact_r2(vx, vy, vz);
+        if (r2 < kp.r2_thresh) {  // fast_length < h
+            const float vlen = __fsqrt_rn(r2);
+            const float density2 = __fmul_rn(posI.w, posJ.w);
+            const float s = __fdiv_rn(__fadd_rn(velI.w, velJ.w), density2);
+            const float hr = __fsub_rn(kp.h, vlen);
+            px = __fadd_rn(px, __fmul_rn(s, __fmul_rn(__fmul_rn(__fdiv_rn(vx, vlen), hr), hr)));
+            py = __fadd_rn(py, __fmul_rn(s, __fmul_rn(__fmul_rn(__fdiv_rn(vy, vlen), hr), hr)));
+            pz = __fadd_rn(pz, __fmul_rn(s, __fmul_rn(__fmul_rn(__fdiv_rn(vz, vlen), hr), hr)));
+            qx = __fadd_rn(qx, __fmul_rn(__fdiv_rn(__fsub_rn(velJ.x, velI.x), density2), hr));
+            qy = __fadd_rn(qy, __fmul_rn(__fdiv_rn(__fsub_rn(velJ.y, velI.y), density2), hr));
+            qz = __fadd_rn(qz, __fmul_rn(__fdiv_rn(__fsub_rn(velJ.z, velI.z), density2), hr));
+        }
+    };
+    auto pair = [&](uint32_t j) {
+        const float4 posJ = spos[j];
+        const float vx = __fsub_rn(posI.x, posJ.x), vy = __fsub_rn(posI.y, posJ.y), vz = __fsub_rn(posI.z, posJ.z);
+        if (exact_r2(vx, vy, vz) < kp.r2_thresh) pair_at(posJ, svel[j]);
+    };
+    bool scan = true;
+    if (LISTED) {
+        __shared__ uint32_t staged[256 / 32][32 * (XL_BLOCK + 1)];
+        uint32_t* block = staged[threadIdx.x >> 5];
+        const uint32_t lane = threadIdx.x & 31u, all = live ? xc[particle] : 0u;
+        scan = all > XL_CAP;
+        const uint32_t nl = scan ? 0u : all, most = __reduce_max_sync(0xffffffffu, nl);
+        const uint4* rows = reinterpret_cast<const uint4*>(xl) + (size_t)(particle - lane) * (XL_CAP / 4);
+        for (uint32_t k0 = 0; k0 < most; k0 += XL_BLOCK) {
+            __syncwarp();
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {  // eight rows a load, four lanes to a row
+                const uint32_t row = 8 * i + lane / 4, q = lane % 4;
+                if (k0 + 4 * q < __shfl_sync(0xffffffffu, nl, (int)row)) {
+                    const uint4 v = rows[row * (XL_CAP / 4) + k0 / 4 + q];
+                    uint32_t* to = block + row * (XL_BLOCK + 1) + 4 * q;
+                    to[0] = v.x;
+                    to[1] = v.y;
+                    to[2] = v.z;
+                    to[3] = v.w;
+                }
+            }
+            __syncwarp();
+            // the next neighbour's position and velocity are loaded while the current pair is computed
+            const uint32_t* mine = block + lane * (XL_BLOCK + 1);
+            const uint32_t m = k0 < nl ? min(nl - k0, XL_BLOCK) : 0u;
+            float4 pn = posI, vn = velI;
+            if (m) {
+                pn = spos[mine[0]];
+                vn = svel[mine[0]];
+            }
+            for (uint32_t k = 0; k < m; ++k) {
+                const float4 posJ = pn, velJ = vn;
+                if (k + 1 < m) {
+                    const uint32_t j = mine[k + 1];
+                    pn = spos[j];
+                    vn = svel[j];
+                }
+                pair_at(posJ, velJ);
+            }
+        }
+        if (!live) return;
+    }
+    if (scan)
+        for_each_neighbour_cell<MODE>(kp, tab, posI, [&](uint32_t start, uint32_t end) {
+            for (uint32_t j = start; j < end; j++)
+                if (j != particle) pair(j);
+        });
+    const uint32_t o = index[particle];
+    float4 f = force[o];
+    f.x = __fadd_rn(f.x, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, px), __fmul_rn(kp.cvisc, qx)), kp.mass));
+    f.y = __fadd_rn(f.y, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, py), __fmul_rn(kp.cvisc, qy)), kp.mass));
+    f.z = __fadd_rn(f.z, __fmul_rn(__fadd_rn(__fmul_rn(kp.cpress, pz), __fmul_rn(kp.cvisc, qz)), kp.mass));
+    f.w = 0.0f;
+    if (!POST) {
+        force[o] = f;
+        return;
+    }
+    // clip + integrate-force + gravity + integrate-velocity, as the four reference kernels
+    // after this one (index is a permutation)
+    f = clip_box_force(kp, posI, velI, f);
+    if (kp.rec_force) kp.rec_force[o] = f;
+    const float4 v = integrate_force(kp, vel[o], f);
+    vel[o] = v;
+    force[o] = kp.gravity;
+    pos[o] = integrate_velocity(kp, pos[o], v);
+}
+
 static __global__ void k_clip_box(const float4* __restrict__ spos, const float4* __restrict__ svel,
                            float4* __restrict__ force, const uint32_t* __restrict__ index, KParams kp) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -548,22 +777,6 @@ static __global__ void k_emitter(float4* __restrict__ pos, float4* __restrict__ 
                                     __double2float_rn(__dadd_rn(0.6, (double)dz)), 1.0f);
         vel[particle] = make_float4(0.0f, emit_speed, 0.0f, 1.0f);
     }
-}
-
-// clip + integrate-force + gravity + integrate-velocity in one pass over sorted slots.
-// Equivalent to the four reference kernels because index is a permutation.
-static __global__ void k_post_fused(const float4* __restrict__ spos, const float4* __restrict__ svel,
-                             const uint32_t* __restrict__ index, float4* __restrict__ pos,
-                             float4* __restrict__ vel, float4* __restrict__ force, KParams kp) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kp.n) return;
-    const uint32_t o = index[i];
-    const float4 f = clip_box_force(kp, spos[i], svel[i], force[o]);
-    if (kp.rec_force) kp.rec_force[o] = f;
-    const float4 v = integrate_force(kp, vel[o], f);
-    vel[o] = v;
-    force[o] = kp.gravity;
-    pos[o] = integrate_velocity(kp, pos[o], v);
 }
 
 // ---- brick (fast, LINEAR_GRID) neighbour kernels ---------------------------------------------
