@@ -1,12 +1,13 @@
 // fluid2d.cu -- the reference's 2D SPH model (double-density relaxation with an image-sampled
 // wall field) on sm_103a: the oclFluid2D replacement behind the C ABI.
 //
-// Each reference kernel of libCL/phys/oclFluid2D.cl becomes one CUDA kernel with the same
-// arithmetic in the same order (round-to-nearest intrinsics, no FMA contraction, IEEE sqrt
-// and division), so results reproduce the FP32 restatement bit for bit. The sort is the
-// library's one-sweep radix sort on the linear cell key. The scene sizes of this model (the
-// reference default is 16,384 particles in a 40 x 36 cell container) are launch-bound, so the
-// whole step is replayed as a CUDA graph.
+// The reference kernels of libCL/phys/oclFluid2D.cl are evaluated with the same arithmetic in
+// the same order (round-to-nearest intrinsics, no FMA contraction, IEEE sqrt and division), so
+// results reproduce the FP32 restatement bit for bit. The sort on the linear cell key is the
+// counting sort of the 3D steps where it fits (16,384 particles in 40 x 36 cells: 16 us with
+// the bounds and the reorder, 24 by two radix passes and four more launches), else the one-sweep
+// radix sort. At the scene sizes of this model launches count, so the whole step is
+// replayed as a CUDA graph: six kernels, eleven nodes before.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -15,8 +16,7 @@
 
 #include <cuda_fp16.h>
 
-#include "device.cuh"
-#include "internal.h"
+#include "count_sort.cuh"
 
 using namespace gbsph;
 
@@ -41,6 +41,7 @@ struct K2 {
     int ncx, ncy;
     uint32_t n, table;
     int W, H;  // wall image size
+    float r2_lo, r2_hi;  // len2 > 1e-7 and len2 < h, on the squares
 };
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
@@ -72,8 +73,55 @@ __device__ __forceinline__ float4 sample(const float4* __restrict__ img, int W, 
     return o;
 }
 
-// clAdvanceState (libCL/phys/oclFluid2D.cl:173-182) fused with clHash (:61-69) and the
-// digit histogram of the sort. Cell coordinates are clamped to the grid.
+// clAdvanceState (libCL/phys/oclFluid2D.cl:173-182) and clHash (:61-69) of particle i. Cell
+// coordinates are clamped to the grid.
+__device__ __forceinline__ uint32_t advance_hash(P2* __restrict__ st, float2* __restrict__ prev, const K2& k, uint32_t i) {
+    P2 p = st[i];
+    prev[i] = make_float2(p.px, p.py);
+    p.vx = fa(p.vx, fm(0.0f, k.dT));
+    p.vy = fa(p.vy, fm(-9.81f, k.dT));
+    p.px = fa(p.px, fm(p.vx, k.dT));
+    p.py = fa(p.py, fm(p.vy, k.dT));
+    st[i] = p;
+    const int gx = min(max((int)floorf(fd(p.px, k.cellSize)), 0), k.ncx - 1);
+    const int gy = min(max((int)floorf(fd(p.py, k.cellSize)), 0), k.ncy - 1);
+    return (uint32_t)(gy * k.ncx + gx);
+}
+
+// Counting sort: key, and a place among the cell's particles (count_sort.cuh).
+__global__ void __launch_bounds__(256) k2_advance_count(P2* __restrict__ st, float2* __restrict__ prev, uint32_t* __restrict__ keys,
+                                                        uint32_t* __restrict__ places, uint32_t* __restrict__ count, K2 k) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= k.n) return;
+    const uint32_t key = advance_hash(st, prev, k, i);
+    keys[i] = key;
+    places[i] = atomicAdd(count + key, 1u);
+}
+
+// Counting sort: sorted keys, permutation and clReorder (libCL/phys/oclFluid2D.cl:71-76), a slot's
+// particle behind those of its cell with smaller ids; the counts are zero again afterwards.
+__global__ void __launch_bounds__(256) k2_order(const uint2* __restrict__ slots, const uint2* __restrict__ table,
+                                                const P2* __restrict__ st, uint32_t* __restrict__ keys, uint32_t* __restrict__ index,
+                                                P2* __restrict__ srt, uint32_t* __restrict__ count, K2 k, uint32_t* err) {
+    const uint32_t s = blockIdx.x * 256u + threadIdx.x;
+    if (s >= k.n) return;
+    const uint2 me = slots[s];
+    const uint2 cell = me.x < k.table ? table[me.x] : make_uint2(0u, 0u);
+    if (cell.y > k.n || s < cell.x || s >= cell.y) {  // a table that does not fit the keys: never write out of range
+        atomicOr(err, DEV_ERR_KEY_RANGE);
+        return;
+    }
+    const P2 p = st[me.y];
+    uint32_t d = cell.x;
+#pragma unroll 4
+    for (uint32_t t = cell.x; t < cell.y; ++t) d += slots[t].y < me.y ? 1u : 0u;
+    keys[s] = me.x;
+    index[d] = me.y;
+    srt[d] = p;
+    if (s == cell.x) count[me.x] = 0u;
+}
+
+// Radix sort (where the counting sort does not fit): keys and the digit histogram of the sort.
 __global__ void k2_advance_hash(P2* __restrict__ st, float2* __restrict__ prev, uint32_t* __restrict__ keys,
                                 uint32_t* __restrict__ hist, K2 k, int end_bit) {
     __shared__ uint32_t s_h[SORT_MAX_PASSES * SORT_RADIX];
@@ -81,16 +129,7 @@ __global__ void k2_advance_hash(P2* __restrict__ st, float2* __restrict__ prev, 
     __syncthreads();
     const int passes = sort_passes(0, end_bit);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.n; i += gridDim.x * blockDim.x) {
-        P2 p = st[i];
-        prev[i] = make_float2(p.px, p.py);
-        p.vx = fa(p.vx, fm(0.0f, k.dT));
-        p.vy = fa(p.vy, fm(-9.81f, k.dT));
-        p.px = fa(p.px, fm(p.vx, k.dT));
-        p.py = fa(p.py, fm(p.vy, k.dT));
-        st[i] = p;
-        const int gx = min(max((int)floorf(fd(p.px, k.cellSize)), 0), k.ncx - 1);
-        const int gy = min(max((int)floorf(fd(p.py, k.cellSize)), 0), k.ncy - 1);
-        const uint32_t key = (uint32_t)(gy * k.ncx + gx);
+        const uint32_t key = advance_hash(st, prev, k, i);
         keys[i] = key;
         for (int q = 0; q < passes; ++q) {
             const int shift = q * SORT_RADIX_BITS;
@@ -109,168 +148,11 @@ __global__ void k2_reorder(const uint32_t* __restrict__ index, const P2* __restr
     if (i < n) srt[i] = st[index[i]];
 }
 
-__device__ __forceinline__ void cells_of(const K2& k, float px, float py, int& x0, int& x1, int& y0, int& y1) {
-    const int gx = (int)floorf(fd(px, k.cellSize)), gy = (int)floorf(fd(py, k.cellSize));
-    x0 = max(gx - 1, 0);
-    x1 = min(gx + 1, k.ncx - 1);
-    y0 = max(gy - 1, 0);
-    y1 = min(gy + 1, k.ncy - 1);
-}
-
-// The neighbour loops of clComputePressure / clComputePosition visit cells x = x0..x1 (outer),
-// y = y0..y1 (inner) and the particles of each cell in sorted order, summing in that order.
-// Here a warp takes one particle: the candidates (the cells' ranges, concatenated in the
-// reference's order) are dealt to the lanes 32 at a time, each lane computes its candidate's
-// terms, and the sums take the in-range terms one by one in candidate order (broadcast by
-// shuffles), so every operation and its order are the reference's.
-struct Cand2 {
-    uint32_t pre;    // lane c < 9: candidates before cell c (of the concatenation)
-    uint32_t start;  // lane c < 9: the cell's first sorted index
-    uint32_t total;  // candidates of all cells (every lane)
-};
-
-__device__ __forceinline__ Cand2 cand2_setup(const K2& k, float px, float py, const uint32_t* __restrict__ cs,
-                                             const uint32_t* __restrict__ ce) {
-    const uint32_t lane = threadIdx.x & 31u;
-    int x0, x1, y0, y1;
-    cells_of(k, px, py, x0, x1, y0, y1);
-    const int ny = y1 - y0 + 1, nc = (x1 - x0 + 1) * ny;
-    uint32_t len = 0, st = 0;
-    if ((int)lane < nc) {
-        const int c = (y0 + (int)lane % ny) * k.ncx + x0 + (int)lane / ny;  // x outer, y inner
-        st = cs[c];
-        if (st != EMPTY2) len = ce[c] - st;
-    }
-    uint32_t incl = len;
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)lane >= o) incl += v;
-    }
-    Cand2 c;
-    c.pre = incl - len;
-    c.start = st;
-    c.total = __shfl_sync(0xffffffffu, incl, 8);
-    return c;
-}
-
-// Sorted index of candidate k < total (from the per-cell values held by lanes 0..8).
-__device__ __forceinline__ uint32_t cand2_index(const Cand2& c, uint32_t k) {
-    uint32_t j = 0;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        const uint32_t pre = __shfl_sync(0xffffffffu, c.pre, q), st = __shfl_sync(0xffffffffu, c.start, q);
-        if (k >= pre) j = st + (k - pre);
-    }
-    return j;
-}
-
-// clComputePressure (libCL/phys/oclFluid2D.cl:185-245), a warp per particle.
-__global__ void k2_pressure(const P2* __restrict__ srt, float4* __restrict__ ps, const uint32_t* __restrict__ cs,
-                            const uint32_t* __restrict__ ce, const float4* __restrict__ bstate, K2 k) {
-    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (i >= k.n) return;  // whole warps
-    const P2 pi = srt[i];
-    float density = 0.f, nearDensity = 0.f;
-    const float4 wall = sample(bstate, k.W, k.H, fd(pi.px, k.cW), fd(pi.py, k.cH));
-    if (wall.x != 0.f) {
-        density = fa(density, wall.x);
-        nearDensity = fa(nearDensity, wall.y);
-    }
-    const Cand2 c = cand2_setup(k, pi.px, pi.py, cs, ce);
-    for (uint32_t base = 0; base < c.total; base += 32) {
-        const uint32_t kk = base + lane;
-        const uint32_t j = cand2_index(c, kk);
-        bool in = false;
-        float td = 0.f, tn = 0.f;
-        if (kk < c.total && j != i) {
-            const float dx = fs(srt[j].px, pi.px), dy = fs(srt[j].py, pi.py);
-            const float r = len2(dx, dy);
-            if (r > 0.0000001f && r < k.h) {
-                const float a = fs(1.f, fd(r, k.h));
-                td = fm(fm(fm(fm(k.m, a), a), a), k.kNorm);
-                tn = fm(fm(fm(fm(fm(k.m, a), a), a), a), k.kNearNorm);
-                in = true;
-            }
-        }
-        for (uint32_t m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
-            const int b = __ffs(m) - 1;
-            density = fa(density, __shfl_sync(0xffffffffu, td, b));
-            nearDensity = fa(nearDensity, __shfl_sync(0xffffffffu, tn, b));
-        }
-    }
-    if (lane == 0)
-        ps[i] = make_float4(density, nearDensity, fm(kStiffness, fs(density, fm(k.m, kRestDensity))),
-                            fm(kNearStiffness, nearDensity));
-}
-
-// clComputePosition (libCL/phys/oclFluid2D.cl:247-326), a warp per particle. The reference's
-// viscosity term uses vel_j - vel_j (:299), which is zero, so it never contributes and is not
-// evaluated here.
-__global__ void k2_position(const P2* __restrict__ srt, const float4* __restrict__ ps, float2* __restrict__ relaxed,
-                            const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
-                            const float4* __restrict__ bstate, const float4* __restrict__ bvec, K2 k) {
-    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (i >= k.n) return;  // whole warps
-    const float4 si = ps[i];
-    const P2 pi = srt[i];
-    float rx = pi.px, ry = pi.py;
-    const float dt2 = fm(k.dT, k.dT);
-    const Cand2 c = cand2_setup(k, pi.px, pi.py, cs, ce);
-    for (uint32_t base = 0; base < c.total; base += 32) {
-        const uint32_t kk = base + lane;
-        const uint32_t j = cand2_index(c, kk);
-        bool in = false;
-        float ux = 0.f, uy = 0.f, wx = 0.f, wy = 0.f;
-        if (kk < c.total && j != i) {
-            const float dx = fs(srt[j].px, pi.px), dy = fs(srt[j].py, pi.py);
-            const float r = len2(dx, dy);
-            if (r > 0.0000001f && r < k.h) {
-                const float4 sj = ps[j];
-                const float a = fs(1.f, fd(r, k.h));
-                const float near = fm(fm(fm(fm(fa(si.w, sj.w), a), a), a), k.kNearNorm);
-                const float far = fm(fm(fm(fa(si.z, sj.z), a), a), k.kNorm);
-                const float d = fd(fm(dt2, fa(near, far)), 2.f);
-                const float rm = fm(r, k.m);
-                ux = fd(fm(dx, d), rm);
-                uy = fd(fm(dy, d), rm);
-                const float surf = fd(fm(fm(fm(dt2, fd(kSurfaceTension, k.m)), k.m),
-                                         fa(fm(fm(fm(a, a), a), k.kNearNorm), fm(fm(a, a), k.kNorm))), 2.f);
-                wx = fm(surf, dx);
-                wy = fm(surf, dy);
-                in = true;
-            }
-        }
-        for (uint32_t m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
-            const int b = __ffs(m) - 1;
-            rx = fs(rx, __shfl_sync(0xffffffffu, ux, b));
-            ry = fs(ry, __shfl_sync(0xffffffffu, uy, b));
-            rx = fa(rx, __shfl_sync(0xffffffffu, wx, b));
-            ry = fa(ry, __shfl_sync(0xffffffffu, wy, b));
-        }
-    }
-    if (lane != 0) return;
-    const float4 wall = sample(bstate, k.W, k.H, fd(rx, k.cW), fd(ry, k.cH));
-    if (wall.x != 0.f) {
-        const float4 normal = sample(bvec, k.W, k.H, fd(rx, k.cW), fd(ry, k.cH));
-        const float a = fs(1.f, fd(normal.z, k.h));
-        const float near = fm(fm(fm(fm(fa(si.w, wall.w), a), a), a), k.kNearNorm);
-        const float far = fm(fm(fm(fa(si.z, wall.z), a), a), k.kNorm);
-        const float d = fd(fm(dt2, fa(near, far)), 2.f);
-        rx = fa(rx, fd(fm(normal.x, d), k.m));
-        ry = fa(ry, fd(fm(normal.y, d), k.m));
-    }
-    relaxed[i] = make_float2(rx, ry);
-}
-
-// clUpdateState (libCL/phys/oclFluid2D.cl:329-339).
-__global__ void k2_update(P2* __restrict__ st, const float2* __restrict__ prev, const float2* __restrict__ relaxed,
-                          const uint32_t* __restrict__ index, K2 k) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= k.n) return;
-    const uint32_t o = index[i];
-    const float2 pr = prev[o], rl = relaxed[i];
-    float dx = fs(rl.x, pr.x), dy = fs(rl.y, pr.y);
+// clUpdateState (libCL/phys/oclFluid2D.cl:329-339) of particle o, relaxed to (rx, ry).
+__device__ __forceinline__ void update_state(P2* __restrict__ st, const float2* __restrict__ prev, uint32_t o, float rx, float ry,
+                                             const K2& k) {
+    const float2 pr = prev[o];
+    float dx = fs(rx, pr.x), dy = fs(ry, pr.y);
     const float l = len2(dx, dy);
     const float cap = fm(4.0f, k.psize);
     const float lim = (cap < l) ? cap : l;  // min(l, 4 * particleSize) with the restatement's NaN rule
@@ -282,6 +164,330 @@ __global__ void k2_update(P2* __restrict__ st, const float2* __restrict__ prev, 
     p.px = fa(pr.x, dx);
     p.py = fa(pr.y, dy);
     st[o] = p;
+}
+
+// The neighbour loops of clComputePressure / clComputePosition visit cells x (outer), y (inner)
+// of the 3 x 3 around a particle and the particles of each cell in sorted order, summing in
+// that order. A warp takes SEARCH_TARGETS consecutive sorted particles and
+//  - for each cell among them goes through the candidates of the nine cells, 32 at a time in
+//    the reference's order, keeps those within h of the box around the cell's targets (no
+//    target is nearer to a candidate than the box, in rounded arithmetic as well: every
+//    operation of the distance is monotone), tests the kept ones against each target and
+//    appends those in range to the target's list;
+//  - then computes the terms of all lists, a lane each, and a lane per target adds them in order.
+// A target with more in range than its list holds is summed by the warp on its own, through the
+// candidates again. At 16,384 particles (the default scene) a warp for every particle, its
+// candidates' terms computed wherever one of 32 was in range and added by shuffles, took 33 us for
+// the pressures and 43 for the positions; this takes 15 and 18. Bound by latency: 27 warps an
+// SM, each a chain of table, candidates, lists, terms and sums. Two targets per warp are no
+// better at this size (116 against 102 us for two steps; 78 against 94 at 4,096), eight 113,
+// and all nine cells instead of those in reach 136.
+constexpr int SEARCH_WARPS = 4;           // per CTA
+constexpr int SEARCH_TARGETS = 4;         // per warp
+constexpr uint32_t LIST2 = 64;            // entries of a target's list
+constexpr uint32_t HELD2 = 128;           // candidates held before they are tested, a multiple of 32
+
+template <class TERM>
+struct Search2 {
+    float2 xy[HELD2];
+    uint32_t id[HELD2];
+    uint32_t base[32];
+    uint32_t j[SEARCH_TARGETS][LIST2];
+    TERM term[SEARCH_TARGETS][LIST2];  // first the neighbour's distance (x, y), then its terms
+};
+
+// Whether particle j at distance (dx, dy) is a neighbour of particle i: r > 1e-7 and r < h.
+__device__ __forceinline__ bool near2(const K2& k, float dx, float dy) {
+    const float r2 = fa(fm(dx, dx), fm(dy, dy));
+    return r2 >= k.r2_lo && r2 < k.r2_hi;
+}
+
+// The candidates of cell (cx, cy) that may be within h of the box (xl..xh, yl..yh): calls
+// f(j, px, py) for 32 at a time (j = EMPTY2 beyond the last), in the reference's order, by the
+// whole warp. Cells are 2 h wide, so that a box in one cell reaches four to six of the nine;
+// the slack is a hundred times what rounding can move a particle against its cell's bounds, and
+// the cells at the grid's edges hold what lies beyond as well.
+template <class F>
+__device__ __forceinline__ void for_candidates2(const K2& k, int cx, int cy, const P2* __restrict__ srt,
+                                                const uint2* __restrict__ table, uint32_t* __restrict__ s_base, float xl, float xh, float yl,
+                                                float yh, F&& f) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
+    uint32_t n = 0, first = 0;
+    if (lane < 9) {
+        const int x = cx - 1 + (int)lane / 3, y = cy - 1 + (int)lane % 3;
+        // out of reach beyond cell c of m: the box lies outside [c, c + 1] cells, give or take h
+        auto far = [&](int c, int m, float lo, float hi) {
+            const float from = (float)c * k.cellSize, to = from + k.cellSize, reach = k.h + 1e-5f * (k.h + to);
+            return (c > 0 && from - hi > reach) || (c < m - 1 && lo - to > reach);
+        };
+        if (x >= 0 && x < k.ncx && y >= 0 && y < k.ncy && !far(x, k.ncx, xl, xh) && !far(y, k.ncy, yl, yh)) {
+            const uint2 e = table[y * k.ncx + x];
+            if (e.x != EMPTY2) {
+                first = e.x;
+                n = e.y - e.x;
+            }
+        }
+    }
+    uint32_t off = n;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(FULL, off, d);
+        if ((int)lane >= d) off += o;
+    }
+    const uint32_t total = __shfl_sync(FULL, off, 8), some = __ballot_sync(FULL, n != 0);
+    off -= n;
+    __syncwarp();
+    if (n) s_base[__popc(some & lt)] = first - off;
+    __syncwarp();
+    uint32_t seen = 0;
+    auto fetch = [&](uint32_t base, float& px, float& py) -> uint32_t {
+        const uint32_t heads = __reduce_or_sync(FULL, n && off - base < 32u ? 1u << (off - base) : 0u);
+        const uint32_t r = seen + (uint32_t)__popc(heads & (lt | 1u << lane)) - 1u;
+        seen += (uint32_t)__popc(heads);
+        if (base + lane >= total) return EMPTY2;
+        const uint32_t j = base + lane + s_base[r];
+        px = srt[j].px;
+        py = srt[j].py;
+        return j;
+    };
+    float px = 0.f, py = 0.f, ax = 0.f, ay = 0.f;
+    uint32_t j = fetch(0, px, py), next = EMPTY2;
+    for (uint32_t base = 0; base < total; base += 32, j = next, px = ax, py = ay) {
+        if (base + 32 < total) next = fetch(base + 32, ax, ay);
+        f(j, px, py);
+    }
+}
+
+// Fills the lists of the warp's targets; lane t's `count` is that of target t (may exceed LIST2).
+template <class TERM>
+__device__ __forceinline__ uint32_t search2(Search2<TERM>& S, const K2& k, uint32_t first, bool live, float px, float py,
+                                            const P2* __restrict__ srt, const uint2* __restrict__ table) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
+    const int gx = (int)floorf(fd(px, k.cellSize)), gy = (int)floorf(fd(py, k.cellSize));
+    uint32_t count = 0;
+    for (uint32_t left = __ballot_sync(FULL, live); left;) {
+        const int lead = __ffs(left) - 1;
+        const int cx = __shfl_sync(FULL, gx, lead), cy = __shfl_sync(FULL, gy, lead);
+        const uint32_t group = __ballot_sync(FULL, live && gx == cx && gy == cy);
+        left &= ~group;
+        const bool in = (group >> lane) & 1u;
+        const float x0 = __shfl_sync(FULL, px, lead), y0 = __shfl_sync(FULL, py, lead);
+        const float xl = warp_min(in ? px : x0), xh = warp_max(in ? px : x0), yl = warp_min(in ? py : y0), yh = warp_max(in ? py : y0);
+        uint32_t held = 0;
+        auto test = [&]() {
+            if (held + lane < ((held + 31u) & ~31u)) S.xy[held + lane].x = INFINITY;  // never in range
+            __syncwarp();
+            for (uint32_t g = group; g; g &= g - 1) {
+                const int t = __ffs(g) - 1;
+                const float x = __shfl_sync(FULL, px, t), y = __shfl_sync(FULL, py, t);
+                const uint32_t self = first + (uint32_t)t;
+                uint32_t c = __shfl_sync(FULL, count, t);
+                for (uint32_t p = 0; p < held; p += 32) {
+                    const float2 q = S.xy[p + lane];
+                    const uint32_t j = S.id[p + lane];
+                    const float dx = fs(q.x, x), dy = fs(q.y, y);
+                    const bool hit = near2(k, dx, dy) && j != self;
+                    const uint32_t m = __ballot_sync(FULL, hit), at = c + (uint32_t)__popc(m & lt);
+                    c += (uint32_t)__popc(m);
+                    if (hit && at < LIST2) {
+                        S.j[t][at] = j;
+                        S.term[t][at].x = dx;
+                        S.term[t][at].y = dy;
+                    }
+                }
+                if ((int)lane == t) count = c;
+            }
+            __syncwarp();
+            held = 0;
+        };
+        for_candidates2(k, cx, cy, srt, table, S.base, xl, xh, yl, yh, [&](uint32_t j, float qx, float qy) {
+            const float dx = fmaxf(fmaxf(fs(xl, qx), fs(qx, xh)), 0.f), dy = fmaxf(fmaxf(fs(yl, qy), fs(qy, yh)), 0.f);
+            const bool keep = j != EMPTY2 && fa(fm(dx, dx), fm(dy, dy)) < k.r2_hi;
+            const uint32_t m = __ballot_sync(FULL, keep);
+            if (keep) {
+                const uint32_t at = held + (uint32_t)__popc(m & lt);
+                S.xy[at] = make_float2(qx, qy);
+                S.id[at] = j;
+            }
+            held += (uint32_t)__popc(m);
+            if (held > HELD2 - 32) test();
+        });
+        if (held) test();
+    }
+    __syncwarp();
+    return count;
+}
+
+// Calls f(t, entry) for every entry of the lists, a lane each (lane t's `n` entries of target t).
+template <class F>
+__device__ __forceinline__ void for_entries2(uint32_t n, F&& f) {
+    constexpr int T = SEARCH_TARGETS;
+    uint32_t before[T + 1];
+    before[0] = 0;
+#pragma unroll
+    for (int t = 0; t < T; ++t) before[t + 1] = before[t] + __shfl_sync(0xffffffffu, n, t);
+    for (uint32_t e = threadIdx.x & 31u; e < before[T]; e += 32) {
+        int t = 0;
+        uint32_t at = e;
+#pragma unroll
+        for (int q = 1; q < T; ++q)
+            if (e >= before[q]) {
+                t = q;
+                at = e - before[q];
+            }
+        f(t, at);
+    }
+    __syncwarp();
+}
+
+struct Pressure2 {
+    // the terms of a neighbour at distance r
+    static __device__ __forceinline__ float2 term(const K2& k, float dx, float dy) {
+        const float a = fs(1.f, fd(len2(dx, dy), k.h));
+        return make_float2(fm(fm(fm(fm(k.m, a), a), a), k.kNorm), fm(fm(fm(fm(fm(k.m, a), a), a), a), k.kNearNorm));
+    }
+};
+
+// clComputePressure (libCL/phys/oclFluid2D.cl:185-245).
+__global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_pressure(const P2* __restrict__ srt, float4* __restrict__ ps,
+                                                                 const uint2* __restrict__ table,
+                                                                 const float4* __restrict__ bstate, K2 k) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    __shared__ Search2<float2> shared[SEARCH_WARPS];
+    Search2<float2>& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * SEARCH_TARGETS, i = first + lane;
+    const bool live = lane < SEARCH_TARGETS && i < k.n;
+    if (first >= k.n) return;  // whole warps
+    const float px = live ? srt[i].px : 0.f, py = live ? srt[i].py : 0.f;
+    const uint32_t count = search2<float2>(S, k, first, live, px, py, srt, table);
+    for_entries2(count <= LIST2 ? count : 0u, [&](int t, uint32_t e) {
+        const float2 d = S.term[t][e];
+        S.term[t][e] = Pressure2::term(k, d.x, d.y);
+    });
+    float density = 0.f, nearDensity = 0.f;
+    if (live) {
+        const float4 wall = sample(bstate, k.W, k.H, fd(px, k.cW), fd(py, k.cH));
+        if (wall.x != 0.f) {
+            density = fa(density, wall.x);
+            nearDensity = fa(nearDensity, wall.y);
+        }
+        if (count <= LIST2) {
+#pragma unroll 4
+            for (uint32_t e = 0; e < count; ++e) {
+                const float2 v = S.term[lane][e];
+                density = fa(density, v.x);
+                nearDensity = fa(nearDensity, v.y);
+            }
+        }
+    }
+    for (uint32_t more = __ballot_sync(FULL, live && count > LIST2); more; more &= more - 1) {
+        const int t = __ffs(more) - 1;
+        const uint32_t self = first + (uint32_t)t;
+        const float x = __shfl_sync(FULL, px, t), y = __shfl_sync(FULL, py, t);
+        for_candidates2(k, (int)floorf(fd(x, k.cellSize)), (int)floorf(fd(y, k.cellSize)), srt, table, S.base, x, x, y, y,
+                        [&](uint32_t j, float qx, float qy) {
+                            const float dx = fs(qx, x), dy = fs(qy, y);
+                            const bool hit = j != EMPTY2 && j != self && near2(k, dx, dy);
+                            const float2 v = hit ? Pressure2::term(k, dx, dy) : make_float2(0.f, 0.f);
+                            for (uint32_t m = __ballot_sync(FULL, hit); m; m &= m - 1) {
+                                const int b = __ffs(m) - 1;
+                                const float vx = __shfl_sync(FULL, v.x, b), vy = __shfl_sync(FULL, v.y, b);
+                                if ((int)lane == t) {
+                                    density = fa(density, vx);
+                                    nearDensity = fa(nearDensity, vy);
+                                }
+                            }
+                        });
+    }
+    if (live)
+        ps[i] = make_float4(density, nearDensity, fm(kStiffness, fs(density, fm(k.m, kRestDensity))),
+                            fm(kNearStiffness, nearDensity));
+}
+
+struct Position2 {
+    // displacements (away by pressure: x, y; towards by surface tension: z, w)
+    static __device__ __forceinline__ float4 term(const K2& k, float dt2, float tension, const float4& si, const float4& sj, float dx,
+                                                  float dy) {
+        const float r = len2(dx, dy);
+        const float a = fs(1.f, fd(r, k.h));
+        const float near = fm(fm(fm(fm(fa(si.w, sj.w), a), a), a), k.kNearNorm);
+        const float far = fm(fm(fm(fa(si.z, sj.z), a), a), k.kNorm);
+        const float d = fd(fm(dt2, fa(near, far)), 2.f);
+        const float rm = fm(r, k.m);
+        const float surf = fd(fm(tension, fa(fm(fm(fm(a, a), a), k.kNearNorm), fm(fm(a, a), k.kNorm))), 2.f);
+        return make_float4(fd(fm(dx, d), rm), fd(fm(dy, d), rm), fm(surf, dx), fm(surf, dy));
+    }
+};
+
+// clComputePosition (libCL/phys/oclFluid2D.cl:247-326) and, as it concerns the particle alone,
+// clUpdateState. The reference's viscosity term uses vel_j - vel_j (:299), which is zero, so
+// it never contributes and is not evaluated here.
+__global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_position(const P2* __restrict__ srt, const float4* __restrict__ ps,
+                                                                 float2* __restrict__ relaxed, const uint2* __restrict__ table,
+                                                                 const float4* __restrict__ bstate,
+                                                                 const float4* __restrict__ bvec, P2* __restrict__ st,
+                                                                 const float2* __restrict__ prev,
+                                                                 const uint32_t* __restrict__ index, K2 k) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    __shared__ Search2<float4> shared[SEARCH_WARPS];
+    Search2<float4>& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * SEARCH_TARGETS, i = first + lane;
+    const bool live = lane < SEARCH_TARGETS && i < k.n;
+    if (first >= k.n) return;  // whole warps
+    const float px = live ? srt[i].px : 0.f, py = live ? srt[i].py : 0.f;
+    const float dt2 = fm(k.dT, k.dT), tension = fm(fm(dt2, fd(kSurfaceTension, k.m)), k.m);
+    const uint32_t count = search2<float4>(S, k, first, live, px, py, srt, table);
+    for_entries2(count <= LIST2 ? count : 0u, [&](int t, uint32_t e) {
+        const float4 d = S.term[t][e];
+        S.term[t][e] = Position2::term(k, dt2, tension, ps[first + t], ps[S.j[t][e]], d.x, d.y);
+    });
+    float rx = px, ry = py;
+    if (live && count <= LIST2) {
+#pragma unroll 4
+        for (uint32_t e = 0; e < count; ++e) {
+            const float4 v = S.term[lane][e];
+            rx = fa(fs(rx, v.x), v.z);
+            ry = fa(fs(ry, v.y), v.w);
+        }
+    }
+    for (uint32_t more = __ballot_sync(FULL, live && count > LIST2); more; more &= more - 1) {
+        const int t = __ffs(more) - 1;
+        const uint32_t self = first + (uint32_t)t;
+        const float x = __shfl_sync(FULL, px, t), y = __shfl_sync(FULL, py, t);
+        const float4 si = ps[self];
+        for_candidates2(k, (int)floorf(fd(x, k.cellSize)), (int)floorf(fd(y, k.cellSize)), srt, table, S.base, x, x, y, y,
+                        [&](uint32_t j, float qx, float qy) {
+                            const float dx = fs(qx, x), dy = fs(qy, y);
+                            const bool hit = j != EMPTY2 && j != self && near2(k, dx, dy);
+                            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (hit) v = Position2::term(k, dt2, tension, si, ps[j], dx, dy);
+                            for (uint32_t m = __ballot_sync(FULL, hit); m; m &= m - 1) {
+                                const int b = __ffs(m) - 1;
+                                const float ux = __shfl_sync(FULL, v.x, b), uy = __shfl_sync(FULL, v.y, b);
+                                const float wx = __shfl_sync(FULL, v.z, b), wy = __shfl_sync(FULL, v.w, b);
+                                if ((int)lane == t) {
+                                    rx = fa(fs(rx, ux), wx);
+                                    ry = fa(fs(ry, uy), wy);
+                                }
+                            }
+                        });
+    }
+    if (!live) return;
+    const float4 si = ps[i];
+    const float4 wall = sample(bstate, k.W, k.H, fd(rx, k.cW), fd(ry, k.cH));
+    if (wall.x != 0.f) {
+        const float4 normal = sample(bvec, k.W, k.H, fd(rx, k.cW), fd(ry, k.cH));
+        const float a = fs(1.f, fd(normal.z, k.h));
+        const float near = fm(fm(fm(fm(fa(si.w, wall.w), a), a), a), k.kNearNorm);
+        const float far = fm(fm(fm(fa(si.z, wall.z), a), a), k.kNorm);
+        const float d = fd(fm(dt2, fa(near, far)), 2.f);
+        rx = fa(rx, fd(fm(normal.x, d), k.m));
+        ry = fa(ry, fd(fm(normal.y, d), k.m));
+    }
+    relaxed[i] = make_float2(rx, ry);
+    update_state(st, prev, index[i], rx, ry, k);
 }
 
 // clComputeBorder (libCL/phys/oclFluid2D.cl:358-443), one thread per pixel.
@@ -372,9 +578,10 @@ struct gbsph_fluid2d_s {
     float2* relaxed = nullptr;
     float2* prev = nullptr;
     uint32_t *keys_a = nullptr, *keys_b = nullptr, *keys_c = nullptr, *vals_a = nullptr, *vals_b = nullptr, *index = nullptr;
-    uint32_t* cs = nullptr;  // cell start / end, `table` entries each
-    uint32_t* ce = nullptr;
-    uint32_t table = 256;
+    uint2* cells = nullptr;  // cell start, end: `table` entries (whole scan tiles allocated)
+    uint32_t* count = nullptr;  // the counting sort's counts, behind them, zero between steps
+    bool count_clean = false;
+    uint32_t table = 0;
     float4* bstate = nullptr;  // wall images W x H
     float4* bvec = nullptr;
     int W = 256, Hh = 256;
@@ -427,6 +634,8 @@ K2 make_k2(const H2* h) {
     k.table = h->table;
     k.W = h->W;
     k.H = h->Hh;
+    k.r2_lo = r2_threshold(std::nextafter(0.0000001f, 1.0f));
+    k.r2_hi = r2_threshold(p.h);
     return k;
 }
 
@@ -458,7 +667,7 @@ int alloc_arrays2(H2* h, size_t n) {
         *a = (uint32_t*)p;
         p += n4 * 4;
     }
-    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, onesweep_scratch_bytes((uint32_t)n, SORT_MAX_PASSES)));
+    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->scratch, sort_scratch_bytes((uint32_t)n)));
     return GBSPH_OK;
 }
 
@@ -490,12 +699,15 @@ int alloc_border2(H2* h, int w, int hh) {
 int alloc_table2(H2* h) {
     const gbsph_fluid2d_params& p = h->params;
     const uint32_t t = (uint32_t)(p.cellCountX * p.cellCountY) / 256 * 256 + 256;
-    if (h->cs && t == h->table) return GBSPH_OK;
-    if (h->cs) cudaFree(h->cs);
-    h->cs = h->ce = nullptr;
-    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->cs, 2 * (size_t)t * 4));
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->cs, 0xFF, 2 * (size_t)t * 4));
-    h->ce = h->cs + t;
+    if (h->cells && t == h->table) return GBSPH_OK;
+    if (h->cells) cudaFree(h->cells);
+    h->cells = nullptr;
+    h->count = nullptr;
+    const size_t words = count_words(t);
+    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->cells, words * 12));
+    GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->cells, 0xFF, words * 8));
+    h->count = (uint32_t*)(h->cells + words);
+    h->count_clean = false;
     h->table = t;
     invalidate2(h);
     return GBSPH_OK;
@@ -514,33 +726,55 @@ int bits_for2(uint64_t cells) {
     } while (0)
 
 int enqueue2(H2* h, const K2& k, cudaStream_t s) {
-    const int end_bit = bits_for2((uint64_t)h->params.cellCountX * h->params.cellCountY);
-    const int P = sort_passes(0, end_bit);
-    GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, k.n, P, s));
-    const int blocks = std::max(1, std::min(grid1(k.n), num_sms() * 8));
-    k2_advance_hash<<<blocks, 256, 0, s>>>((P2*)h->state, h->prev, h->keys_a, (uint32_t*)h->scratch, k, end_bit);
-    GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
-    OnesweepArgs a;
-    a.keys_in = h->keys_a;
-    a.keys_out = h->keys_c;
-    a.vals_out = h->index;
-    a.tmp_keys[0] = h->keys_b;
-    a.tmp_vals[0] = h->vals_b;
-    a.tmp_keys[1] = h->keys_a;
-    a.tmp_vals[1] = h->vals_a;
-    a.n = k.n;
-    a.start_bit = 0;
-    a.end_bit = end_bit;
-    a.scratch = h->scratch;
-    a.err = h->err;
-    GBSPH_CUDA_TRY(&h->last_error, onesweep_passes(a, s));
-    k2_reorder<<<grid1(k.n), 256, 0, s>>>(h->index, (const P2*)h->state, h->sorted, k.n);
-    GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
-    GBSPH_CUDA_TRY(&h->last_error, cell_bounds_launch(h->keys_c, k.n, h->cs, h->ce, h->table, h->err, s));
-    const unsigned wgrid = (unsigned)(((size_t)k.n * 32 + 255) / 256);  // a warp per particle
-    k2_pressure<<<wgrid, 256, 0, s>>>(h->sorted, h->pstate, h->cs, h->ce, h->bstate, k);
-    k2_position<<<wgrid, 256, 0, s>>>(h->sorted, h->pstate, h->relaxed, h->cs, h->ce, h->bstate, h->bvec, k);
-    k2_update<<<grid1(k.n), 256, 0, s>>>((P2*)h->state, h->prev, h->relaxed, h->index, k);
+    const unsigned g = (unsigned)grid1(k.n);
+    P2* state = (P2*)h->state;
+    if (count_sort_fits(k.table, k.n)) {
+        const uint32_t tiles = scan_tiles(k.table);
+        uint32_t* sums = (uint32_t*)((char*)h->scratch + SORT_HEADER_BYTES);
+        uint2* slots = (uint2*)h->vals_a;  // and vals_b behind it
+        k2_advance_count<<<g, 256, 0, s>>>(state, h->prev, h->keys_a, h->keys_b, h->count, k);
+        if (k.table <= SCAN_DIRECT) {
+            k_scan_cells<4, true, true><<<tiles, SCAN_THREADS, 0, s>>>(h->count, h->cells, sums);
+        } else if (scan_items(k.table) == 4) {
+            k_tile_sums<4><<<tiles, SCAN_THREADS, 0, s>>>(h->count, sums);
+            k_scan_cells<4, true, false><<<tiles, SCAN_THREADS, 0, s>>>(h->count, h->cells, sums);
+        } else {
+            k_tile_sums<16><<<tiles, SCAN_THREADS, 0, s>>>(h->count, sums);
+            k_scan_cells<16, true, false><<<tiles, SCAN_THREADS, 0, s>>>(h->count, h->cells, sums);
+        }
+        k_scatter_ids<<<g, 256, 0, s>>>(h->keys_a, h->keys_b, h->cells, slots, k.n, h->err);
+        k2_order<<<g, 256, 0, s>>>(slots, h->cells, state, h->keys_c, h->index, h->sorted, h->count, k, h->err);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+    } else {
+        const int end_bit = bits_for2((uint64_t)h->params.cellCountX * h->params.cellCountY);
+        const int P = sort_passes(0, end_bit);
+        GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, k.n, P, s));
+        const int blocks = std::max(1, std::min(grid1(k.n), num_sms() * 8));
+        k2_advance_hash<<<blocks, 256, 0, s>>>(state, h->prev, h->keys_a, (uint32_t*)h->scratch, k, end_bit);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+        OnesweepArgs a;
+        a.keys_in = h->keys_a;
+        a.keys_out = h->keys_c;
+        a.vals_out = h->index;
+        a.tmp_keys[0] = h->keys_b;
+        a.tmp_vals[0] = h->vals_b;
+        a.tmp_keys[1] = h->keys_a;
+        a.tmp_vals[1] = h->vals_a;
+        a.n = k.n;
+        a.start_bit = 0;
+        a.end_bit = end_bit;
+        a.scratch = h->scratch;
+        a.err = h->err;
+        GBSPH_CUDA_TRY(&h->last_error, onesweep_passes(a, s));
+        k2_reorder<<<g, 256, 0, s>>>(h->index, state, h->sorted, k.n);
+        GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->cells, 0xFF, (size_t)k.table * 8, s));
+        k_bounds_hash<<<g, 256, 0, s>>>(h->keys_c, k.n, h->cells, k.table, h->err);
+        GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
+    }
+    const uint32_t per = SEARCH_TARGETS * SEARCH_WARPS, blocks = (k.n + per - 1) / per;
+    k2_pressure<<<blocks, 32 * SEARCH_WARPS, 0, s>>>(h->sorted, h->pstate, h->cells, h->bstate, k);
+    k2_position<<<blocks, 32 * SEARCH_WARPS, 0, s>>>(h->sorted, h->pstate, h->relaxed, h->cells, h->bstate, h->bvec, state, h->prev,
+                                                     h->index, k);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
@@ -595,7 +829,7 @@ GBSPH_API int gbsph_fluid2d_destroy(gbsph_fluid2d_t h) {
     cudaSetDevice(h->device);
     invalidate2(h);
     if (h->state_owned && h->state) cudaFree(h->state);
-    void* ptrs[6] = {h->block, h->scratch, h->cs, h->bstate, h->bvec, h->err};
+    void* ptrs[6] = {h->block, h->scratch, h->cells, h->bstate, h->bvec, h->err};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->cap_stream) cudaStreamDestroy(h->cap_stream);
@@ -722,7 +956,12 @@ GBSPH_API int gbsph_fluid2d_compute(gbsph_fluid2d_t h, void* stream) {
         }
         h->gkey = key;
     }
+    // the step leaves the counts as it finds them, all zero
+    if (!h->count_clean)
+        GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, count_words(h->table) * 4, (cudaStream_t)stream));
+    h->count_clean = false;
     GBSPH_CUDA_TRY(&h->last_error, cudaGraphLaunch(h->gexec, (cudaStream_t)stream));
+    h->count_clean = true;
     return GBSPH_OK;
 }
 
@@ -733,8 +972,8 @@ GBSPH_API int gbsph_fluid2d_get_cell_bounds(gbsph_fluid2d_t h, uint32_t* cell_st
         return fail(&h->last_error, GBSPH_ERR_SIZE_MISMATCH, "n_cells must equal the table size");
     GBSPH_CUDA_TRY(&h->last_error, cudaSetDevice(h->device));
     cudaStream_t s = (cudaStream_t)stream;
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemcpyAsync(cell_start, h->cs, n_cells * 4, cudaMemcpyDeviceToDevice, s));
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemcpyAsync(cell_end, h->ce, n_cells * 4, cudaMemcpyDeviceToDevice, s));
+    k_table_split<<<grid1((uint32_t)n_cells), 256, 0, s>>>(h->cells, (uint32_t)n_cells, cell_start, cell_end);
+    GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
 
