@@ -1,8 +1,10 @@
 // adjoint3d.cu -- host side of the 3D step's adjoint (gbsph_adjoint3d_*).
 //
 // forward(): `steps` ordinary compute() calls on the fluid, with a copy of (position, velocity,
-// force) taken before every K-th step. backward(): for each segment of K steps, last first,
-// the fluid is reset to the segment's checkpoint and stepped again with force recording on;
+// force) taken before every K-th step; the steps of the last segment are recorded as they are
+// made. backward(): for each segment of K steps, last first, the fluid is reset to the
+// segment's checkpoint and stepped again with recording on (not the last one, as long as the
+// tape still holds it: 30 steps for 20 with K = 10 where there were 40);
 // after each step the permutation, sorted keys, sorted state and the force after the clip box
 // are copied into the segment's tape (one kernel), and the density pass writes each
 // particle's neighbour list (sorted indices) into the step's tape slot. The step's adjoint
@@ -38,6 +40,7 @@ struct gbsph_adjoint3d_s {
     uint2* tables = nullptr;  // two cell tables, used by alternate steps
     size_t table_cells = 0;
     bool forward_done = false;
+    bool last_taped = false;  // the tape holds the last segment's steps
     gbsph_fluid3d_params params{};
     std::string last_error;
 };
@@ -108,19 +111,27 @@ struct RecordGuard {
     ~RecordGuard() { fluid3d_set_record(f, nullptr); }
 };
 
+void record_on(A* a) { fluid3d_set_record(a->fluid, a->rec, a->lists, a->lcnt, a->slot_dev, (uint32_t)a->n4); }
+
+// One step of the fluid, recorded in tape slot k.
+int record_step(A* a, const FluidAccess& fa, uint32_t k, const char* what, cudaStream_t s) {
+    GBSPH_CUDA_TRY(&a->last_error, cudaMemcpyAsync(a->slot_dev, a->slot_ids + k, 4, cudaMemcpyDeviceToDevice, s));
+    // no list unless the step's density pass records one (the per-stage kernels do not)
+    GBSPH_CUDA_TRY(&a->last_error, cudaMemsetAsync(a->lcnt + (size_t)k * a->n4, 0xFF, a->n4 * 4, s));
+    const int rc = gbsph_fluid3d_compute(a->fluid, (void*)s);
+    if (rc) return fail(&a->last_error, rc, std::string(what) + gbsph_fluid3d_last_error(a->fluid));
+    k_tape_record<<<grid1(a->n), 256, 0, s>>>(slot(a, k), fa.index, fa.keys, fa.spos, fa.svel, a->rec, (uint32_t)a->n);
+    GBSPH_CUDA_TRY(&a->last_error, cudaGetLastError());
+    return GBSPH_OK;
+}
+
 int backward_segment(A* a, const FluidAccess& fa, const KParams& kp, uint32_t seg, float c45, cudaStream_t s) {
     const uint32_t s0 = seg * a->every, s1 = std::min(a->steps, s0 + a->every);
-    RC(copy_state(a, fa, a->ckpt + (size_t)seg * 3 * a->n4, true, s));
-    for (uint32_t st = s0; st < s1; st++) {
-        const uint32_t k = st - s0;  // the tape slot this step's lists go to
-        GBSPH_CUDA_TRY(&a->last_error, cudaMemcpyAsync(a->slot_dev, a->slot_ids + k, 4, cudaMemcpyDeviceToDevice, s));
-        // no list unless the step's density pass records one (the per-stage kernels do not)
-        GBSPH_CUDA_TRY(&a->last_error, cudaMemsetAsync(a->lcnt + (size_t)k * a->n4, 0xFF, a->n4 * 4, s));
-        const int rc = gbsph_fluid3d_compute(a->fluid, (void*)s);
-        if (rc) return fail(&a->last_error, rc, std::string("recompute: ") + gbsph_fluid3d_last_error(a->fluid));
-        k_tape_record<<<grid1(a->n), 256, 0, s>>>(slot(a, st - s0), fa.index, fa.keys, fa.spos, fa.svel, a->rec,
-                                                   (uint32_t)a->n);
-        GBSPH_CUDA_TRY(&a->last_error, cudaGetLastError());
+    if (seg + 1 < a->nseg || !a->last_taped) {
+        a->last_taped = false;
+        RC(copy_state(a, fa, a->ckpt + (size_t)seg * 3 * a->n4, true, s));
+        for (uint32_t st = s0; st < s1; st++) RC(record_step(a, fa, st - s0, "recompute: ", s));
+        a->last_taped = seg + 1 == a->nseg;
     }
     GBSPH_CUDA_TRY(&a->last_error, cudaMemsetAsync(a->tables, 0xFF, 2ull * a->table_cells * sizeof(uint2), s));
     for (uint32_t st = s1; st-- > s0;) {
@@ -206,19 +217,25 @@ GBSPH_API int gbsph_adjoint3d_destroy(gbsph_adjoint3d_t a) {
 
 GBSPH_API int gbsph_adjoint3d_forward(gbsph_adjoint3d_t a, void* stream) {
     if (!a) return GBSPH_ERR_ARGUMENT;
-    a->forward_done = false;
+    a->forward_done = a->last_taped = false;
     FluidAccess fa;
     KParams kp;
     RC(check_fluid(a, &fa, &kp));
     cudaStream_t s = (cudaStream_t)stream;
     for (uint32_t st = 0; st < a->steps; st++) {
         if (st % a->every == 0) RC(copy_state(a, fa, a->ckpt + (size_t)(st / a->every) * 3 * a->n4, false, s));
-        const int rc = gbsph_fluid3d_compute(a->fluid, stream);
-        if (rc) return fail(&a->last_error, rc, std::string("forward: ") + gbsph_fluid3d_last_error(a->fluid));
+        if (st / a->every + 1 == a->nseg) {
+            RecordGuard guard{a->fluid};
+            record_on(a);
+            RC(record_step(a, fa, st % a->every, "forward: ", s));
+        } else {
+            const int rc = gbsph_fluid3d_compute(a->fluid, stream);
+            if (rc) return fail(&a->last_error, rc, std::string("forward: ") + gbsph_fluid3d_last_error(a->fluid));
+        }
     }
     RC(copy_state(a, fa, a->fin, false, s));
     std::memcpy(&a->params, gbsph_fluid3d_get_params(a->fluid), sizeof(a->params));
-    a->forward_done = true;
+    a->forward_done = a->last_taped = true;
     return GBSPH_OK;
 }
 
@@ -247,12 +264,15 @@ GBSPH_API int gbsph_adjoint3d_backward(gbsph_adjoint3d_t a, const float* grad_po
     const float c45 = (float)(45.0 / (pi * std::pow((double)a->params.cellSize, 6.0)));
     {
         RecordGuard guard{a->fluid};
-        fluid3d_set_record(a->fluid, a->rec, a->lists, a->lcnt, a->slot_dev, (uint32_t)a->n4);
+        record_on(a);
         for (uint32_t seg = a->nseg; seg-- > 0;) RC(backward_segment(a, fa, kp, seg, c45, s));
     }
     RC(copy_state(a, fa, a->fin, true, s));
     if (grad_params) {
-        k_adj_reduce<<<1, 1024, 0, s>>>(a->acc, (uint32_t)a->n, grad_params);
+        const uint32_t shares = std::min<uint32_t>(ADJ_SHARES, ((uint32_t)a->n + 1023u) / 1024u);
+        double* sums = (double*)a->w;  // free by now
+        k_adj_reduce<<<shares, 256, 0, s>>>(a->acc, (uint32_t)a->n, sums);
+        k_adj_reduce<<<1, 256, 0, s>>>((const double2*)sums, shares, grad_params);
         GBSPH_CUDA_TRY(&a->last_error, cudaGetLastError());
     }
     if (grad_position0)

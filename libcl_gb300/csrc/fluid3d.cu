@@ -86,6 +86,8 @@ struct gbsph_fluid3d_s {
     size_t io_grav_n = 0;
     cudaGraphExec_t gexec_io = nullptr;
     std::vector<char> gkey_io;
+    cudaGraphExec_t gexec_rec = nullptr;  // of steps an adjoint records
+    std::vector<char> gkey_rec;
     // getParamBuffer: a device copy of `params`, refreshed on the stream before a step whenever
     // the host struct differs from the copy last written (`dparams_shadow`)
     gbsph_fluid3d_params* dparams = nullptr;
@@ -220,6 +222,9 @@ void invalidate_graph(H* h) {
     if (h->gexec_io) cudaGraphExecDestroy(h->gexec_io);
     h->gexec_io = nullptr;
     h->gkey_io.clear();
+    if (h->gexec_rec) cudaGraphExecDestroy(h->gexec_rec);
+    h->gexec_rec = nullptr;
+    h->gkey_rec.clear();
 }
 
 // Host state of gbsph_fluid3d_compute_host: three float4[n] inputs and outputs.
@@ -894,7 +899,7 @@ GBSPH_API int gbsph_fluid3d_stage_times(gbsph_fluid3d_t h, float* ms, int max_st
 namespace {
 
 // One step on `s`; with `io` (compute_host) the upload and download are part of it. The
-// default path replays a captured graph (one per kind: with and without host copies).
+// default path replays a captured graph (one per kind: plain, with host copies, recorded).
 int compute_impl(H* h, cudaStream_t s, const HostIO* io, bool io_graph) {
     RC(validate_params(h));
     GBSPH_CUDA_TRY(&h->last_error, cudaSetDevice(h->device));
@@ -925,8 +930,8 @@ int compute_impl(H* h, cudaStream_t s, const HostIO* io, bool io_graph) {
         std::memcpy(key.data() + o, io, sizeof(HostIO));
         std::memcpy(key.data() + o + sizeof(HostIO), &h->io_grav, sizeof(void*));
     }
-    cudaGraphExec_t& gexec = io ? h->gexec_io : h->gexec;
-    std::vector<char>& gkey = io ? h->gkey_io : h->gkey;
+    cudaGraphExec_t& gexec = io ? h->gexec_io : kp.rec_force ? h->gexec_rec : h->gexec;
+    std::vector<char>& gkey = io ? h->gkey_io : kp.rec_force ? h->gkey_rec : h->gkey;
     if (!gexec || key != gkey) {
         if (gexec) cudaGraphExecDestroy(gexec);
         gexec = nullptr;
