@@ -923,13 +923,13 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
         cp_async_mbar_arrive(full);
         ++fill;
     };
-    uint32_t b = 0;
-    if (lane == 0) b = atomicAdd(queue, 1u);
-    b = __shfl_sync(0xffffffffu, b, 0);
-    uint32_t bid = b < n_bricks ? bricks[b] : 0u;
+    // The first brick goes by the CTA's own number, the queue deals out those behind: a scene of
+    // few bricks is spared a trip to the queue, and the brick is read beside their number
+    // (`bricks` has a word per particle). 16,384 particles in 2D: a step 29.6 -> 25.5 us.
+    uint32_t b = blockIdx.x, bid = ld_relaxed_gpu(bricks + min(b, kp.n - 1u));
     while (b < n_bricks) {
         uint32_t nb = 0;  // the next brick's ticket, asked for early
-        if (lane == 0) nb = atomicAdd(queue, 1u);
+        if (lane == 0) nb = gridDim.x + atomicAdd(queue, 1u);
         const SceneDev* sc = BATCH ? kp.scenes + scene_of<2>(kp.scenes, kp.n_scenes, bid) : nullptr;
         const int nx = BATCH ? sc->nx : kp.nx, ny = BATCH ? sc->ny : kp.ny, nz = BATCH ? sc->nz : kp.nz;
         const uint32_t bxn = BATCH ? (uint32_t)sc->bxn : (uint32_t)kp.bxn;
