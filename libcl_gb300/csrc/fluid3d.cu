@@ -369,8 +369,10 @@ int st_sort(H* h, const KParams& kp, cudaStream_t s, bool gather, cudaEvent_t be
     return GBSPH_OK;
 }
 
+bool use_rank_sort(const H* h, const KParams& kp) { return h->opt_fused && rank_sort_fits(kp.table_cells, kp.n); }
+
 bool use_count_sort(const H* h, const KParams& kp) {
-    return h->count && count_sort_fits(kp.table_cells, kp.n) && count_words(kp.table_cells) <= h->count_words;
+    return !use_rank_sort(h, kp) && h->count && count_sort_fits(kp.table_cells, kp.n) && count_words(kp.table_cells) <= h->count_words;
 }
 
 int st_count_sort(H* h, const KParams& kp, cudaStream_t s, bool clear, bool gather_vel) {
@@ -392,7 +394,7 @@ int st_count_sort(H* h, const KParams& kp, cudaStream_t s, bool clear, bool gath
     a.err = h->err;
     a.clear = clear;
     a.full = !linear;
-    GBSPH_CUDA_TRY(&h->last_error, count_sort<false>(a, kp, s));
+    GBSPH_CUDA_TRY(&h->last_error, use_rank_sort(h, kp) ? rank_sort(a, kp, s) : count_sort<false>(a, kp, s));
     return GBSPH_OK;
 }
 
@@ -588,8 +590,11 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
     if (io) GBSPH_CUDA_TRY(&h->last_error, cudaStreamWaitEvent(s, h->io_ev[1], 0));
     // with host input the sort does not wait for the velocity upload: the sorted velocities
     // are gathered after it (before the density pass, which writes their w)
-    const bool counting = use_count_sort(h, kp);
-    if (counting) {
+    const bool ranking = use_rank_sort(h, kp), counting = use_count_sort(h, kp);
+    if (ranking) {
+        RC(mark(h, 1, s));
+        RC(st_count_sort(h, kp, s, clear, io == nullptr));
+    } else if (counting) {
         if (!h->count_clean) GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, h->count_words * 4, s));
         h->count_clean = false;
         RC(mark(h, 1, s));
@@ -608,7 +613,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
     };
     RC(mark(h, 2, s));
     if (linear) {
-        if (!counting) {
+        if (!counting && !ranking) {
             // counters were zeroed with the sort scratch in st_hash
             k_bounds_linear<<<(kp.n + BOUNDS_TILE - 1) / BOUNDS_TILE, 256, 0, s>>>(h->keys_c, kp, h->table, h->bricks, counters(h), h->err);
             GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
@@ -621,7 +626,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
         if (io) GBSPH_CUDA_TRY(&h->last_error, cudaStreamWaitEvent(s, h->io_ev[3], 0));
         RC(st_force_brick(h, kp, s, h->hook == nullptr));
     } else {
-        if (!counting) RC(st_bounds(h, kp, s, true));
+        if (!counting && !ranking) RC(st_bounds(h, kp, s, true));
         RC(gather_velocity());
         RC(mark(h, 3, s));
         RC(st_density_exact(h, kp, s, true));
