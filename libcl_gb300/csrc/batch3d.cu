@@ -52,7 +52,7 @@ static_assert(SORT_MAX_PASSES * SORT_RADIX * 4 <= STEP_SMEM, "hash phase layout"
 // integration, with a grid-wide barrier between phases. Every phase takes its work from an
 // atomic queue (sort tiles, brick ids) or strides over the grid, so the grid is whatever is
 // resident: occupancy x SMs. Data written by one phase and read by a later one is read
-// through L2 (ld_phase<true>) or by bulk copies after the barrier's proxy fence.
+// through L2 (ld_phase<true>, asynchronous copies).
 template <int ITEMS>
 __global__ void __launch_bounds__(BRICK_THREADS, 3) k_batch_step(BatchStepArgs a, KParams kp) {
     extern __shared__ float4 s_dyn[];

@@ -193,7 +193,7 @@ static __global__ void __launch_bounds__(256) k_scatter_ids(const uint32_t* __re
 }
 
 // Sorted keys, permutation and state: a slot's particle goes behind those of its cell with smaller
-// ids. With BRICKS the ids of the occupied bricks are appended to `bricks` (k_bounds_linear).
+// ids. With BRICKS the ids of the occupied bricks are appended to `bricks`.
 template <bool BRICKS, bool VEL, class BrickOf>
 __device__ __forceinline__ void order_cells(const uint2* __restrict__ slots, const uint2* __restrict__ table,
                                             const float4* __restrict__ pos, const float4* __restrict__ vel,

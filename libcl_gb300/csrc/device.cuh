@@ -1,5 +1,5 @@
 // device.cuh -- device-side helpers: relaxed global loads/stores for look-back words,
-// bulk-copy (TMA, non-tensor) + mbarrier wrappers with bounded waits, small vector ops.
+// mbarrier and asynchronous-copy wrappers with bounded waits, small vector ops.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -52,12 +52,6 @@ __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Orders this thread's generic-proxy accesses to global memory with its async-proxy ones
-// (bulk copies), both ways.
-__device__ __forceinline__ void fence_proxy_async_global() {
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-}
-
 // Load of data that another CTA of the same launch wrote before a grid-wide barrier: through
 // L2 only (ld.global.cg), never from a copy an earlier phase left in this SM's L1 or
 // read-only cache. COH = false is an ordinary load.
@@ -89,7 +83,7 @@ __device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
 }
 
-// ---- mbarrier + cp.async.bulk (global -> shared, no tensor map) ----------------------
+// ---- mbarrier + cp.async (global -> shared) -------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
@@ -103,10 +97,6 @@ __device__ __forceinline__ void mbar_inval(uint64_t* bar) {
 
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -129,17 +119,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
         "{\n\t.reg .b64 st;\n\t"
         "mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_addr(bar)),
         "r"(bytes)
-        : "memory");
-}
-
-// One bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned) from global to
-// this CTA's shared memory, completing on `bar`.
-__device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes,
-                                         uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
-        "[%3];" ::"r"(smem_addr(dst_smem)),
-        "l"(src_gmem), "r"(bytes), "r"(smem_addr(bar))
         : "memory");
 }
 

@@ -1,9 +1,9 @@
 // fluid3d.cu -- host side of the 3D SPH fluid: the oclFluid3D replacement behind the C ABI.
 //
 // One step (libCL/phys/oclFluid3D.cpp:293-342) is enqueued on the caller's stream as:
-//   memset(sort scratch) -> k_hash (+digit histogram, +sparse clear of last step's cells)
-//   -> one-sweep passes (last pass gathers sorted position/velocity = clReorder)
-//   -> cell bounds (+ occupied-brick list) -> density -> forces (+clip/integrate/gravity)
+//   sort by cell with the cell table, the occupied bricks and clReorder's gather (count_sort.cuh;
+//   where that does not fit: k_hash, one-sweep radix passes, bounds)
+//   -> density -> forces (+clip/integrate/gravity)
 // and, once the cell table is in steady state, replayed as a captured CUDA graph.
 #include <algorithm>
 #include <cmath>

@@ -16,8 +16,7 @@ namespace gbsph {
 //
 // Memory: thread 0's fences around the arrival make the CTA's writes before the barrier
 // visible to every CTA after it (plain loads; loads of lines an earlier phase may have left
-// in L1 or the read-only cache go through ld_phase<true>). The proxy fences order the writes
-// with bulk copies (async proxy) that read them after the barrier.
+// in L1 or the read-only cache go through ld_phase<true>, and asynchronous copies through L2).
 struct GridSync {
     uint32_t* w;     // [0] arrivals, [1] barriers completed, [2] abort flag
     uint32_t* err;   // device error word
@@ -25,7 +24,6 @@ struct GridSync {
     uint32_t ctas;   // CTAs that arrive at each barrier (gridDim.x)
 
     __device__ __forceinline__ bool sync(uint32_t* s_flag) {
-        fence_proxy_async_global();  // this thread's writes, before bulk copies read them
         __syncthreads();
         const uint32_t target = ++epoch;
         if (threadIdx.x == 0) {
@@ -50,7 +48,6 @@ struct GridSync {
                 }
             }
             __threadfence();
-            fence_proxy_async_global();  // bulk copies issued after the barrier see the writes
             if (ld_relaxed_gpu(w + 2)) ok = false;
             *s_flag = ok ? 1u : 0u;
         }

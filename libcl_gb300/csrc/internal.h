@@ -14,7 +14,7 @@ namespace gbsph {
 // with atomicOr and keep going (or return); the host reads the word in *_sync_status.
 enum : uint32_t {
     DEV_ERR_LOOKBACK_TIMEOUT = 1u,  // decoupled look-back spin hit its limit
-    DEV_ERR_MBAR_TIMEOUT = 2u,      // bulk-copy mbarrier wait hit its limit
+    DEV_ERR_MBAR_TIMEOUT = 2u,      // mbarrier wait hit its limit
     DEV_ERR_KEY_RANGE = 4u,         // a key fell outside its cell table
     DEV_ERR_CAPACITY = 8u,          // a fixed-capacity list overflowed
     DEV_ERR_GRID_TIMEOUT = 16u      // a persistent kernel's grid-wide barrier wait hit its limit
