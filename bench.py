@@ -1,8 +1,8 @@
 #!/usr/bin/env python
 """SPH particle-steps/s of the 3D block collapse (1,048,576 particles) on one GB300.
 
-One "step" is one oclFluid3D::compute() of the whole scene: hash, one-sweep sort (+reorder),
-cell bounds, density, forces + integration. Default: N=1 GPU, 500 timed steps after 5
+One "step" is one oclFluid3D::compute() of the whole scene: cell keys, sort (+reorder), cell
+bounds, density, forces + integration. Default: N=1 GPU, 500 timed steps after 5
 warm-up steps, L2 flushed (512 MiB write) between timed steps, each step timed with CUDA
 events on the stream it runs on. Prints one JSON line.
 
@@ -39,11 +39,12 @@ L2_FLUSH_BYTES = 512 << 20
 # byte budget: each array counted once per stage; neighbour re-reads, neighbour lists and
 # cell-table reads not counted), mapped onto the fused step's launches:
 STAGE_BYTES_PER_PARTICLE = {
-    "front_end": 16 + 4 + 4,          # hash: R pos 16, W key 4, W index 4
-    "sort": (4 + 16 * 3) + 68,        # histogram R key + 3 x 8-bit passes (R/W key, index), and the
-                                      # reorder fused into the last pass: R index 4, R pos, vel 32,
-                                      # W sorted pos, vel 32
-    "bounds": 4,                      # R sorted key (+8 B per occupied cell, added below)
+    # the counting sort does the work of the budget's hash (R pos 16, W key 4, W index 4), sort
+    # (histogram R key + 3 x 8-bit passes, R/W key, index), reorder (R index 4, R pos, vel 32, W sorted
+    # pos, vel 32) and bounds (R sorted key, +8 B per occupied cell, added below) rows
+    "front_end": 0,
+    "sort": (16 + 4 + 4) + (4 + 16 * 3) + 68 + 4,
+    "bounds": 0,
     "density": 16 + 4,                # R sorted pos 16, W density/pressure 4
     "forces": 16 + 16 + 4 + 4 + 32,   # R sorted pos, vel, density/pressure, index; W pos, vel
 }
@@ -811,9 +812,8 @@ def main(argv=None) -> int:
         print(f"device status {status}: {fluid.last_error()}", file=sys.stderr)
         return 1
     value = scene.n * args.steps * world / (t_ms * 1e-3)
-    # linear grid: hash, 3 sort passes, bounds, density, forces; reference hash: the same with
-    # the exact density and forces, plus the fused clip-box / integration kernel
-    launches_per_step = 7 if args.keys == "linear" else 8
+    # count, tile sums, scan, scatter, order, density, forces (brick or exact kernels)
+    launches_per_step = 7
 
     result = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -821,7 +821,7 @@ def main(argv=None) -> int:
         "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded jittered lattice, block_collapse_3d seed 2)",
         "config": workload_config(world),
-        "keys": ("linear grid 200x100x200, 3 x 8-bit one-sweep passes" if args.keys == "linear" else
+        "keys": ("linear grid 200x100x200, counting sort by cell" if args.keys == "linear" else
                  "reference hash (262,144 buckets), exact kernels"),
         "graph": True,
         "gpu_launches": launches_per_step * args.steps,
@@ -847,7 +847,7 @@ def main(argv=None) -> int:
         peak, peak_kind = measured_peaks()
         stage_gbs = {}
         for k, ms in stage_ms.items():
-            b = STAGE_BYTES_PER_PARTICLE[k] * scene.n + (8 * n_cells_occ if k == "bounds" else 0)
+            b = STAGE_BYTES_PER_PARTICLE[k] * scene.n + (8 * n_cells_occ if k == "sort" else 0)
             stage_gbs[k] = b / (ms * 1e-3) / 1e9
         dom = max(stage_ms, key=stage_ms.get)
         dom_bytes = STAGE_BYTES_PER_PARTICLE[dom] * scene.n

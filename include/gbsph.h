@@ -207,7 +207,9 @@ enum {
                                   stage (the reference's CL_QUEUE_PROFILING_ENABLE events,
                                   libCL/oclDevice.cpp:31, libCL/oclKernel.cpp:162-202) */
     GBSPH_OPT_RADIX_BITS = 4,  /* batches: key bits sorted per radix pass (5..8, default 8; at
-                                  most four passes over the batch's key width) */
+                                  most four passes over the batch's key width). Like the tile,
+                                  for steps that sort by radix passes: the persistent form, and
+                                  batches with too many cells for the counting sort */
     GBSPH_OPT_SORT_TILE = 5,   /* batches: keys per thread of a sort tile (8 or 16; 0, the
                                   default: 8 up to 2^21 keys, else 16) */
     GBSPH_OPT_PERSISTENT = 6   /* batches: 1 = the whole step (hash, sort passes, cell bounds,
