@@ -433,6 +433,9 @@ int st_bounds(H* h, const KParams& kp, cudaStream_t s, bool full_clear) {
 // with 2 / 4 / 8 / 16: 4,096 particles 9.6 / 11.6 / 13.8 / 19.9, 16,384 17.8 / 13.7 / 13.8 / 19.9,
 // 32,768 26.0 / 19.8 / 17.9 / 21.2, 65,536 46.5 / 30.4 / 28.1 / 26.0, 1,048,576: 8 463, 16 377, 32 426.
 constexpr uint32_t EXACT_FEW = 8192, EXACT_SOME = 49152;
+// Up to this the force kernel that computes the terms of a warp's lists side by side (18.4 us at 32,768
+// particles, 20.5 a thread per particle; 28.7 / 24.6 at 65,536).
+constexpr uint32_t EXACT_LISTED = 32768;
 
 // Exact (reference-order) density and forces. With lists (the fused REFERENCE_HASH step, where
 // the two run back to back on the same sorted state) the density kernel records each
@@ -467,7 +470,15 @@ int st_forces_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false,
         kern<<<grid1(kp.n), 256, 0, s>>>(h->spos, h->svel, P4(h, 2), h->index, table, kp, xl, xc, P4(h, 0), P4(h, 1));
     };
     constexpr int LIN = GBSPH_KEY_LINEAR_GRID, HASH = GBSPH_KEY_REFERENCE_HASH;
-    if (kp.key_mode == LIN) launch(k_forces_exact<LIN, false, false>, h->table);
+    if (lists && kp.key_mode == HASH && kp.n <= EXACT_LISTED) {
+        auto listed = [&](auto kern) {
+            const uint32_t per = LISTED_TARGETS * LISTED_WARPS;
+            kern<<<(kp.n + per - 1) / per, 32 * LISTED_WARPS, 0, s>>>(h->spos, h->svel, P4(h, 2), h->index, h->hash_table, kp, xl, xc, P4(h, 0),
+                                                                      P4(h, 1));
+        };
+        if (post) listed(k_forces_listed<HASH, true>);
+        else listed(k_forces_listed<HASH, false>);
+    } else if (kp.key_mode == LIN) launch(k_forces_exact<LIN, false, false>, h->table);
     else if (lists && post) launch(k_forces_exact<HASH, true, true>, h->hash_table);
     else if (lists) launch(k_forces_exact<HASH, true, false>, h->hash_table);
     else launch(k_forces_exact<HASH, false, false>, h->hash_table);

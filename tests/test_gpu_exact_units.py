@@ -34,7 +34,7 @@ def positions(kind, n, h, rng):
 
 @pytest.mark.parametrize("dims", [3, 2])
 @pytest.mark.parametrize("kind", ["sparse", "one cell", "wide cell", "mixed"])
-@pytest.mark.parametrize("n", [3, 31, 33, 129, 700, 8193, 49153])
+@pytest.mark.parametrize("n", [3, 31, 33, 129, 700, 8193, 32769, 49153])
 def test_reference_order_kernels(cuda, kind, n, dims):
     if n > 1000 and kind in ("one cell", "wide cell"):
         pytest.skip("all pairs of one cell")
@@ -58,3 +58,24 @@ def test_reference_order_kernels(cuda, kind, n, dims):
             assert np.array_equal(out[name].view(np.uint32), want.view(np.uint32)), name
         for name, want in (("pos", pos), ("vel", v), ("force", force)):
             assert np.array_equal(st[name].view(np.uint32), want.view(np.uint32)), name
+
+
+@pytest.mark.parametrize("n", [31, 5000, 40000])
+def test_forces_left_to_a_hook(cuda, n):
+    """With an integrate hook the fused step leaves the force before clipping: as the staged step's."""
+    sc = hash_block(4)
+    rng = np.random.default_rng(n)
+    sc.pos = positions("mixed", n, float(sc.params.cellSize), rng)
+    vel = np.zeros((n, 4), np.float32)
+    vel[:, :3] = rng.uniform(-1, 1, (n, 3))
+    sc.vel = vel
+    force = rng.uniform(-1, 1, (n, 4)).astype(np.float32)
+    out = []
+    for fused in (True, False):
+        f = make_fluid(sc, fused=fused, vel=vel, force=force)
+        f.addEventHandler(lambda fluid, stream: 0)
+        f.compute()
+        out.append(state(f))
+    for name in ("pos", "vel", "force"):
+        assert np.array_equal(out[0][name].view(np.uint32), out[1][name].view(np.uint32)), name
+    assert not np.array_equal(out[0]["force"], force)
