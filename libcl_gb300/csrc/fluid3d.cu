@@ -431,7 +431,8 @@ int st_bounds(H* h, const KParams& kp, cudaStream_t s, bool full_clear) {
 // Targets per warp of the exact density kernel. Few targets leave each warp a short chain and
 // spread a small scene over the chip; many share the search for their cells' candidates. Us
 // with 2 / 4 / 8 / 16: 4,096 particles 9.6 / 11.6 / 13.8 / 19.9, 16,384 17.8 / 13.7 / 13.8 / 19.9,
-// 32,768 26.0 / 19.8 / 17.9 / 21.2, 65,536 46.5 / 30.4 / 28.1 / 26.0, 1,048,576: 8 463, 16 377, 32 426.
+// 32,768 26.0 / 19.8 / 17.9 / 21.2, 65,536 46.5 / 30.4 / 28.1 / 26.0, 1,048,576: 8 463, 16 377, 32 426
+// (all before full lists were added up on the way, which costs 4 %).
 constexpr uint32_t EXACT_FEW = 8192, EXACT_SOME = 49152;
 // Up to this the force kernel that computes the terms of a warp's lists side by side (18.4 us at 32,768
 // particles, 20.5 a thread per particle; 28.7 / 24.6 at 65,536).

@@ -368,13 +368,15 @@ struct ExactWarp {
 //    fl(target - candidate) is at least the rounded distance to the box in magnitude
 //    (rounding is monotone), and exact_r2 grows with each: none that is left out is in range;
 //  - for each target tests the held candidates, two to a lane, and appends r2 of those in
-//    range to the target's list.
-// Then a thread sums its target's list. A thread that scans its 27 buckets by itself (12 of
+//    range to the target's list, whose terms are added up as often as it is full.
+// Then the rest of each list is summed. A thread that scans its 27 buckets by itself (12 of
 // the 32 lanes at work, and the root and the sum executed for nearly every candidate because
 // some lane is in range) took 522 us for 1,048,576 particles, 324 candidates and 34 in range
-// each, and 23.6 us for 256, all of it the chain of table reads; this takes 377 and 7.7 us.
-// Bound by instruction issue (76% of cycles). Tried: 64 and 192 candidates held (388 / 391), 32
-// targets per warp (426), the two candidates of a lane next to each other (397).
+// each, and 23.6 us for 256, all of it the chain of table reads; this takes 393 and 7.7 us.
+// Bound by instruction issue (76% of cycles). A list that is summed only
+// at the end and, beyond XL_CAP, from the buckets again: 377, but 2.6 ms instead of 0.9 at 0.7 x the
+// spacing (100 in range). Tried with that: 64 and 192 candidates held (+3 %), 32 targets per
+// warp (+13 %), the two candidates of a lane next to each other (+5 %).
 template <int MODE, bool RECORD, int T>
 __global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __restrict__ spos, float4* __restrict__ svel,
                                                                     const uint2* __restrict__ tab, KParams kp,
@@ -391,7 +393,22 @@ __global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __re
     int gx, gy, gz;
     neighbour_centre<MODE>(kp, posI, gx, gy, gz);
     const int l = (int)lane, ox = l % 3 - 1, oy = l / 3 % 3 - 1, oz = kp.dims == 2 ? 0 : l / 9 - 1;  // place in the visiting order
-    uint32_t count = 0;
+    float density = 0.0f;              // lane t: the sum of target t's first `summed` terms,
+    uint32_t count = 0, summed = 0;    // of `count` so far; the others' r2 are in its list
+    auto term = [&](float r2) {
+        const float vlen = __fsqrt_rn(r2);
+        const float u = __fsub_rn(__fmul_rn(kp.h, kp.h), __fmul_rn(vlen, vlen));
+        return __fmul_rn(__fmul_rn(u, u), u);
+    };
+    // d plus the terms of the n entries of target t's list, in order (by the whole warp)
+    auto add_list = [&](int t, uint32_t n, float d) {
+        float* list = S.list + t;
+        for (uint32_t k = lane; k < n; k += 32) list[k * (T + 1)] = term(list[k * (T + 1)]);
+        __syncwarp();
+#pragma unroll 4
+        for (uint32_t k = 0; k < n; ++k) d = __fadd_rn(d, list[k * (T + 1)]);
+        return d;
+    };
     while (left) {
         const int lead = __ffs(left) - 1;
         const int cx = __shfl_sync(FULL, gx, lead), cy = __shfl_sync(FULL, gy, lead), cz = __shfl_sync(FULL, gz, lead);
@@ -452,7 +469,7 @@ __global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __re
                 const float x = __shfl_sync(FULL, posI.x, t), y = __shfl_sync(FULL, posI.y, t), z = __shfl_sync(FULL, posI.z, t);
                 const uint64_t x2 = f2_pack(x, x), y2 = f2_pack(y, y), z2 = f2_pack(z, z);
                 const uint32_t self = first + (uint32_t)t;
-                uint32_t c = __shfl_sync(FULL, count, t);
+                uint32_t c = __shfl_sync(FULL, count, t), base = __shfl_sync(FULL, summed, t);
                 float* list = S.list + t;
                 uint32_t* rec = RECORD ? xl + (size_t)self * XL_CAP : nullptr;
                 for (uint32_t p = 0; p < np; ++p) {
@@ -468,20 +485,29 @@ __global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __re
                     const uint32_t j0 = __float_as_uint(b.z), j1 = __float_as_uint(b.w);
                     const bool in0 = r0 < kp.r2_thresh && j0 != self, in1 = r1 < kp.r2_thresh && j1 != self;  // fast_length < h
                     const uint32_t m0 = __ballot_sync(FULL, in0), m1 = __ballot_sync(FULL, in1);
-                    const uint32_t k0 = c + (uint32_t)__popc(m0 & lt);
-                    c += (uint32_t)__popc(m0);
-                    const uint32_t k1 = c + (uint32_t)__popc(m1 & lt);
-                    c += (uint32_t)__popc(m1);
-                    if (in0 && k0 < XL_CAP) {
-                        list[k0 * (T + 1)] = r0;
-                        if (RECORD) rec[k0] = j0;
+                    const uint32_t k0 = c + (uint32_t)__popc(m0 & lt), n0 = c + (uint32_t)__popc(m0);
+                    const uint32_t k1 = n0 + (uint32_t)__popc(m1 & lt), n1 = n0 + (uint32_t)__popc(m1);
+                    if (n1 - base > XL_CAP) {  // the list is full: its terms are added up now
+                        __syncwarp();
+                        const float d = add_list(t, c - base, __shfl_sync(FULL, density, t));
+                        if (l == t) density = d;
+                        __syncwarp();
+                        base = c;
                     }
-                    if (in1 && k1 < XL_CAP) {
-                        list[k1 * (T + 1)] = r1;
-                        if (RECORD) rec[k1] = j1;
+                    c = n1;
+                    if (in0) {
+                        list[(k0 - base) * (T + 1)] = r0;
+                        if (RECORD && k0 < XL_CAP) rec[k0] = j0;
+                    }
+                    if (in1) {
+                        list[(k1 - base) * (T + 1)] = r1;
+                        if (RECORD && k1 < XL_CAP) rec[k1] = j1;
                     }
                 }
-                if (l == t) count = c;
+                if (l == t) {
+                    count = c;
+                    summed = base;
+                }
             }
             __syncwarp();
             held = 0;
@@ -512,17 +538,11 @@ __global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __re
     }
     __syncwarp();
     // 32 / T lanes share a target: each computes every (32 / T)-th term, all add them in order
-    auto term = [&](float r2) {
-        const float vlen = __fsqrt_rn(r2);
-        const float t = __fsub_rn(__fmul_rn(kp.h, kp.h), __fmul_rn(vlen, vlen));
-        return __fmul_rn(__fmul_rn(t, t), t);
-    };
-    float density = 0.0f;
     {
         constexpr uint32_t SHARE = 32 / T;
         const int t = l / (int)SHARE, first_lane = l - l % (int)SHARE;
-        const uint32_t mine = __shfl_sync(FULL, count, t), most = warp_max(mine <= XL_CAP ? mine : 0u);
-        float d = 0.0f;
+        const uint32_t mine = __shfl_sync(FULL, count - summed, t), most = warp_max(mine);
+        float d = __shfl_sync(FULL, density, t);
         for (uint32_t k = 0; k < most; k += SHARE) {
             const uint32_t at = k + lane % SHARE;
             const float v = at < mine ? term(S.list[at * (T + 1) + (uint32_t)t]) : 0.0f;
@@ -535,17 +555,6 @@ __global__ void __launch_bounds__(32 * EXACT_WARPS) k_density_exact(float4* __re
         density = __shfl_sync(FULL, d, (l * (int)SHARE) & 31);
     }
     if (!live) return;
-    if (count > XL_CAP) {  // more than the list holds: through the buckets again
-        density = 0.0f;
-        for_each_neighbour_cell<MODE>(kp, tab, posI, [&](uint32_t start, uint32_t end) {
-            for (uint32_t j = start; j < end; j++) {
-                if (j == particle) continue;
-                const float4 pj = spos[j];
-                const float r2 = exact_r2(__fsub_rn(posI.x, pj.x), __fsub_rn(posI.y, pj.y), __fsub_rn(posI.z, pj.z));
-                if (r2 < kp.r2_thresh) density = __fadd_rn(density, term(r2));
-            }
-        });
-    }
     if (RECORD) xc[particle] = count;
     // The reference writes .w in place while other work-items read .xyz only. Here the
     // candidates' positions are loaded as whole float4s, so a load may race with another
