@@ -265,7 +265,7 @@ int enqueue_batch(B* h, const KParams& kp, cudaStream_t s) {
         GBSPH_CUDA_TRY(&h->last_error, count_sort<true>(c, kp, s));
         h->count_clean = true;
     } else {
-        GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, kp.n, sort_passes(0, kp.end_bit, kp.digit_bits), s));
+        GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, kp.n, sort_passes(0, kp.end_bit, kp.digit_bits), s, h->sort_items));
         const int blocks = std::max(1, std::min((int)((kp.n + 255) / 256), num_sms() * 8));
         if (clear)
             k_hash_batch<true><<<blocks, 256, 0, s>>>(h->pos, kp, h->keys_a, (uint32_t*)h->scratch, h->keys_c, h->table);
@@ -314,7 +314,7 @@ int enqueue_persistent(B* h, const KParams& kp, cudaStream_t s) {
     const bool clear = h->table_clean;
     if (!clear) GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->table, 0xFF, h->cells * sizeof(uint2), s));
     h->table_clean = false;
-    GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, kp.n, sort_passes(0, kp.end_bit, kp.digit_bits), s));
+    GBSPH_CUDA_TRY(&h->last_error, onesweep_prepare(h->scratch, kp.n, sort_passes(0, kp.end_bit, kp.digit_bits), s, sort_items_of(h)));
     BatchStepArgs a;
     a.pos = h->pos;
     a.vel = h->vel;

@@ -200,15 +200,22 @@ size_t onesweep_scratch_bytes(uint32_t n, int passes) {
     return SORT_HEADER_BYTES + (size_t)std::max(passes, 1) * sort_tiles(std::max(n, 1u)) * SORT_RADIX * 4;
 }
 
-cudaError_t onesweep_prepare(void* scratch, uint32_t n, int passes, cudaStream_t s) {
-    return cudaMemsetAsync(scratch, 0, onesweep_scratch_bytes(n, passes), s);
+// Bytes of the look-back words that passes of `items` keys per thread (0: the default) use: a
+// quarter of what the scratch has room for where its tiles are the largest, so that a sort of
+// 16,777,216 keys clears 17 MB before it starts, not 67.
+static size_t lookback_bytes(uint32_t n, int passes, int items) {
+    const int used = items ? items : sort_items_for(n);
+    return (size_t)std::max(passes, 1) * sort_tiles(std::max(n, 1u), SORT_THREADS * used) * SORT_RADIX * 4;
 }
 
-cudaError_t onesweep_reset_progress(void* scratch, uint32_t n, int passes, cudaStream_t s) {
+cudaError_t onesweep_prepare(void* scratch, uint32_t n, int passes, cudaStream_t s, int items) {
+    return cudaMemsetAsync(scratch, 0, SORT_HEADER_BYTES + lookback_bytes(n, passes, items), s);
+}
+
+cudaError_t onesweep_reset_progress(void* scratch, uint32_t n, int passes, cudaStream_t s, int items) {
     cudaError_t e = cudaMemsetAsync((char*)scratch + 4096, 0, 16, s);
     if (e != cudaSuccess) return e;
-    return cudaMemsetAsync((char*)scratch + SORT_HEADER_BYTES, 0,
-                           onesweep_scratch_bytes(n, passes) - SORT_HEADER_BYTES, s);
+    return cudaMemsetAsync((char*)scratch + SORT_HEADER_BYTES, 0, lookback_bytes(n, passes, items), s);
 }
 
 cudaError_t onesweep_histogram(const uint32_t* keys, uint32_t n, int start_bit, int end_bit,
