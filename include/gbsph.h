@@ -211,7 +211,7 @@ enum {
                                   for steps that sort by radix passes: the persistent form, and
                                   batches with too many cells for the counting sort */
     GBSPH_OPT_SORT_TILE = 5,   /* batches: keys per thread of a sort tile (8 or 16; 0, the
-                                  default: 8 up to 2^21 keys, else 16) */
+                                  default: 8 up to 786,432 keys, else 16) */
     GBSPH_OPT_PERSISTENT = 6   /* batches: 1 = the whole step (hash, sort passes, cell bounds,
                                   density, forces and integration) as one cooperative kernel
                                   whose CTAs stay resident and meet at grid-wide barriers;

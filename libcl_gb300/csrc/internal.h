@@ -63,8 +63,10 @@ __host__ __device__ inline int sort_passes(int start_bit, int end_bit, int digit
 }
 __host__ __device__ inline uint32_t sort_tiles(uint32_t n, uint32_t tile = SORT_MIN_TILE) { return (n + tile - 1) / tile; }
 // Keys per thread of a pass over n keys: small sorts use small tiles (more tiles in flight,
-// shorter per-tile latency), large ones the largest tile (fewer look-back steps).
-inline int sort_items_for(uint32_t n) { return n <= (1u << 21) ? 8 : 16; }
+// shorter per-tile latency), large ones the largest tile (fewer look-back steps). Us of a 24-bit
+// sort with 8 / 16: 150,000 keys 49.6 / 55.7, 600,000 62.7 / 62.1, 1,050,000 75.6 / 74.0,
+// 1,500,000 89.5 / 87.0, 2,000,000 97.2 / 96.6 (32 bits: 111.9 / 107.9 at 1,500,000).
+inline int sort_items_for(uint32_t n) { return n <= 3u << 18 ? 8 : 16; }
 size_t onesweep_scratch_bytes(uint32_t n, int passes);
 
 // Optional gather fused into the last pass: dst[k][dest] = src[k][value] for k < n_gather.
