@@ -143,6 +143,25 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return true;
 }
 
+// A wait for threads that may be at work for long: the limit begins again whenever `progress`, a word
+// of shared memory that they count on, has changed.
+__device__ __forceinline__ bool mbar_wait_progress(uint64_t* bar, uint32_t parity, const volatile uint32_t* progress) {
+    uint32_t polls = 0, seen = 0;
+    uint64_t start = 0;
+    while (!mbar_try_wait(bar, parity)) {
+        if ((++polls & 31u) != 0u) continue;
+        const uint64_t now = globaltimer_ns();
+        const uint32_t p = *progress;
+        if (start == 0 || p != seen) {
+            start = now;
+            seen = p;
+        } else if (now - start > WAIT_LIMIT_NS) {
+            return false;
+        }
+    }
+    return true;
+}
+
 // Least and greatest value over the warp's 32 lanes (NaNs are left out while another lane has a number).
 __device__ __forceinline__ float warp_min(float v) {
     float r;

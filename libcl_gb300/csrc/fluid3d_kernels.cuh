@@ -893,6 +893,11 @@ static __global__ void k_emitter(float4* __restrict__ pos, float4* __restrict__ 
 // two passes need not cut the bricks alike. Staged by rows, the window is nine short pieces,
 // and the row loop around them cost as many instructions as the candidates themselves.
 //
+// A consumer waits for copies and for a task at most; the producer waits for whole units, and a unit
+// that is not staged may take long (8,000 particles in one cell: 64 ms for both passes; 60,000:
+// seconds). So consumers count the cells that they read from global memory in S.progress, and
+// the producer gives up only after a second in which nothing moved.
+//
 // A cell's particles are taken in pairs (two consecutive sorted particles; the last of an odd
 // cell alone), numbered through the unit, and both passes give four lanes to a pair and eight
 // pairs to a warp whatever cells they are in. A lane holds both targets, so a candidate read
@@ -936,6 +941,7 @@ struct BrickUnit {
 
 struct BrickShared {
     BrickUnit unit[2];
+    uint32_t progress;              // cells that consumers have begun to read from global memory
     unsigned long long full[2], empty[2];
 };
 
@@ -980,6 +986,7 @@ __device__ __forceinline__ void brick_init(BrickShared& S) {
             mbar_init(reinterpret_cast<uint64_t*>(&S.full[i]), 64);
             mbar_init(reinterpret_cast<uint64_t*>(&S.empty[i]), blockDim.x / 32u - 1u);
         }
+        S.progress = 0u;
         fence_mbar_init();
     }
     __syncthreads();
@@ -1010,7 +1017,7 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
     // Waits until the buffer of the next unit is free.
     auto acquire = [&]() -> bool {
         if (fill < 2) return true;
-        const bool ok = mbar_wait_bounded(reinterpret_cast<uint64_t*>(&S.empty[fill & 1u]), ((fill >> 1) - 1u) & 1u);
+        const bool ok = mbar_wait_progress(reinterpret_cast<uint64_t*>(&S.empty[fill & 1u]), ((fill >> 1) - 1u) & 1u, &S.progress);
         if (!ok) atomicOr(err, DEV_ERR_MBAR_TIMEOUT);
         return __all_sync(0xffffffffu, ok);
     };
@@ -1151,7 +1158,10 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
         b = nb;
         bid = nbid;
     }
-    if (!acquire()) return false;
+    if (!acquire()) {
+        cp_async_wait_all();
+        return false;
+    }
     if (lane == 0) S.unit[fill & 1u].ncell = 0;
     __syncwarp();
     hand_over();
@@ -1317,6 +1327,7 @@ __device__ __forceinline__ bool density_brick_run(float4* s_buf, BrickShared& S,
                 }
             } else {  // unstaged unit: candidates from global memory, no lists
                 for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
+                    if (lane == 0u) atomicAdd(&S.progress, 1u);
                     const uint32_t n = U.off[i + 1] - U.off[i], first = U.cell[i].x;
                     for (uint32_t k = q; k < n; k += 4u) {
                         mA = mB = 0u;
@@ -1546,6 +1557,7 @@ __device__ __forceinline__ bool force_brick_run(float4* s_buf, BrickShared& S, c
                 }
             } else {
                 for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
+                    if (lane == 0u) atomicAdd(&S.progress, 1u);
                     const uint32_t cnt = U.off[i + 1] - U.off[i], first = U.cell[i].x;
                     for (uint32_t j = l; j < cnt; j += 4u) both(ld_phase<COH>(spos + first + j), ld_phase<COH>(svel + first + j));
                 }
