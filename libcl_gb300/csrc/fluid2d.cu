@@ -223,7 +223,7 @@ __device__ __forceinline__ void for_candidates2(const K2& k, int cx, int cy, con
         };
         if (x >= 0 && x < k.ncx && y >= 0 && y < k.ncy && !far(x, k.ncx, xl, xh) && !far(y, k.ncy, yl, yh)) {
             const uint2 e = table[y * k.ncx + x];
-            if (e.x != EMPTY2) {
+            if (e.x <= e.y && e.y <= k.n) {  // not empty, and never out of range
                 first = e.x;
                 n = e.y - e.x;
             }
@@ -705,9 +705,12 @@ int alloc_table2(H2* h) {
     h->count = nullptr;
     const size_t words = count_words(t);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->cells, words * 12));
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->cells, 0xFF, words * 8));
     h->count = (uint32_t*)(h->cells + words);
-    h->count_clean = false;
+    // complete before any step, on whatever stream; steps that only a captured graph holds find zeros too
+    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->cells, 0xFF, words * 8, h->cap_stream));
+    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, words * 4, h->cap_stream));
+    GBSPH_CUDA_TRY(&h->last_error, cudaStreamSynchronize(h->cap_stream));
+    h->count_clean = true;
     h->table = t;
     invalidate2(h);
     return GBSPH_OK;
@@ -985,6 +988,7 @@ GBSPH_API int gbsph_fluid2d_sync_status(gbsph_fluid2d_t h, void* stream) {
     GBSPH_CUDA_TRY(&h->last_error, cudaMemcpy(&bits, h->err, 4, cudaMemcpyDeviceToHost));
     if (bits) {
         GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->err, 0, 4));
+        h->count_clean = false;  // a step that refused a particle leaves its cell's count
         return fail(&h->last_error, dev_err_to_status(bits), "device error word 0x" + std::to_string(bits));
     }
     return GBSPH_OK;
