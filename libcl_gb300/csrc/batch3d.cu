@@ -519,9 +519,7 @@ GBSPH_API int gbsph_batch3d_set_scenes(gbsph_batch3d_t h, const gbsph_fluid3d_pa
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->sdev, n_scenes * sizeof(SceneDev)));
     if (count_sort_fits((uint32_t)cells, (uint32_t)n)) {
         GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->count, count_words((uint32_t)cells) * 4));
-        // complete before any step, on whatever stream
-        GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, count_words((uint32_t)cells) * 4, h->cap_stream));
-        GBSPH_CUDA_TRY(&h->last_error, cudaStreamSynchronize(h->cap_stream));
+        GBSPH_CUDA_TRY(&h->last_error, fill_now(h->count, 0, count_words((uint32_t)cells) * 4));
     }
     h->count_clean = true;
     h->sdev_bw = -1;

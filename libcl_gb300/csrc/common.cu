@@ -39,6 +39,21 @@ int num_sms() {
     return sms > 0 ? sms : 148;
 }
 
+cudaError_t fill_now(void* p, int byte, size_t bytes) {
+    cudaStreamCaptureStatus capture;
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e == cudaErrorStreamCaptureImplicit) {
+        cudaGetLastError();
+        e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    }
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(p, byte, bytes, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (s) cudaStreamDestroy(s);
+    return e;
+}
+
 namespace {
 
 float bits_to_float(uint32_t b) {

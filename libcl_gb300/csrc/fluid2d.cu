@@ -706,10 +706,8 @@ int alloc_table2(H2* h) {
     const size_t words = count_words(t);
     GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->cells, words * 12));
     h->count = (uint32_t*)(h->cells + words);
-    // complete before any step, on whatever stream; steps that only a captured graph holds find zeros too
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->cells, 0xFF, words * 8, h->cap_stream));
-    GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, words * 4, h->cap_stream));
-    GBSPH_CUDA_TRY(&h->last_error, cudaStreamSynchronize(h->cap_stream));
+    GBSPH_CUDA_TRY(&h->last_error, fill_now(h->cells, 0xFF, words * 8));
+    GBSPH_CUDA_TRY(&h->last_error, fill_now(h->count, 0, words * 4));
     h->count_clean = true;
     h->table = t;
     invalidate2(h);

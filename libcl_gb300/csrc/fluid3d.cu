@@ -314,9 +314,7 @@ int ensure_tables(H* h) {
         h->count = nullptr;
         h->count_words = 0;
         GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->count, count_words((uint32_t)cells) * 4));
-        // complete before any step, on whatever stream
-        GBSPH_CUDA_TRY(&h->last_error, cudaMemsetAsync(h->count, 0, count_words((uint32_t)cells) * 4, h->cap_stream));
-        GBSPH_CUDA_TRY(&h->last_error, cudaStreamSynchronize(h->cap_stream));
+        GBSPH_CUDA_TRY(&h->last_error, fill_now(h->count, 0, count_words((uint32_t)cells) * 4));
         h->count_words = count_words((uint32_t)cells);
         h->count_clean = true;
         invalidate_graph(h);

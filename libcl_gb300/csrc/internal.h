@@ -112,6 +112,11 @@ cudaError_t cell_bounds_launch(const uint32_t* sorted_keys, uint32_t n, uint32_t
 
 int num_sms();
 
+// Fills freshly allocated device memory, complete on return, so that a step may follow on whatever
+// stream. On the legacy stream (once another has had work, the steps of small scenes were 3 %
+// slower), except while a blocking stream is capturing, when that one may not be used.
+cudaError_t fill_now(void* p, int byte, size_t bytes);
+
 // Smallest float x >= 0 with sqrtf(x) >= h (common.cu). sqrtf is correctly rounded and monotone, so
 // for every float r2 >= 0: (sqrtf(r2) < h) == (r2 < r2_threshold(h)).
 float r2_threshold(float h);
