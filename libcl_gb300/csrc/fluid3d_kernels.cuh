@@ -1458,6 +1458,112 @@ __device__ __forceinline__ float integrate_force_lane(const KParams& kp, float v
     return __fadd_rn(v, __fmul_rn(f, kp.dt));
 }
 
+// The lane's part of a pair's state: component l of the two particles' force, velocity and position.
+struct PairState {
+    uint32_t oA, oB;  // the particles
+    float fA, fB, vA, vB, pA, pB;
+};
+
+template <bool FUSED, bool COH>
+__device__ __forceinline__ PairState pair_state(const PairTask& t, uint32_t l, const uint32_t* __restrict__ index,
+                                                const float4* pos, const float4* vel, const float4* force) {
+    PairState s{};
+    s.oA = ld_phase<COH>(index + t.gi);
+    s.oB = ld_phase<COH>(index + t.gi + (t.two ? 1u : 0u));
+    s.fA = reinterpret_cast<const float*>(force + s.oA)[l];
+    s.fB = reinterpret_cast<const float*>(force + s.oB)[l];
+    if (FUSED) {
+        s.vA = reinterpret_cast<const float*>(vel + s.oA)[l];
+        s.vB = reinterpret_cast<const float*>(vel + s.oB)[l];
+        s.pA = reinterpret_cast<const float*>(pos + s.oA)[l];
+        s.pB = reinterpret_cast<const float*>(pos + s.oB)[l];
+    }
+    return s;
+}
+
+// Pressure and viscosity terms together, then the sums over the pair's lanes.
+__device__ __forceinline__ void pair_sums(const KParams& kp, float cvisc, const float* accA, const float* accB, float (*f)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        f[0][k] = fmaf(kp.cpress, accA[k], cvisc * accA[3 + k]);
+        f[1][k] = fmaf(kp.cpress, accB[k], cvisc * accB[3 + k]);
+#pragma unroll
+        for (uint32_t m = 1; m < 4u; m <<= 1) {
+            f[0][k] += __shfl_xor_sync(0xffffffffu, f[0][k], m);
+            f[1][k] += __shfl_xor_sync(0xffffffffu, f[1][k], m);
+        }
+    }
+}
+
+// Lane l takes component l of the pair's new state, target A and then target B.
+template <int DIMS, bool FUSED>
+__device__ __forceinline__ void pair_finish(const KParams& kp, const BrickUnit& U, const PairTask& t, uint32_t l, const PairState& s,
+                                            const float (*f)[3], const float4& pA, const float4& pB, const float4& vA,
+                                            const float4& vB, float4* __restrict__ pos, float4* __restrict__ vel,
+                                            float4* __restrict__ force) {
+    const float g = l == 0u ? kp.gravity.x : (l == 1u ? kp.gravity.y : (l == 2u ? kp.gravity.z : kp.gravity.w));
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const bool live = t.live && (w == 0 || t.two);
+        const uint32_t o = w ? s.oB : s.oA;
+        const float add = l == 0u ? f[w][0] : (l == 1u ? f[w][1] : f[w][2]);
+        float F = l == 3u ? 0.0f : __fadd_rn(w ? s.fB : s.fA, __fmul_rn(add, kp.mass));
+        if (FUSED) {
+            F = clip_box_lane<DIMS>(kp, U.box_min, U.box_max, w ? pB : pA, w ? vB : vA, F, l, live);
+            if (kp.rec_force && live) reinterpret_cast<float*>(kp.rec_force + o)[l] = F;
+            const float v = integrate_force_lane(kp, w ? s.vB : s.vA, F);
+            if (live) {
+                reinterpret_cast<float*>(vel + o)[l] = v;
+                reinterpret_cast<float*>(force + o)[l] = g;
+                reinterpret_cast<float*>(pos + o)[l] = __fadd_rn(w ? s.pB : s.pA, __fmul_rn(v, kp.dt));
+            }
+        } else if (live) {
+            reinterpret_cast<float*>(force + o)[l] = F;
+        }
+    }
+}
+
+// A warp's task in a unit that is not staged: a pair's lanes take every fourth candidate of the cells in
+// global memory, with correctly rounded reciprocals of the densities (the staged tasks use the
+// hardware's, which differ by one unit in the last place for one density in eight). Out of line and with few
+// arguments, so that the staged tasks keep their registers and spill nothing: 1,048,576 particles
+// 152 us, 149 without this code, 159 with it in line; 48 scenes a step 787, 802 and 822. `what`: the target's
+// column, 8: two targets, 16: live.
+template <int DIMS, bool FUSED, bool COH>
+__device__ __noinline__ void force_unstaged(BrickShared& S, uint32_t use, uint32_t gi, uint32_t what, const float4* __restrict__ spos,
+                                            const float4* __restrict__ svel, const uint32_t* __restrict__ index,
+                                            float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ force,
+                                            const KParams& kp) {
+    constexpr int R = DIMS == 3 ? 9 : 3;
+    const BrickUnit& U = S.unit[use & 1u];
+    PairTask t{};
+    t.gi = gi;
+    t.c = (int)(what & 7u);
+    t.two = (what & 8u) != 0u;
+    t.live = (what & 16u) != 0u;
+    const uint32_t lane = threadIdx.x & 31u, l = lane & 3u, two = t.two ? 1u : 0u;
+    const uint32_t thr = max(__float_as_uint(kp.r2_thresh), MIN_NORMAL) - MIN_NORMAL;
+    const PairState st = pair_state<FUSED, COH>(t, l, index, pos, vel, force);
+    const float4 pA = ld_phase<COH>(spos + t.gi), pB = ld_phase<COH>(spos + t.gi + two);
+    const float4 vA = ld_phase<COH>(svel + t.gi), vB = ld_phase<COH>(svel + t.gi + two);
+    const float aA = __frcp_rn(pA.w), aB = __frcp_rn(pB.w);
+    float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
+        if (lane == 0u) atomicAdd(&S.progress, 1u);
+        const uint32_t cnt = U.off[i + 1] - U.off[i], first = U.cell[i].x;
+        for (uint32_t j = l; j < cnt; j += 4u) {
+            const float4 pj = ld_phase<COH>(spos + first + j), vj = ld_phase<COH>(svel + first + j);
+            const float aj = __frcp_rn(pj.w);
+            force_pair<DIMS>(pA, vA, aA, pj, vj, aj, kp.h, thr, accA);
+            force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
+        }
+    }
+    __syncwarp();
+    float f[2][3];
+    pair_sums(kp, U.cvisc, accA, accB, f);
+    pair_finish<DIMS, FUSED>(kp, U, t, l, st, f, pA, pB, vA, vB, pos, vel, force);
+}
+
 // Forces (pressure + viscosity) for every particle of the occupied bricks
 // (clCalculateForces, libCL/phys/oclFluid3D.cl:202-255). A pair's lane l evaluates entries 2 l and
 // 2 l + 1 of each 8-entry chunk of the pair's list for both targets; the lists' first LIST_AHEAD
@@ -1501,36 +1607,21 @@ __device__ __forceinline__ bool force_brick_run(float4* s_buf, BrickShared& S, c
         const int tasks = (int)((U.npair + TASK_PAIRS - 1u) / TASK_PAIRS);
         for (; turn < tasks; turn += consumers) {
             const PairTask t = pair_task<R, RC>(U, (uint32_t)turn * TASK_PAIRS + (lane >> 2));
+            if (!staged) {
+                force_unstaged<DIMS, FUSED, COH>(S, use, t.gi, (uint32_t)t.c | (t.two ? 8u : 0u) | (t.live ? 16u : 0u), spos, svel,
+                                                 index, pos, vel, force, kp);
+                continue;
+            }
             const uint32_t two = t.two ? 1u : 0u;
             // everything from global memory at once: the list's length and first chunks (whatever
-            // its length), the targets' particles and, with those known, the lane's component of
-            // their force, velocity and position
+            // its length), the targets' particles and, with those known, the lane's part of their state
             const uint32_t meta = ld_phase<COH>(nbr_meta + t.gi);
-            const uint32_t oA = ld_phase<COH>(index + t.gi), oB = ld_phase<COH>(index + t.gi + two);
+            const PairState st = pair_state<FUSED, COH>(t, l, index, pos, vel, force);
             const uint32_t* list = reinterpret_cast<const uint32_t*>(nbr) + (size_t)t.gi * (NBR_CAP / 2) + l;
             uint32_t ch[LIST_AHEAD];
 #pragma unroll
             for (uint32_t k = 0; k < LIST_AHEAD; ++k) ch[k] = ld_phase<COH>(list + 4u * k);
-            const float f_A = reinterpret_cast<const float*>(force + oA)[l], f_B = reinterpret_cast<const float*>(force + oB)[l];
-            float v_A = 0.f, v_B = 0.f, p_A = 0.f, p_B = 0.f;
-            if (FUSED) {
-                v_A = reinterpret_cast<const float*>(vel + oA)[l];
-                v_B = reinterpret_cast<const float*>(vel + oB)[l];
-                p_A = reinterpret_cast<const float*>(pos + oA)[l];
-                p_B = reinterpret_cast<const float*>(pos + oB)[l];
-            }
-            float4 pA, pB, vA, vB;
-            if (staged) {
-                pA = s_pos[t.self];
-                pB = s_pos[t.self + two];
-                vA = s_vel[t.self];
-                vB = s_vel[t.self + two];
-            } else {
-                pA = ld_phase<COH>(spos + t.gi);
-                pB = ld_phase<COH>(spos + t.gi + two);
-                vA = ld_phase<COH>(svel + t.gi);
-                vB = ld_phase<COH>(svel + t.gi + two);
-            }
+            const float4 pA = s_pos[t.self], pB = s_pos[t.self + two], vA = s_vel[t.self], vB = s_vel[t.self + two];
             const float aA = rcp_approx(pA.w), aB = rcp_approx(pB.w);
             float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             auto both = [&](const float4& pj, const float4& vj) {
@@ -1539,89 +1630,49 @@ __device__ __forceinline__ bool force_brick_run(float4* s_buf, BrickShared& S, c
                 force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
             };
             const bool scan = meta == NBR_SCAN;
-            if (staged) {
-                const uint32_t n = scan ? 0u : meta, win = smem_addr(s_pos + t.lo);
-                auto entry = [&](uint32_t v) { both(lds_f4(win + v), lds_f4(win + v + FORCE_CAP * 16u)); };
-                for (uint32_t k0 = 2u * l; k0 < n; k0 += 8u * LIST_AHEAD) {
-                    if (k0 >= 8u * LIST_AHEAD) {
+            const uint32_t n = scan ? 0u : meta, win = smem_addr(s_pos + t.lo);
+            auto entry = [&](uint32_t v) { both(lds_f4(win + v), lds_f4(win + v + FORCE_CAP * 16u)); };
+            for (uint32_t k0 = 2u * l; k0 < n; k0 += 8u * LIST_AHEAD) {
+                if (k0 >= 8u * LIST_AHEAD) {
 #pragma unroll
-                        for (uint32_t k = 0; k < LIST_AHEAD; ++k)
-                            if (k0 + 8u * k < n) ch[k] = ld_phase<COH>(list + 4u * k + ((k0 >> 3) << 2));
-                    }
-#pragma unroll
-                    for (uint32_t k = 0; k < LIST_AHEAD; ++k) {
-                        if (k0 + 8u * k >= n) break;
-                        entry(ch[k] & 0xFFFFu);
-                        if (k0 + 8u * k + 1u < n) entry(ch[k] >> 16);
-                    }
+                    for (uint32_t k = 0; k < LIST_AHEAD; ++k)
+                        if (k0 + 8u * k < n) ch[k] = ld_phase<COH>(list + 4u * k + ((k0 >> 3) << 2));
                 }
-            } else {
-                for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
-                    if (lane == 0u) atomicAdd(&S.progress, 1u);
-                    const uint32_t cnt = U.off[i + 1] - U.off[i], first = U.cell[i].x;
-                    for (uint32_t j = l; j < cnt; j += 4u) both(ld_phase<COH>(spos + first + j), ld_phase<COH>(svel + first + j));
+#pragma unroll
+                for (uint32_t k = 0; k < LIST_AHEAD; ++k) {
+                    if (k0 + 8u * k >= n) break;
+                    entry(ch[k] & 0xFFFFu);
+                    if (k0 + 8u * k + 1u < n) entry(ch[k] >> 16);
                 }
             }
-            // pressure and viscosity terms together, then the sums over the pair's lanes
             float f[2][3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                f[0][k] = fmaf(kp.cpress, accA[k], cvisc * accA[3 + k]);
-                f[1][k] = fmaf(kp.cpress, accB[k], cvisc * accB[3 + k]);
-#pragma unroll
-                for (uint32_t m = 1; m < 4u; m <<= 1) {
-                    f[0][k] += __shfl_xor_sync(0xffffffffu, f[0][k], m);
-                    f[1][k] += __shfl_xor_sync(0xffffffffu, f[1][k], m);
-                }
-            }
-            if (staged) {
-                // pairs without a list: the whole warp scans each one's window in turn
-                uint32_t pend = __ballot_sync(0xffffffffu, t.live && scan && l == 0u);
-                while (pend) {
-                    const int src = __ffs((int)pend) - 1;
-                    pend &= pend - 1u;
-                    const uint32_t self = __shfl_sync(0xffffffffu, t.self, src), lo = __shfl_sync(0xffffffffu, t.lo, src),
-                                   len = __shfl_sync(0xffffffffu, t.len, src), more = __shfl_sync(0xffffffffu, two, src);
+            pair_sums(kp, cvisc, accA, accB, f);
+            // pairs without a list: the whole warp scans each one's window in turn
+            uint32_t pend = __ballot_sync(0xffffffffu, t.live && scan && l == 0u);
+            while (pend) {
+                const int src = __ffs((int)pend) - 1;
+                pend &= pend - 1u;
+                const uint32_t self = __shfl_sync(0xffffffffu, t.self, src), lo = __shfl_sync(0xffffffffu, t.lo, src),
+                               len = __shfl_sync(0xffffffffu, t.len, src), more = __shfl_sync(0xffffffffu, two, src);
 #pragma unroll 1
-                    for (uint32_t w = 0; w <= more; ++w) {
-                        const float4 ps = s_pos[self + w], vs = s_vel[self + w];
-                        const float as = rcp_approx(ps.w);
-                        float a[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                        for (uint32_t j = lo + lane; j < lo + len; j += 32u)
-                            force_pair<DIMS>(ps, vs, as, s_pos[j], s_vel[j], rcp_approx(s_pos[j].w), kp.h, thr, a);
+                for (uint32_t w = 0; w <= more; ++w) {
+                    const float4 ps = s_pos[self + w], vs = s_vel[self + w];
+                    const float as = rcp_approx(ps.w);
+                    float a[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    for (uint32_t j = lo + lane; j < lo + len; j += 32u)
+                        force_pair<DIMS>(ps, vs, as, s_pos[j], s_vel[j], rcp_approx(s_pos[j].w), kp.h, thr, a);
 #pragma unroll
-                        for (int k = 0; k < 3; ++k) {
-                            float x = fmaf(kp.cpress, a[k], cvisc * a[3 + k]);
-                            for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
-                            if ((lane >> 2) == (uint32_t)src >> 2) {
-                                if (w) f[1][k] = x;
-                                else f[0][k] = x;
-                            }
+                    for (int k = 0; k < 3; ++k) {
+                        float x = fmaf(kp.cpress, a[k], cvisc * a[3 + k]);
+                        for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+                        if ((lane >> 2) == (uint32_t)src >> 2) {
+                            if (w) f[1][k] = x;
+                            else f[0][k] = x;
                         }
                     }
                 }
             }
-            // lane l takes component l, target A and then target B
-            const float g = l == 0u ? kp.gravity.x : (l == 1u ? kp.gravity.y : (l == 2u ? kp.gravity.z : kp.gravity.w));
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const bool live = t.live && (w == 0 || t.two);
-                const uint32_t o = w ? oB : oA;
-                const float add = l == 0u ? f[w][0] : (l == 1u ? f[w][1] : f[w][2]);
-                float F = l == 3u ? 0.0f : __fadd_rn(w ? f_B : f_A, __fmul_rn(add, kp.mass));
-                if (FUSED) {
-                    F = clip_box_lane<DIMS>(kp, U.box_min, U.box_max, w ? pB : pA, w ? vB : vA, F, l, live);
-                    if (kp.rec_force && live) reinterpret_cast<float*>(kp.rec_force + o)[l] = F;
-                    const float v = integrate_force_lane(kp, w ? v_B : v_A, F);
-                    if (live) {
-                        reinterpret_cast<float*>(vel + o)[l] = v;
-                        reinterpret_cast<float*>(force + o)[l] = g;
-                        reinterpret_cast<float*>(pos + o)[l] = __fadd_rn(w ? p_B : p_A, __fmul_rn(v, kp.dt));
-                    }
-                } else if (live) {
-                    reinterpret_cast<float*>(force + o)[l] = F;
-                }
-            }
+            pair_finish<DIMS, FUSED>(kp, U, t, l, st, f, pA, pB, vA, vB, pos, vel, force);
         }
         turn -= tasks;
         unit_release(S, use);
@@ -1638,7 +1689,7 @@ __global__ void __launch_bounds__(32 * FORCE_CONSUMERS + 32, FORCE_CTAS) k_force
                                                                float4* __restrict__ force,
                                                                const uint2* __restrict__ table,
                                                                const uint32_t* __restrict__ bricks,
-                                                               uint32_t* counters, KParams kp,
+                                                               uint32_t* counters, const __grid_constant__ KParams kp,
                                                                const uint16_t* __restrict__ nbr,
                                                                const uint32_t* __restrict__ nbr_meta,
                                                                uint32_t* err) {
