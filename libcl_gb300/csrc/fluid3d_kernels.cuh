@@ -770,7 +770,9 @@ constexpr int LISTED_WARPS = 2, LISTED_TARGETS = 4;  // per CTA, per warp
 // gathers one after the other, and few particles leave nothing beside them: 20.5 us for 4,096 or
 // 16,384 particles where this takes 10.2 and 12.3. From some 50,000 on its six stores and loads per
 // pair cost more than the wait (65,536: 28.7 / 24.6; 1,048,576: 426 / 217). Two particles per warp
-// 10.2 and 14.3, five 12.3 and 12.3.
+// 10.2 and 14.3, five 12.3 and 12.3. Particles with more neighbours than a list holds take the whole
+// warp as well: left to a lane each, a step of 32,768 particles at twice the usual density a side
+// (four spacings a cell) took 1,251 us, 459 so, 1,008 with a thread per particle.
 template <int MODE, bool POST>
 __global__ void __launch_bounds__(32 * LISTED_WARPS) k_forces_listed(const float4* __restrict__ spos, const float4* __restrict__ svel,
                                                                      float4* __restrict__ force, const uint32_t* __restrict__ index,
@@ -785,6 +787,45 @@ __global__ void __launch_bounds__(32 * LISTED_WARPS) k_forces_listed(const float
     const bool live = lane < T && particle < kp.n;
     const uint32_t all = live ? xc[particle] : 0u;
     const bool scan = all > XL_CAP;
+    // particles without a list, one after the other: the warp goes through the buckets, 32 candidates at a
+    // time, and adds the terms up as often as the particle's rows are full; the sums wait in the rows' last entry
+    for (uint32_t left = __ballot_sync(FULL, scan); left; left &= left - 1) {
+        const uint32_t t = (uint32_t)__ffs((int)left) - 1u, i = first + t;
+        const float4 pi = spos[i], vi = svel[i];
+        uint32_t n = 0;
+        float part = 0.0f;  // of component `lane`
+        auto add = [&]() {
+            __syncwarp();
+            if (lane < 6) {
+#pragma unroll 4
+                for (uint32_t k = 0; k < n; ++k) part = __fadd_rn(part, term[lane * T + t][k]);
+            }
+            __syncwarp();
+            n = 0;
+        };
+        for_each_neighbour_cell<MODE>(kp, tab, pi, [&](uint32_t start, uint32_t end) {
+            for (uint32_t base = start; base < end; base += 32) {
+                const uint32_t j = base + lane;
+                float4 pj = pi;
+                bool in = j < end && j != i;
+                if (in) {
+                    pj = spos[j];
+                    in = exact_r2(__fsub_rn(pi.x, pj.x), __fsub_rn(pi.y, pj.y), __fsub_rn(pi.z, pj.z)) < kp.r2_thresh;
+                }
+                const uint32_t m = __ballot_sync(FULL, in), at = (uint32_t)__popc(m & lanemask_lt());
+                if (n + (uint32_t)__popc(m) > XL_CAP) add();
+                if (in) {
+                    float x[6];
+                    exact_pair(kp, pi, vi, pj, svel[j], x);
+#pragma unroll
+                    for (uint32_t c = 0; c < 6; ++c) term[c * T + t][n + at] = x[c];
+                }
+                n += (uint32_t)__popc(m);
+            }
+        });
+        add();
+        if (lane < 6) term[lane * T + t][XL_CAP] = part;
+    }
     uint32_t before[T + 1];
     before[0] = 0;
 #pragma unroll
@@ -804,9 +845,11 @@ __global__ void __launch_bounds__(32 * LISTED_WARPS) k_forces_listed(const float
         for (uint32_t c = 0; c < 6; ++c) term[c * T + t][k] = v[c];
     }
     __syncwarp();
-    const uint32_t mine = __shfl_sync(FULL, scan ? 0u : all, (int)(lane % T));
+    const uint32_t mine = __shfl_sync(FULL, all, (int)(lane % T));
     float sum = 0.0f;
-    if (lane < 6 * T) {
+    if (lane < 6 * T && mine > XL_CAP) {
+        sum = term[lane][XL_CAP];
+    } else if (lane < 6 * T) {
 #pragma unroll 4
         for (uint32_t k = 0; k < mine; ++k) sum = __fadd_rn(sum, term[lane][k]);
     }
@@ -815,18 +858,6 @@ __global__ void __launch_bounds__(32 * LISTED_WARPS) k_forces_listed(const float
     for (uint32_t c = 0; c < 6; ++c) v[c] = __shfl_sync(FULL, sum, (int)(c * T + lane % T));
     if (!live) return;
     const float4 posI = spos[particle], velI = svel[particle];
-    if (scan)
-        for_each_neighbour_cell<MODE>(kp, tab, posI, [&](uint32_t start, uint32_t end) {
-            for (uint32_t j = start; j < end; j++) {
-                if (j == particle) continue;
-                const float4 p = spos[j];
-                if (!(exact_r2(__fsub_rn(posI.x, p.x), __fsub_rn(posI.y, p.y), __fsub_rn(posI.z, p.z)) < kp.r2_thresh)) continue;
-                float t[6];
-                exact_pair(kp, posI, velI, p, svel[j], t);
-#pragma unroll
-                for (int c = 0; c < 6; ++c) v[c] = __fadd_rn(v[c], t[c]);
-            }
-        });
     exact_finish<POST>(kp, particle, posI, velI, v[0], v[1], v[2], v[3], v[4], v[5], force, index, pos, vel);
 }
 
