@@ -168,32 +168,38 @@ __device__ __forceinline__ void update_state(P2* __restrict__ st, const float2* 
 
 // The neighbour loops of clComputePressure / clComputePosition visit cells x (outer), y (inner)
 // of the 3 x 3 around a particle and the particles of each cell in sorted order, summing in
-// that order. A warp takes SEARCH_TARGETS consecutive sorted particles and
+// that order. A warp takes T consecutive sorted particles and
 //  - for each cell among them goes through the candidates of the nine cells, 32 at a time in
 //    the reference's order, keeps those within h of the box around the cell's targets (no
 //    target is nearer to a candidate than the box, in rounded arithmetic as well: every
 //    operation of the distance is monotone), tests the kept ones against each target and
 //    appends those in range to the target's list;
 //  - then computes the terms of all lists, a lane each, and a lane per target adds them in order.
-// A target with more in range than its list holds is summed by the warp on its own, through the
-// candidates again. At 16,384 particles (the default scene) a warp for every particle, its
-// candidates' terms computed wherever one of 32 was in range and added by shuffles, took 33 us for
-// the pressures and 43 for the positions; this takes 15 and 18. Bound by latency: 27 warps an
-// SM, each a chain of table, candidates, lists, terms and sums. Two targets per warp are no
-// better at this size (116 against 102 us for two steps; 78 against 94 at 4,096), eight 113,
-// and all nine cells instead of those in reach 136.
+// A target with more in range than its list holds takes the warp to itself, through the candidates
+// again, the list as a buffer whose terms are computed side by side whenever it is half full. (With
+// the terms computed where they were found and added by shuffles, 1,024 particles at half the
+// spacing took 164 us a step, 62 now; 16,384 particles 257 and 206. Adding all lists up whenever
+// one was full 124, but 2 to 5 % more for every scene without such targets.)
+// At 16,384 particles (the default scene) a warp for every particle, its candidates' terms computed
+// wherever one of 32 was in range and added by shuffles, took 33 us for the pressures and 43 for
+// the positions; this takes 15 and 18. Bound by latency: 27 warps an SM, each a chain of table,
+// candidates, lists, terms and sums. All nine cells instead of those in reach: 136 us for two
+// steps instead of 102.
+// T: 4, or 2 or 1 where few particles leave the chip idle and only the length of a warp's chain
+// counts. Us a step with 1 / 2 / 4: 2,025 particles 34.5 / 36.9 / 41.6, 4,096 35.4 / 38.6 / 42.4, 5,184 38.0 / 39.5 / 43.5,
+// 8,100 47.4 / 41.3 / 44.5, 10,000 50.6 / 43.6 / 46.2, 12,100 57.3 / 48.4 / 46.6; eight at 16,384: 113 for two steps.
 constexpr int SEARCH_WARPS = 4;           // per CTA
-constexpr int SEARCH_TARGETS = 4;         // per warp
+constexpr uint32_t SEARCH_ONE = 4096, SEARCH_TWO = 8192;  // particles up to which T is 1, 2
 constexpr uint32_t LIST2 = 64;            // entries of a target's list
 constexpr uint32_t HELD2 = 128;           // candidates held before they are tested, a multiple of 32
 
-template <class TERM>
+template <class TERM, int T>
 struct Search2 {
     float2 xy[HELD2];
     uint32_t id[HELD2];
     uint32_t base[32];
-    uint32_t j[SEARCH_TARGETS][LIST2];
-    TERM term[SEARCH_TARGETS][LIST2];  // first the neighbour's distance (x, y), then its terms
+    uint32_t j[T][LIST2];
+    TERM term[T][LIST2];  // first the neighbour's distance (x, y), then its terms
 };
 
 // Whether particle j at distance (dx, dy) is a neighbour of particle i: r > 1e-7 and r < h.
@@ -203,8 +209,8 @@ __device__ __forceinline__ bool near2(const K2& k, float dx, float dy) {
 }
 
 // The candidates of cell (cx, cy) that may be within h of the box (xl..xh, yl..yh): calls
-// f(j, px, py) for 32 at a time (j = EMPTY2 beyond the last), in the reference's order, by the
-// whole warp. Cells are 2 h wide, so that a box in one cell reaches four to six of the nine;
+// f(j, px, py, last) for 32 at a time (j = EMPTY2 beyond the last), in the reference's order, by
+// the whole warp. Cells are 2 h wide, so that a box in one cell reaches four to six of the nine;
 // the slack is a hundred times what rounding can move a particle against its cell's bounds, and
 // the cells at the grid's edges hold what lies beyond as well.
 template <class F>
@@ -255,13 +261,13 @@ __device__ __forceinline__ void for_candidates2(const K2& k, int cx, int cy, con
     uint32_t j = fetch(0, px, py), next = EMPTY2;
     for (uint32_t base = 0; base < total; base += 32, j = next, px = ax, py = ay) {
         if (base + 32 < total) next = fetch(base + 32, ax, ay);
-        f(j, px, py);
+        f(j, px, py, base + 32 >= total);
     }
 }
 
 // Fills the lists of the warp's targets; lane t's `count` is that of target t (may exceed LIST2).
-template <class TERM>
-__device__ __forceinline__ uint32_t search2(Search2<TERM>& S, const K2& k, uint32_t first, bool live, float px, float py,
+template <class TERM, int T>
+__device__ __forceinline__ uint32_t search2(Search2<TERM, T>& S, const K2& k, uint32_t first, bool live, float px, float py,
                                             const P2* __restrict__ srt, const uint2* __restrict__ table) {
     constexpr uint32_t FULL = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
@@ -302,7 +308,7 @@ __device__ __forceinline__ uint32_t search2(Search2<TERM>& S, const K2& k, uint3
             __syncwarp();
             held = 0;
         };
-        for_candidates2(k, cx, cy, srt, table, S.base, xl, xh, yl, yh, [&](uint32_t j, float qx, float qy) {
+        for_candidates2(k, cx, cy, srt, table, S.base, xl, xh, yl, yh, [&](uint32_t j, float qx, float qy, bool) {
             const float dx = fmaxf(fmaxf(fs(xl, qx), fs(qx, xh)), 0.f), dy = fmaxf(fmaxf(fs(yl, qy), fs(qy, yh)), 0.f);
             const bool keep = j != EMPTY2 && fa(fm(dx, dx), fm(dy, dy)) < k.r2_hi;
             const uint32_t m = __ballot_sync(FULL, keep);
@@ -321,9 +327,8 @@ __device__ __forceinline__ uint32_t search2(Search2<TERM>& S, const K2& k, uint3
 }
 
 // Calls f(t, entry) for every entry of the lists, a lane each (lane t's `n` entries of target t).
-template <class F>
+template <int T, class F>
 __device__ __forceinline__ void for_entries2(uint32_t n, F&& f) {
-    constexpr int T = SEARCH_TARGETS;
     uint32_t before[T + 1];
     before[0] = 0;
 #pragma unroll
@@ -351,18 +356,19 @@ struct Pressure2 {
 };
 
 // clComputePressure (libCL/phys/oclFluid2D.cl:185-245).
+template <int T>
 __global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_pressure(const P2* __restrict__ srt, float4* __restrict__ ps,
                                                                  const uint2* __restrict__ table,
                                                                  const float4* __restrict__ bstate, K2 k) {
     constexpr uint32_t FULL = 0xffffffffu;
-    __shared__ Search2<float2> shared[SEARCH_WARPS];
-    Search2<float2>& S = shared[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * SEARCH_TARGETS, i = first + lane;
-    const bool live = lane < SEARCH_TARGETS && i < k.n;
+    __shared__ Search2<float2, T> shared[SEARCH_WARPS];
+    Search2<float2, T>& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * T, i = first + lane;
+    const bool live = lane < T && i < k.n;
     if (first >= k.n) return;  // whole warps
     const float px = live ? srt[i].px : 0.f, py = live ? srt[i].py : 0.f;
-    const uint32_t count = search2<float2>(S, k, first, live, px, py, srt, table);
-    for_entries2(count <= LIST2 ? count : 0u, [&](int t, uint32_t e) {
+    const uint32_t count = search2<float2, T>(S, k, first, live, px, py, srt, table);
+    for_entries2<T>(count <= LIST2 ? count : 0u, [&](int t, uint32_t e) {
         const float2 d = S.term[t][e];
         S.term[t][e] = Pressure2::term(k, d.x, d.y);
     });
@@ -386,19 +392,27 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_pressure(const P2* __res
         const int t = __ffs(more) - 1;
         const uint32_t self = first + (uint32_t)t;
         const float x = __shfl_sync(FULL, px, t), y = __shfl_sync(FULL, py, t);
+        uint32_t n = 0;
         for_candidates2(k, (int)floorf(fd(x, k.cellSize)), (int)floorf(fd(y, k.cellSize)), srt, table, S.base, x, x, y, y,
-                        [&](uint32_t j, float qx, float qy) {
+                        [&](uint32_t j, float qx, float qy, bool last) {
                             const float dx = fs(qx, x), dy = fs(qy, y);
                             const bool hit = j != EMPTY2 && j != self && near2(k, dx, dy);
-                            const float2 v = hit ? Pressure2::term(k, dx, dy) : make_float2(0.f, 0.f);
-                            for (uint32_t m = __ballot_sync(FULL, hit); m; m &= m - 1) {
-                                const int b = __ffs(m) - 1;
-                                const float vx = __shfl_sync(FULL, v.x, b), vy = __shfl_sync(FULL, v.y, b);
-                                if ((int)lane == t) {
-                                    density = fa(density, vx);
-                                    nearDensity = fa(nearDensity, vy);
+                            const uint32_t m = __ballot_sync(FULL, hit);
+                            if (hit) S.term[t][n + (uint32_t)__popc(m & lanemask_lt())] = make_float2(dx, dy);
+                            n += (uint32_t)__popc(m);
+                            if (n <= LIST2 - 32 && !last) return;
+                            __syncwarp();
+                            for (uint32_t e = lane; e < n; e += 32) S.term[t][e] = Pressure2::term(k, S.term[t][e].x, S.term[t][e].y);
+                            __syncwarp();
+                            if ((int)lane == t) {
+#pragma unroll 4
+                                for (uint32_t e = 0; e < n; ++e) {
+                                    density = fa(density, S.term[t][e].x);
+                                    nearDensity = fa(nearDensity, S.term[t][e].y);
                                 }
                             }
+                            __syncwarp();
+                            n = 0;
                         });
     }
     if (live)
@@ -424,6 +438,7 @@ struct Position2 {
 // clComputePosition (libCL/phys/oclFluid2D.cl:247-326) and, as it concerns the particle alone,
 // clUpdateState. The reference's viscosity term uses vel_j - vel_j (:299), which is zero, so
 // it never contributes and is not evaluated here.
+template <int T>
 __global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_position(const P2* __restrict__ srt, const float4* __restrict__ ps,
                                                                  float2* __restrict__ relaxed, const uint2* __restrict__ table,
                                                                  const float4* __restrict__ bstate,
@@ -431,15 +446,15 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_position(const P2* __res
                                                                  const float2* __restrict__ prev,
                                                                  const uint32_t* __restrict__ index, K2 k) {
     constexpr uint32_t FULL = 0xffffffffu;
-    __shared__ Search2<float4> shared[SEARCH_WARPS];
-    Search2<float4>& S = shared[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * SEARCH_TARGETS, i = first + lane;
-    const bool live = lane < SEARCH_TARGETS && i < k.n;
+    __shared__ Search2<float4, T> shared[SEARCH_WARPS];
+    Search2<float4, T>& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * T, i = first + lane;
+    const bool live = lane < T && i < k.n;
     if (first >= k.n) return;  // whole warps
     const float px = live ? srt[i].px : 0.f, py = live ? srt[i].py : 0.f;
     const float dt2 = fm(k.dT, k.dT), tension = fm(fm(dt2, fd(kSurfaceTension, k.m)), k.m);
-    const uint32_t count = search2<float4>(S, k, first, live, px, py, srt, table);
-    for_entries2(count <= LIST2 ? count : 0u, [&](int t, uint32_t e) {
+    const uint32_t count = search2<float4, T>(S, k, first, live, px, py, srt, table);
+    for_entries2<T>(count <= LIST2 ? count : 0u, [&](int t, uint32_t e) {
         const float4 d = S.term[t][e];
         S.term[t][e] = Position2::term(k, dt2, tension, ps[first + t], ps[S.j[t][e]], d.x, d.y);
     });
@@ -457,21 +472,34 @@ __global__ void __launch_bounds__(32 * SEARCH_WARPS) k2_position(const P2* __res
         const uint32_t self = first + (uint32_t)t;
         const float x = __shfl_sync(FULL, px, t), y = __shfl_sync(FULL, py, t);
         const float4 si = ps[self];
+        uint32_t n = 0;
         for_candidates2(k, (int)floorf(fd(x, k.cellSize)), (int)floorf(fd(y, k.cellSize)), srt, table, S.base, x, x, y, y,
-                        [&](uint32_t j, float qx, float qy) {
+                        [&](uint32_t j, float qx, float qy, bool last) {
                             const float dx = fs(qx, x), dy = fs(qy, y);
                             const bool hit = j != EMPTY2 && j != self && near2(k, dx, dy);
-                            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (hit) v = Position2::term(k, dt2, tension, si, ps[j], dx, dy);
-                            for (uint32_t m = __ballot_sync(FULL, hit); m; m &= m - 1) {
-                                const int b = __ffs(m) - 1;
-                                const float ux = __shfl_sync(FULL, v.x, b), uy = __shfl_sync(FULL, v.y, b);
-                                const float wx = __shfl_sync(FULL, v.z, b), wy = __shfl_sync(FULL, v.w, b);
-                                if ((int)lane == t) {
-                                    rx = fa(fs(rx, ux), wx);
-                                    ry = fa(fs(ry, uy), wy);
+                            const uint32_t m = __ballot_sync(FULL, hit);
+                            if (hit) {
+                                const uint32_t at = n + (uint32_t)__popc(m & lanemask_lt());
+                                S.j[t][at] = j;
+                                S.term[t][at].x = dx;
+                                S.term[t][at].y = dy;
+                            }
+                            n += (uint32_t)__popc(m);
+                            if (n <= LIST2 - 32 && !last) return;
+                            __syncwarp();
+                            for (uint32_t e = lane; e < n; e += 32)
+                                S.term[t][e] = Position2::term(k, dt2, tension, si, ps[S.j[t][e]], S.term[t][e].x, S.term[t][e].y);
+                            __syncwarp();
+                            if ((int)lane == t) {
+#pragma unroll 4
+                                for (uint32_t e = 0; e < n; ++e) {
+                                    const float4 v = S.term[t][e];
+                                    rx = fa(fs(rx, v.x), v.z);
+                                    ry = fa(fs(ry, v.y), v.w);
                                 }
                             }
+                            __syncwarp();
+                            n = 0;
                         });
     }
     if (!live) return;
@@ -772,10 +800,15 @@ int enqueue2(H2* h, const K2& k, cudaStream_t s) {
         k_bounds_hash<<<g, 256, 0, s>>>(h->keys_c, k.n, h->cells, k.table, h->err);
         GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     }
-    const uint32_t per = SEARCH_TARGETS * SEARCH_WARPS, blocks = (k.n + per - 1) / per;
-    k2_pressure<<<blocks, 32 * SEARCH_WARPS, 0, s>>>(h->sorted, h->pstate, h->cells, h->bstate, k);
-    k2_position<<<blocks, 32 * SEARCH_WARPS, 0, s>>>(h->sorted, h->pstate, h->relaxed, h->cells, h->bstate, h->bvec, state, h->prev,
-                                                     h->index, k);
+    auto relax = [&](uint32_t targets, auto pressure, auto position) {
+        const uint32_t per = targets * SEARCH_WARPS, blocks = (k.n + per - 1) / per;
+        pressure<<<blocks, 32 * SEARCH_WARPS, 0, s>>>(h->sorted, h->pstate, h->cells, h->bstate, k);
+        position<<<blocks, 32 * SEARCH_WARPS, 0, s>>>(h->sorted, h->pstate, h->relaxed, h->cells, h->bstate, h->bvec, state, h->prev, h->index,
+                                                      k);
+    };
+    if (k.n <= SEARCH_ONE) relax(1, k2_pressure<1>, k2_position<1>);
+    else if (k.n <= SEARCH_TWO) relax(2, k2_pressure<2>, k2_position<2>);
+    else relax(4, k2_pressure<4>, k2_position<4>);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
