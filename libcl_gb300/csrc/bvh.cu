@@ -631,9 +631,9 @@ __device__ __forceinline__ bool collide_box(const float4& lo, const float4& hi, 
 }
 
 constexpr uint32_t QUEUE_SIZE = 256;
-constexpr uint32_t COLLIDE_THREADS = 128, COLLIDE_LANES = 8;
+constexpr uint32_t COLLIDE_THREADS = 128;
 
-// COLLIDE_LANES lanes take a particle: they pop that many queue entries at a time (a triangle
+// LANES lanes take a particle: they pop that many queue entries at a time (a triangle
 // test or two box tests each) and push the hit children at the places a sequential run gives
 // them, so the order of the tests, and with it the first triangle hit, is the reference's. Where
 // a batch could fill the 256-entry ring, which then counts as empty, entries go one by one, as
@@ -646,6 +646,11 @@ constexpr uint32_t COLLIDE_THREADS = 128, COLLIDE_LANES = 8;
 // (720-900 us, L1 thrashing). 8 lanes: 590 us; three-operand min / max for tame rays: 475 us; the
 // triangles in batches: 425 us. 4 lanes 640 us, 16 lanes 650 us. Bound by the ALU pipe and by the
 // latency of the nodes.
+// A tree of few nodes does not fill eight lanes, nor the ring: its nodes all fit a smaller one, which
+// then never wraps. Us for 1,000,000 particles with 1 / 4 / 8 lanes and by a thread per particle with its
+// queue in local memory: 2 triangles 45 / 97 / 163 / 50, 8 127 / 167 / 295 / 154, 33 - / 290 / 463 / 360, 63 - / 432 / 524 / 604; for 256 and
+// 4 to 8 triangles one lane takes 22 to 24, four or eight 18 to 20.
+template <uint32_t LANES, uint32_t RING>
 __global__ void __launch_bounds__(COLLIDE_THREADS, 8) k_collide_bvh(float4* __restrict__ force, float4* __restrict__ position,
                                                              float4* __restrict__ velocity, uint32_t np,
                                                              CollideParams P, const gbsph_bvh_node* __restrict__ bvh,
@@ -653,14 +658,14 @@ __global__ void __launch_bounds__(COLLIDE_THREADS, 8) k_collide_bvh(float4* __re
                                                              const uint32_t* __restrict__ index,
                                                              const float4* __restrict__ vertex, uint32_t nv,
                                                              uint32_t* err) {
-    __shared__ uint32_t s_queue[COLLIDE_THREADS / COLLIDE_LANES][QUEUE_SIZE];
-    __shared__ uint32_t s_leaf[COLLIDE_THREADS / COLLIDE_LANES][2 * COLLIDE_LANES];
-    const uint32_t lane = threadIdx.x & 31u, gl = lane % COLLIDE_LANES;
-    const uint32_t group = ((1u << COLLIDE_LANES) - 1u) << (lane - gl), before = group & lanemask_lt();
-    uint32_t* queue = s_queue[threadIdx.x / COLLIDE_LANES];
-    uint32_t* leaf = s_leaf[threadIdx.x / COLLIDE_LANES];
+    __shared__ uint32_t s_queue[COLLIDE_THREADS / LANES][RING];
+    __shared__ uint32_t s_leaf[COLLIDE_THREADS / LANES][2 * LANES];
+    const uint32_t lane = threadIdx.x & 31u, gl = lane % LANES;
+    const uint32_t group = ((1u << LANES) - 1u) << (lane - gl), before = group & lanemask_lt();
+    uint32_t* queue = s_queue[threadIdx.x / LANES];
+    uint32_t* leaf = s_leaf[threadIdx.x / LANES];
     uint32_t leaves = 0;  // triangles popped and not tested yet
-    const uint32_t p = blockIdx.x * (COLLIDE_THREADS / COLLIDE_LANES) + threadIdx.x / COLLIDE_LANES;
+    const uint32_t p = blockIdx.x * (COLLIDE_THREADS / LANES) + threadIdx.x / LANES;
     bool active = p < np;
     F4 pos{}, vel{};
     if (active) {
@@ -683,9 +688,9 @@ __global__ void __launch_bounds__(COLLIDE_THREADS, 8) k_collide_bvh(float4* __re
     __syncwarp();
     for (;;) {
         const bool going = __any_sync(0xffffffffu, active);
-        if (!going || __any_sync(0xffffffffu, leaves >= COLLIDE_LANES)) {
+        if (!going || __any_sync(0xffffffffu, leaves >= LANES)) {
             // the triangles that wait, a lane each, in the order they were popped
-            const uint32_t n = min(leaves, COLLIDE_LANES), tri = leaf[gl], next = leaf[COLLIDE_LANES + gl];
+            const uint32_t n = min(leaves, LANES), tri = leaf[gl], next = leaf[LANES + gl];
             bool hit = false;
             if (gl < n) {
                 F4 x = pos, v = vel, f{};
@@ -710,10 +715,10 @@ __global__ void __launch_bounds__(COLLIDE_THREADS, 8) k_collide_bvh(float4* __re
             if (!going && !__any_sync(0xffffffffu, leaves != 0u)) break;
             if (!going) continue;
         }
-        const uint32_t waiting = (tail - head) % QUEUE_SIZE;
-        uint32_t k = active ? min(COLLIDE_LANES, waiting) : 0u;
-        if (waiting + k >= QUEUE_SIZE) k = min(k, 1u);
-        const uint32_t it = queue[(head + gl) % QUEUE_SIZE];
+        const uint32_t waiting = (tail - head) % RING;
+        uint32_t k = active ? min(LANES, waiting) : 0u;
+        if (waiting + k >= RING) k = min(k, 1u);
+        const uint32_t it = queue[(head + gl) % RING];
         __syncwarp();
         bool hl = false, hr = false, tri = false;
         int4 w = make_int4(0, 0, 0, 0);
@@ -737,10 +742,10 @@ __global__ void __launch_bounds__(COLLIDE_THREADS, 8) k_collide_bvh(float4* __re
         if (tri) leaf[leaves + (uint32_t)__popc(bt & before)] = (uint32_t)w.z;
         leaves += (uint32_t)__popc(bt);
         const uint32_t at = tail + (uint32_t)__popc(bl & before) + (uint32_t)__popc(br & before);
-        if (hl) queue[at % QUEUE_SIZE] = (uint32_t)w.x;
-        if (hr) queue[(at + (hl ? 1u : 0u)) % QUEUE_SIZE] = (uint32_t)w.y;
-        head = (head + k) % QUEUE_SIZE;
-        tail = (tail + (uint32_t)__popc(bl) + (uint32_t)__popc(br)) % QUEUE_SIZE;
+        if (hl) queue[at % RING] = (uint32_t)w.x;
+        if (hr) queue[(at + (hl ? 1u : 0u)) % RING] = (uint32_t)w.y;
+        head = (head + k) % RING;
+        tail = (tail + (uint32_t)__popc(bl) + (uint32_t)__popc(br)) % RING;
         steps += k;
         if (active && steps > 4u * n_nodes + 4u) {  // not a tree: report and stop
             if (gl == 0) atomicOr(err, DEV_ERR_KEY_RANGE);
@@ -773,11 +778,16 @@ extern "C" GBSPH_API int gbsph_bvh_collide(gbsph_bvh_t h, const gbsph_fluid3d_pa
     P.h = params->cellSize;
     P.mass = params->mass;
     const uint32_t np = (uint32_t)n_particles;
-    constexpr uint32_t per = COLLIDE_THREADS / COLLIDE_LANES;
-    k_collide_bvh<<<(np + per - 1u) / per, COLLIDE_THREADS, 0, s>>>(reinterpret_cast<float4*>(force), reinterpret_cast<float4*>(position),
-                                                   reinterpret_cast<float4*>(velocity), np, P, h->node, h->root,
-                                                   2 * h->n - 1, index, reinterpret_cast<const float4*>(vertex),
-                                                   (uint32_t)n_vertices, h->err);
+    auto collide = [&](auto kern, uint32_t lanes) {
+        const uint32_t per = COLLIDE_THREADS / lanes;
+        kern<<<(np + per - 1u) / per, COLLIDE_THREADS, 0, s>>>(reinterpret_cast<float4*>(force), reinterpret_cast<float4*>(position),
+                                                               reinterpret_cast<float4*>(velocity), np, P, h->node, h->root, 2 * h->n - 1,
+                                                               index, reinterpret_cast<const float4*>(vertex), (uint32_t)n_vertices, h->err);
+    };
+    const uint32_t nodes = 2 * h->n - 1;
+    if (nodes < 16 && np >= 1u << 16) collide(k_collide_bvh<1, 16>, 1);
+    else if (nodes < 128) collide(k_collide_bvh<4, 128>, 4);
+    else collide(k_collide_bvh<8, QUEUE_SIZE>, 8);
     GBSPH_CUDA_TRY(&h->last_error, cudaGetLastError());
     return GBSPH_OK;
 }
