@@ -307,18 +307,6 @@ int ensure_tables(H* h) {
             invalidate_graph(h);
         }
     }
-    // the counting sort's counts, only where it is used
-    const size_t cells = h->params.keyMode == GBSPH_KEY_LINEAR_GRID ? h->table_cells : (size_t)REF_BUCKETS;
-    if (h->opt_fused && count_sort_fits((uint32_t)cells, (uint32_t)h->n) && count_words((uint32_t)cells) > h->count_words) {
-        if (h->count) cudaFree(h->count);
-        h->count = nullptr;
-        h->count_words = 0;
-        GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->count, count_words((uint32_t)cells) * 4));
-        GBSPH_CUDA_TRY(&h->last_error, fill_now(h->count, 0, count_words((uint32_t)cells) * 4));
-        h->count_words = count_words((uint32_t)cells);
-        h->count_clean = true;
-        invalidate_graph(h);
-    }
     return GBSPH_OK;
 }
 
@@ -371,6 +359,28 @@ int st_sort(H* h, const KParams& kp, cudaStream_t s, bool gather, cudaEvent_t be
 }
 
 bool use_rank_sort(const H* h, const KParams& kp) { return h->opt_fused && rank_sort_fits(kp.table_cells, kp.n); }
+
+// The counting sort's counts, where it is used.
+int ensure_counts(H* h, const KParams& kp, cudaStream_t s) {
+    const size_t words = count_words(kp.table_cells);
+    if (!h->opt_fused || rank_sort_fits(kp.table_cells, kp.n) || !count_sort_fits(kp.table_cells, kp.n) || words <= h->count_words)
+        return GBSPH_OK;
+    if (h->count) cudaFree(h->count);
+    h->count = nullptr;
+    h->count_words = 0;
+    GBSPH_CUDA_TRY(&h->last_error, cudaMalloc(&h->count, words * 4));
+    h->count_words = words;
+    // The step sets them to zero first; if it is only being captured, the next one may run before it.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool eager = cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (!eager) {
+        cudaGetLastError();
+        GBSPH_CUDA_TRY(&h->last_error, fill_now(h->count, 0, words * 4));
+    }
+    h->count_clean = !eager;
+    invalidate_graph(h);
+    return GBSPH_OK;
+}
 
 bool use_count_sort(const H* h, const KParams& kp) {
     return !use_rank_sort(h, kp) && h->count && count_sort_fits(kp.table_cells, kp.n) && count_words(kp.table_cells) <= h->count_words;
@@ -925,6 +935,7 @@ int compute_impl(H* h, cudaStream_t s, const HostIO* io, bool io_graph) {
     RC(ensure_tables(h));
     RC(refresh_param_buffer(h, s));
     const KParams kp = make_kparams(h);
+    RC(ensure_counts(h, kp, s));
     const size_t bytes = (size_t)kp.n * 16;
     if (!h->opt_fused) {
         if (io)
