@@ -606,15 +606,21 @@ GBSPH_API int gbsph_batch3d_autotune(gbsph_batch3d_t h, void* stream, int* best_
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    // every combination of brick width x digit width x sort tile x step form
+    // every combination of brick width x digit width x sort tile x step form; a staged step by the
+    // counting sort uses neither digits nor tiles: once a width, with the values that are set
     const int widths[3] = {4, 8, 16}, digits[3] = {6, 7, 8}, items[2] = {8, 16};
     const int forms = (h->step_blocks[0] && h->step_blocks[1]) ? 2 : 1;
     const int end_bit = bits_for_b(h->cells);
     float best = 1e30f;
+    const int set_d = sort_passes(0, end_bit, h->digit_bits) > SORT_MAX_PASSES ? SORT_RADIX_BITS : h->digit_bits, set_i = sort_items_of(h);
     int best_w = h->bw, best_d = h->digit_bits, best_i = h->sort_items, best_p = h->persistent, rc = GBSPH_OK;
+    bool counted[3] = {};  // widths timed with the counting sort
     for (int c = 0; c < 3 * 3 * 2 * forms && !rc; c++) {
-        const int w = widths[c / (3 * 2 * forms)], d = digits[(c / (2 * forms)) % 3], it = items[(c / forms) % 2],
-                  pf = c % forms;
+        const int wi = c / (3 * 2 * forms), w = widths[wi], pf = c % forms;
+        const bool count = h->count && !pf;
+        if (count && counted[wi]) continue;
+        counted[wi] = counted[wi] || count;
+        const int d = count ? set_d : digits[(c / (2 * forms)) % 3], it = count ? set_i : items[(c / forms) % 2];
         if (sort_passes(0, end_bit, d) > SORT_MAX_PASSES) continue;
         h->bw = w;
         h->digit_bits = d;
