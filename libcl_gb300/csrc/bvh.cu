@@ -512,7 +512,7 @@ GBSPH_API int gbsph_bvh_sync_status(gbsph_bvh_t h, void* stream) {
     GBSPH_CUDA_TRY(&h->last_error, cudaMemcpy(&bits, h->err, 4, cudaMemcpyDeviceToHost));
     if (bits) {
         GBSPH_CUDA_TRY(&h->last_error, cudaMemset(h->err, 0, 4));
-        return fail(&h->last_error, dev_err_to_status(bits), "a triangle index is outside the vertex buffer");
+        return fail(&h->last_error, dev_err_to_status(bits), "a triangle index is outside the vertex buffer, or collide() met a root or tree that is not the build's");
     }
     return GBSPH_OK;
 }
