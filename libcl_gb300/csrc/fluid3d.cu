@@ -330,8 +330,7 @@ int st_hash(H* h, const KParams& kp, cudaStream_t s, bool clear) {
 
 // Sorts the keys; with `gather` the last pass also gathers the sorted positions and, with
 // gather_vel, the sorted velocities.
-int st_sort(H* h, const KParams& kp, cudaStream_t s, bool gather, cudaEvent_t before_last = nullptr,
-            bool gather_vel = true) {
+int st_sort(H* h, const KParams& kp, cudaStream_t s, bool gather, bool gather_vel = true) {
     OnesweepArgs a;
     a.keys_in = h->keys_a;
     a.vals_in = nullptr;
@@ -353,7 +352,6 @@ int st_sort(H* h, const KParams& kp, cudaStream_t s, bool gather, cudaEvent_t be
         a.gather.dst[0] = h->spos;
         a.gather.dst[1] = h->svel;
     }
-    a.before_last = before_last;
     GBSPH_CUDA_TRY(&h->last_error, onesweep_passes(a, s));
     return GBSPH_OK;
 }
@@ -488,8 +486,8 @@ int st_forces_exact(H* h, const KParams& kp, cudaStream_t s, bool lists = false,
             kern<<<(kp.n + per - 1) / per, 32 * LISTED_WARPS, 0, s>>>(h->spos, h->svel, P4(h, 2), h->index, h->hash_table, kp, xl, xc, P4(h, 0),
                                                                       P4(h, 1));
         };
-        if (post) listed(k_forces_listed<HASH, true>);
-        else listed(k_forces_listed<HASH, false>);
+        if (post) listed(k_forces_listed<true>);
+        else listed(k_forces_listed<false>);
     } else if (kp.key_mode == LIN) launch(k_forces_exact<LIN, false, false>, h->table);
     else if (lists && post) launch(k_forces_exact<HASH, true, true>, h->hash_table);
     else if (lists) launch(k_forces_exact<HASH, true, false>, h->hash_table);
@@ -626,7 +624,7 @@ int enqueue_fused(H* h, const KParams& kp, cudaStream_t s, const HostIO* io = nu
     } else {
         RC(st_hash(h, kp, s, clear));
         RC(mark(h, 1, s));
-        RC(st_sort(h, kp, s, true, nullptr, io == nullptr));
+        RC(st_sort(h, kp, s, true, io == nullptr));
     }
     auto gather_velocity = [&]() -> int {
         if (!io) return GBSPH_OK;

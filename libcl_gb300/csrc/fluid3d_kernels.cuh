@@ -775,7 +775,7 @@ constexpr int LISTED_WARPS = 2, LISTED_TARGETS = 4;  // per CTA, per warp
 // 10.2 and 14.3, five 12.3 and 12.3. Particles with more neighbours than a list holds take the whole
 // warp as well: left to a lane each, a step of 32,768 particles at twice the usual density a side
 // (four spacings a cell) took 1,251 us, 459 so, 1,008 with a thread per particle.
-template <int MODE, bool POST>
+template <bool POST>
 __global__ void __launch_bounds__(32 * LISTED_WARPS) k_forces_listed(const float4* __restrict__ spos, const float4* __restrict__ svel,
                                                                      float4* __restrict__ force, const uint32_t* __restrict__ index,
                                                                      const uint2* __restrict__ tab, KParams kp,
@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(32 * LISTED_WARPS) k_forces_listed(const float
             __syncwarp();
             n = 0;
         };
-        for_each_neighbour_cell<MODE>(kp, tab, pi, [&](uint32_t start, uint32_t end) {
+        for_each_neighbour_cell<GBSPH_KEY_REFERENCE_HASH>(kp, tab, pi, [&](uint32_t start, uint32_t end) {
             for (uint32_t base = start; base < end; base += 32) {
                 const uint32_t j = base + lane;
                 float4 pj = pi;

@@ -88,7 +88,6 @@ struct OnesweepArgs {
     void* scratch = nullptr;
     uint32_t* err = nullptr;
     SortGather gather;
-    cudaEvent_t before_last = nullptr;  // if set: the last pass waits for it (its gather's inputs)
     int digit_bits = SORT_RADIX_BITS;   // bits per pass (1 to 8, at most SORT_MAX_PASSES passes)
     int items = 0;                      // keys per thread of a tile (8 or 16); 0: by key count
 };
