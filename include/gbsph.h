@@ -293,9 +293,12 @@ GBSPH_API int gbsph_fluid3d_sync_status(gbsph_fluid3d_t h, void* stream);
  * y = 0.6 (10 per row, 2 particleRadius apart) with velocity (0, emit_speed, 0). */
 GBSPH_API int gbsph_fluid3d_emit(gbsph_fluid3d_t h, uint32_t emit, float emit_speed, void* stream);
 /* With GBSPH_OPT_PROFILE on: waits for the last profiled compute() and writes the duration
- * in milliseconds of each of its stages (front end = scratch clear + hash, sort passes incl.
- * the fused reorder, cell bounds, density, forces + integration) into ms[0..4]. Returns the
- * number of stages written (5) or a negative status. Replaces oclKernel::getStartTime /
+ * in milliseconds of each of its stages (front end, sort, cell bounds, density, forces +
+ * integration) into ms[0..4]. Where a step sorts by counting cells or by comparing particles (the
+ * usual case), sort holds keys, sort, reorder and bounds together, and front end and bounds next
+ * to nothing (the clearing of tables at most); by radix passes front end is the scratch clear
+ * and the keys, sort the passes with the reorder. Returns the number of stages written (5) or a
+ * negative status. Replaces oclKernel::getStartTime /
  * getEndTime (libCL/oclKernel.cpp:167-202). */
 GBSPH_API int gbsph_fluid3d_stage_times(gbsph_fluid3d_t h, float* ms, int max_stages);
 GBSPH_API const char* gbsph_fluid3d_last_error(gbsph_fluid3d_t h);
@@ -332,8 +335,10 @@ GBSPH_API void* gbsph_batch3d_get_buffer(gbsph_batch3d_t h, int which, size_t* c
 /* First particle and particle count of scene `s`. */
 GBSPH_API int gbsph_batch3d_scene_range(gbsph_batch3d_t h, int s, size_t* first, size_t* count);
 /* GBSPH_OPT_CUDA_GRAPH, GBSPH_OPT_BRICK_WIDTH, GBSPH_OPT_RADIX_BITS, GBSPH_OPT_SORT_TILE,
- * GBSPH_OPT_PERSISTENT. A digit width that needs more than four passes over the batch's
- * keys is refused by compute() (GBSPH_ERR_ARGUMENT). */
+ * GBSPH_OPT_PERSISTENT. Digit width and sort tile serve the persistent form and batches of more
+ * than 32 cells per particle; other staged steps sort by counting cells and use neither. A digit
+ * width that needs more than four passes over the batch's keys is refused by compute()
+ * (GBSPH_ERR_ARGUMENT) in any form. */
 GBSPH_API int gbsph_batch3d_set_option(gbsph_batch3d_t h, int option, int value);
 /* Current value of one of the options above. */
 GBSPH_API int gbsph_batch3d_get_option(gbsph_batch3d_t h, int option, int* value);
@@ -342,7 +347,7 @@ GBSPH_API int gbsph_batch3d_compute(gbsph_batch3d_t h, void* stream);
 /* Times the step on the current state (which is saved and restored) for every combination
  * of brick width (4, 8, 16), sort digit width (6, 7, 8 bits, where four passes cover the
  * keys), sort tile (8 or 16 keys per thread) and step form (staged graph or persistent
- * kernel), keeps the fastest and returns its brick width through best_width (the others
+ * kernel; a staged form that uses neither digits nor tiles once a width, with those set), keeps the fastest and returns its brick width through best_width (the others
  * through gbsph_batch3d_get_option). Synchronises `stream`. */
 GBSPH_API int gbsph_batch3d_autotune(gbsph_batch3d_t h, void* stream, int* best_width);
 GBSPH_API int gbsph_batch3d_sync_status(gbsph_batch3d_t h, void* stream);

@@ -412,7 +412,8 @@ class Fluid3D:
         self._check(self._lib.gbsph_fluid3d_emit(self._h, emit, emit_speed, _stream(stream)))
 
     def stage_times(self) -> dict:
-        """Per-stage milliseconds of the last compute() run with OPT_PROFILE on."""
+        """Per-stage milliseconds of the last compute() run with OPT_PROFILE on (with the counting or the
+        comparison sort, "sort" holds keys, sort, reorder and bounds together)."""
         buf = (C.c_float * 5)()
         n = self._lib.gbsph_fluid3d_stage_times(self._h, buf, 5)
         if n < 0:

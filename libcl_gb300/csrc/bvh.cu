@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_bvh_tree(const uint32_t* __res
                                                           uint32_t n, typename T::Prims prims, typename T::Node* node,
                                                           unsigned long long* link, uint32_t* __restrict__ root) {
     using Box = typename T::Box;
-    __shared__ uint32_t s_key[TREE_THREADS + 2];  // keys base - 1 ... base + 256
+    __shared__ uint32_t s_key[TREE_THREADS + 2];  // keys base - 1 ... base + TREE_THREADS
     __shared__ Box s_box[2][TREE_THREADS];         // a node's left and right child
     __shared__ uint2 s_end[2][TREE_THREADS];       // their far ends and ids
     __shared__ uint32_t s_came[TREE_THREADS];      // bit 0: left, bit 1: right
@@ -644,8 +644,8 @@ constexpr uint32_t COLLIDE_THREADS = 128;
 // local memory) every pop waited for its node and its children in turn: 1,120 us, 640 us with
 // the ray's constants taken out of the box tests, and more resident threads were slower
 // (720-900 us, L1 thrashing). 8 lanes: 590 us; three-operand min / max for tame rays: 475 us; the
-// triangles in batches: 425 us. 4 lanes 640 us, 16 lanes 650 us. Bound by the ALU pipe and by the
-// latency of the nodes.
+// triangles in batches: 425 us. 4 lanes 640 us, 16 lanes 650 us. Bound by the latency of
+// the nodes (the longest of its stalls; issue 56% of cycles, the LSU pipe 61%).
 // A tree of few nodes does not fill eight lanes, nor the ring: its nodes all fit a smaller one, which
 // then never wraps. Us for 1,000,000 particles with 1 / 4 / 8 lanes and by a thread per particle with its
 // queue in local memory: 2 triangles 45 / 97 / 163 / 50, 8 127 / 167 / 295 / 154, 33 - / 290 / 463 / 360, 63 - / 432 / 524 / 604; for 256 and

@@ -182,8 +182,8 @@ __device__ __forceinline__ void update_state(P2* __restrict__ st, const float2* 
 // one was full 124, but 2 to 5 % more for every scene without such targets.)
 // At 16,384 particles (the default scene) a warp for every particle, its candidates' terms computed
 // wherever one of 32 was in range and added by shuffles, took 33 us for the pressures and 43 for
-// the positions; this takes 15 and 18. Bound by latency: 27 warps an SM, each a chain of table,
-// candidates, lists, terms and sums. All nine cells instead of those in reach: 136 us for two
+// the positions; this takes 15 and 18. Bound by latency: 27 warps an SM (issue
+// 60% of cycles), each a chain of table, candidates, lists, terms and sums. All nine cells instead of those in reach: 136 us for two
 // steps instead of 102.
 // T: 4, or 2 or 1 where few particles leave the chip idle and only the length of a warp's chain
 // counts. Us a step with 1 / 2 / 4: 2,025 particles 34.5 / 36.9 / 41.6, 4,096 35.4 / 38.6 / 42.4, 5,184 38.0 / 39.5 / 43.5,

@@ -48,7 +48,7 @@ struct gbsph_fluid3d_s {
     uint32_t *keys_a = nullptr, *keys_b = nullptr, *keys_c = nullptr;
     uint32_t *vals_a = nullptr, *vals_b = nullptr, *index = nullptr, *bricks = nullptr;
     uint16_t* nbr = nullptr;      // per particle NBR_CAP neighbour slots (density -> forces)
-    uint32_t* nbr_meta = nullptr;  // per particle: list length or scan flag, cell x
+    uint32_t* nbr_meta = nullptr;  // per pair's first particle: list length or scan flag
     uint2* hash_table = nullptr;      // REFERENCE_HASH: start, end of each bucket
     uint32_t* count = nullptr;        // the counting sort's cell counts, zero between steps
     size_t count_words = 0;

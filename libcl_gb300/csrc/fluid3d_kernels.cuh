@@ -1,7 +1,8 @@
 // fluid3d_kernels.cuh -- device code of the 3D (and 2D poly6/spiky) SPH step.
 //
 // Two families of neighbour kernels:
-//   * "exact" kernels (thread per sorted particle) restate clCalculateDensity /
+//   * "exact" kernels (the density by warps of several particles, the forces a thread per particle or by
+//     warps) restate clCalculateDensity /
 //     clCalculateForces (libCL/phys/oclFluid3D.cl:150-255) operation for operation with
 //     round-to-nearest intrinsics (no FMA contraction, IEEE sqrt and division), visiting the
 //     27 (or 9) neighbour cells in the reference's z, y, x order. In REFERENCE_HASH mode that
@@ -373,7 +374,7 @@ struct ExactWarp {
 // the 32 lanes at work, and the root and the sum executed for nearly every candidate because
 // some lane is in range) took 522 us for 1,048,576 particles, 324 candidates and 34 in range
 // each, and 23.6 us for 256, all of it the chain of table reads; this takes 393 and 7.7 us.
-// Bound by instruction issue (76% of cycles). A list that is summed only
+// Bound by instruction issue (78% of cycles). A list that is summed only
 // at the end and, beyond XL_CAP, from the buckets again: 377, but 2.6 ms instead of 0.9 at 0.7 x the
 // spacing (100 in range). Tried with that: 64 and 192 candidates held (+3 %), 32 targets per
 // warp (+13 %), the two candidates of a lane next to each other (+5 %).
@@ -939,10 +940,10 @@ static __global__ void k_emitter(float4* __restrict__ pos, float4* __restrict__ 
 //
 // 1,048,576 particles at the start of the block collapse (8 per cell, 216 candidates and 34 in
 // range each): density 137 us (213 us with the rows staged by bulk copies, a warp per cell and
-// lists appended per candidate), forces 150 us (184 us with two lanes per target and the lists
-// staged). Density is bound by instruction issue (79% of cycles; 63 of the 137 us are the
+// lists appended per candidate), forces 150 to 152 us (184 us with two lanes per target and the lists
+// staged). Density is bound by instruction issue (77% of cycles; 63 of the 137 us are the
 // candidate loop at 21 instructions for 64 pairs, 20 the lists, 16 the staging), forces by issue
-// and shared-memory wavefronts (55% and 64%).
+// and the LSU pipe's wavefronts (57% and 66%).
 // Tried: a bulk copy per cell instead of the 16-byte asynchronous copies (170 / 260 us: the
 // small copies queue), two producers, one per buffer (139 / 178), 3 to 7 consumers at 3 to 6
 // CTAs per SM (density 133-137, forces 150-172).
