@@ -54,7 +54,7 @@ static_assert(SORT_MAX_PASSES * SORT_RADIX * 4 <= STEP_SMEM, "hash phase layout"
 // resident: occupancy x SMs. Data written by one phase and read by a later one is read
 // through L2 (ld_phase<true>, asynchronous copies).
 template <int ITEMS>
-__global__ void __launch_bounds__(BRICK_THREADS, 3) k_batch_step(BatchStepArgs a, const __grid_constant__ KParams kp) {
+__global__ void __launch_bounds__(BRICK_THREADS, 3) k_batch_step(BatchStepArgs a, KParams kp) {
     extern __shared__ float4 s_dyn[];
     __shared__ BrickShared S;
     __shared__ uint32_t s_flag;

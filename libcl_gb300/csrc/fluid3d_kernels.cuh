@@ -15,6 +15,8 @@
 //     tolerance.
 #pragma once
 
+#include <type_traits>
+
 #include "device.cuh"
 #include "internal.h"
 
@@ -939,8 +941,8 @@ static __global__ void k_emitter(float4* __restrict__ pos, float4* __restrict__ 
 // of either (about 46 entries where each has 34).
 //
 // 1,048,576 particles at the start of the block collapse (8 per cell, 216 candidates and 34 in
-// range each): density 137 us (213 us with the rows staged by bulk copies, a warp per cell and
-// lists appended per candidate), forces 150 to 152 us (184 us with two lanes per target and the lists
+// range each): density 136 us (213 us with the rows staged by bulk copies, a warp per cell and
+// lists appended per candidate), forces 149 us (184 us with two lanes per target and the lists
 // staged). Density is bound by instruction issue (77% of cycles; 63 of the 137 us are the
 // candidate loop at 21 instructions for 64 pairs, 20 the lists, 16 the staging), forces by issue
 // and the LSU pipe's wavefronts (57% and 66%).
@@ -961,14 +963,15 @@ constexpr uint32_t LIST_STRIDE = 2 * NBR_CAP + 8;  // halves between a warp's li
 constexpr uint32_t NBR_SCAN = 0xFFFFFFFFu;        // nbr_meta: no list, the force pass scans
 constexpr uint32_t REC_SCAN = 0xFFFFFFFFu;        // rec_cnt: no recorded list for this particle
 
-// One staged unit.
+// One unit.
 struct BrickUnit {
     uint32_t off[BRICK_CELLS + 1];  // staged place of cell (column * R + row); the last entry: all candidates
     uint2 cell[BRICK_CELLS];        // the cell's first sorted index; staged place | count << 16 (staged units)
     uint32_t pair[BRICK_UNIT];      // pairs before target cell c (beyond the last cell: npair)
     uint32_t npair;
-    int ncell;                      // target cells (columns 1 .. ncell); 0: no more units
+    int ncell;                      // target cells (columns 1 .. ncell); 0: an end
     int staged;                     // 0: the candidates did not fit, read them from global memory
+    int more;                       // at an end: units of the other kind follow
     float stiff, cvisc;             // the scene's parameters (they differ within a batch)
     float4 box_min, box_max;
 };
@@ -1038,8 +1041,11 @@ __device__ __forceinline__ void brick_fini(BrickShared& S) {
 
 // The producer warp's loop (see above). `queue` is the pass's brick counter; a0 (and a1 with
 // NARR = 2) the sorted arrays to stage: buffer s holds a0's candidates at s_buf + s * NARR * CAP
-// and a1's CAP entries behind. Returns false if a wait gave up.
-template <int DIMS, bool BATCH, uint32_t CAP, int NARR>
+// and a1's CAP entries behind. With SPLIT a brick that has units of both kinds, staged and not, is gone
+// through once for either, and an end is put between units of different kinds, so that consumers have a loop
+// for each: with both in one, the staged targets of the force pass took 149 to 153 us where they
+// take 147 now. Returns false if a wait gave up.
+template <int DIMS, bool BATCH, uint32_t CAP, int NARR, bool SPLIT>
 __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, const float4* __restrict__ a0,
                                               const float4* __restrict__ a1, const uint2* __restrict__ table,
                                               const uint32_t* __restrict__ bricks, uint32_t n_bricks, uint32_t* queue,
@@ -1065,6 +1071,21 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
     // few bricks is spared a trip to the queue, and the brick is read beside their number
     // (`bricks` has a word per particle). 16,384 particles in 2D: a step 29.6 -> 25.5 us.
     uint32_t b = blockIdx.x, bid = ld_relaxed_gpu(bricks + min(b, kp.n - 1u));
+    bool slow = false;  // SPLIT: units that are not staged are handed over now
+    // Ends the units (of one kind).
+    auto end = [&](bool more) -> bool {
+        if (!acquire()) {
+            cp_async_wait_all();
+            return false;
+        }
+        if (lane == 0) {
+            S.unit[fill & 1u].ncell = 0;
+            S.unit[fill & 1u].more = more;
+        }
+        __syncwarp();
+        hand_over();
+        return true;
+    };
     while (b < n_bricks) {
         uint32_t nb = 0;  // the next brick's ticket, asked for early
         if (lane == 0) nb = gridDim.x + atomicAdd(queue, 1u);
@@ -1096,8 +1117,8 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
 #pragma unroll
         for (int r = 0; r < R; ++r) tot += cn[r];
         if (bad) atomicOr(err, DEV_ERR_KEY_RANGE);
-        nb = __shfl_sync(0xffffffffu, nb, 0);
-        const uint32_t nbid = nb < n_bricks ? bricks[nb] : 0u;
+        b = __shfl_sync(0xffffffffu, nb, 0);
+        bid = b < n_bricks ? bricks[b] : 0u;
         uint32_t incl = tot;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1105,6 +1126,7 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
             if (lane >= o) incl += v;
         }
         const uint32_t excl = incl - tot, incl_next = __shfl_down_sync(0xffffffffu, incl, 1);
+        bool other = false, again = false;  // there are units of the other kind; it is their turn
         for (int c0 = 0; c0 < ncell;) {
             // targets: columns c0 + 1 .. c1, the most that fit the staging with their neighbours
             const uint32_t e0 = __shfl_sync(0xffffffffu, excl, c0);
@@ -1113,7 +1135,9 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
             const int c1 = fits ? 31 - __clz((int)fits) : c0 + 1;
             const uint32_t mine = lane > c0 && lane <= c1 ? cn[RC] : 0u;
             const uint32_t some = __ballot_sync(0xffffffffu, mine != 0u);
-            if (some) {
+            const bool turn = !SPLIT || (fits == 0u) == slow;
+            if (some && !turn) other = true;
+            if (some && turn) {
                 uint32_t pairs = (mine + 1u) >> 1;  // inclusive count of the pairs up to this column
                 const uint32_t own = pairs;
 #pragma unroll
@@ -1188,17 +1212,15 @@ __device__ __forceinline__ bool brick_produce(BrickShared& S, float4* s_buf, con
                 hand_over();
             }
             c0 = c1;
+            if (SPLIT && c0 >= ncell && other && !again) {
+                if (!end(true)) return false;
+                slow = !slow;
+                again = true;
+                c0 = 0;
+            }
         }
-        b = nb;
-        bid = nbid;
     }
-    if (!acquire()) {
-        cp_async_wait_all();
-        return false;
-    }
-    if (lane == 0) S.unit[fill & 1u].ncell = 0;
-    __syncwarp();
-    hand_over();
+    if (!end(false)) return false;
     cp_async_wait_all();
     return true;
 }
@@ -1212,6 +1234,23 @@ __device__ __forceinline__ bool unit_wait(BrickShared& S, uint32_t use, uint32_t
 __device__ __forceinline__ void unit_release(BrickShared& S, uint32_t use) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(reinterpret_cast<uint64_t*>(&S.empty[use & 1u]));
+}
+
+// What ends a consumer's loop over the units of one kind.
+constexpr int UNITS_DONE = 0, UNITS_MORE = 1, UNITS_GAVE_UP = 2;
+__device__ __forceinline__ int units_end(BrickShared& S, uint32_t& use) {
+    const int more = S.unit[use & 1u].more;
+    unit_release(S, use++);
+    return more ? UNITS_MORE : UNITS_DONE;
+}
+// The staged units, then those that are not, and so on while there are more. Returns false if a wait gave up.
+template <class F>
+__device__ __forceinline__ bool both_kinds(F&& units) {
+    for (;;) {
+        int r = units(std::true_type());
+        if (r == UNITS_MORE) r = units(std::false_type());
+        if (r != UNITS_MORE) return r == UNITS_DONE;
+    }
 }
 
 // min(r^2 - h^2, 0) of a candidate: its sign bit says whether the candidate is in range (a NaN
@@ -1293,7 +1332,7 @@ __device__ __forceinline__ bool density_brick_run(float4* s_buf, BrickShared& S,
     brick_init(S);
     const uint32_t n_bricks = __ldcg(counters);  // written by the bounds pass (an earlier kernel or phase)
     if (warp == consumers) {
-        const bool ok = brick_produce<DIMS, BATCH, DENSITY_CAP, 1>(S, s_buf, spos, nullptr, table, bricks, n_bricks,
+        const bool ok = brick_produce<DIMS, BATCH, DENSITY_CAP, 1, false>(S, s_buf, spos, nullptr, table, bricks, n_bricks,
                                                                    &counters[1], kp, err);
         if (!ok) atomicExch(&counters[3], 1u);
         return ok;
@@ -1557,47 +1596,6 @@ __device__ __forceinline__ void pair_finish(const KParams& kp, const BrickUnit& 
     }
 }
 
-// A warp's task in a unit that is not staged: a pair's lanes take every fourth candidate of the cells in
-// global memory, with correctly rounded reciprocals of the densities (the staged tasks use the
-// hardware's, which differ by one unit in the last place for one density in eight). Out of line and with few
-// arguments, so that the staged tasks keep their registers and spill nothing: 1,048,576 particles
-// 152 us, 149 without this code, 159 with it in line; 48 scenes a step 787, 802 and 822. `what`: the target's
-// column, 8: two targets, 16: live.
-template <int DIMS, bool FUSED, bool COH>
-__device__ __noinline__ void force_unstaged(BrickShared& S, uint32_t use, uint32_t gi, uint32_t what, const float4* __restrict__ spos,
-                                            const float4* __restrict__ svel, const uint32_t* __restrict__ index,
-                                            float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ force,
-                                            const KParams& kp) {
-    constexpr int R = DIMS == 3 ? 9 : 3;
-    const BrickUnit& U = S.unit[use & 1u];
-    PairTask t{};
-    t.gi = gi;
-    t.c = (int)(what & 7u);
-    t.two = (what & 8u) != 0u;
-    t.live = (what & 16u) != 0u;
-    const uint32_t lane = threadIdx.x & 31u, l = lane & 3u, two = t.two ? 1u : 0u;
-    const uint32_t thr = max(__float_as_uint(kp.r2_thresh), MIN_NORMAL) - MIN_NORMAL;
-    const PairState st = pair_state<FUSED, COH>(t, l, index, pos, vel, force);
-    const float4 pA = ld_phase<COH>(spos + t.gi), pB = ld_phase<COH>(spos + t.gi + two);
-    const float4 vA = ld_phase<COH>(svel + t.gi), vB = ld_phase<COH>(svel + t.gi + two);
-    const float aA = __frcp_rn(pA.w), aB = __frcp_rn(pB.w);
-    float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
-        if (lane == 0u) atomicAdd(&S.progress, 1u);
-        const uint32_t cnt = U.off[i + 1] - U.off[i], first = U.cell[i].x;
-        for (uint32_t j = l; j < cnt; j += 4u) {
-            const float4 pj = ld_phase<COH>(spos + first + j), vj = ld_phase<COH>(svel + first + j);
-            const float aj = __frcp_rn(pj.w);
-            force_pair<DIMS>(pA, vA, aA, pj, vj, aj, kp.h, thr, accA);
-            force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
-        }
-    }
-    __syncwarp();
-    float f[2][3];
-    pair_sums(kp, U.cvisc, accA, accB, f);
-    pair_finish<DIMS, FUSED>(kp, U, t, l, st, f, pA, pB, vA, vB, pos, vel, force);
-}
-
 // Forces (pressure + viscosity) for every particle of the occupied bricks
 // (clCalculateForces, libCL/phys/oclFluid3D.cl:202-255). A pair's lane l evaluates entries 2 l and
 // 2 l + 1 of each 8-entry chunk of the pair's list for both targets; the lists' first LIST_AHEAD
@@ -1626,92 +1624,120 @@ __device__ __forceinline__ bool force_brick_run(float4* s_buf, BrickShared& S, c
     // pass gave up, which leaves particles without a list
     const uint32_t n_bricks = __ldcg(counters + 3) ? 0u : __ldcg(counters);
     if (warp == consumers)
-        return brick_produce<DIMS, BATCH, FORCE_CAP, 2>(S, s_buf, spos, svel, table, bricks, n_bricks, &counters[2], kp,
+        return brick_produce<DIMS, BATCH, FORCE_CAP, 2, true>(S, s_buf, spos, svel, table, bricks, n_bricks, &counters[2], kp,
                                                         err);
     const uint32_t thr = max(__float_as_uint(kp.r2_thresh), MIN_NORMAL) - MIN_NORMAL;
     int turn = warp;  // tasks of eight pairs are dealt to the consumer warps in turn, across units
-    for (uint32_t use = 0;; ++use) {
-        if (!unit_wait(S, use, err)) return false;
-        const BrickUnit& U = S.unit[use & 1u];
-        if (U.ncell == 0) break;
-        const float4* s_pos = s_buf + (use & 1u) * 2u * FORCE_CAP;
-        const float4* s_vel = s_pos + FORCE_CAP;
-        const bool staged = U.staged != 0;
-        const float cvisc = U.cvisc;
-        const int tasks = (int)((U.npair + TASK_PAIRS - 1u) / TASK_PAIRS);
-        for (; turn < tasks; turn += consumers) {
-            const PairTask t = pair_task<R, RC>(U, (uint32_t)turn * TASK_PAIRS + (lane >> 2));
-            if (!staged) {
-                force_unstaged<DIMS, FUSED, COH>(S, use, t.gi, (uint32_t)t.c | (t.two ? 8u : 0u) | (t.live ? 16u : 0u), spos, svel,
-                                                 index, pos, vel, force, kp);
-                continue;
-            }
-            const uint32_t two = t.two ? 1u : 0u;
-            // everything from global memory at once: the list's length and first chunks (whatever
-            // its length), the targets' particles and, with those known, the lane's part of their state
-            const uint32_t meta = ld_phase<COH>(nbr_meta + t.gi);
-            const PairState st = pair_state<FUSED, COH>(t, l, index, pos, vel, force);
-            const uint32_t* list = reinterpret_cast<const uint32_t*>(nbr) + (size_t)t.gi * (NBR_CAP / 2) + l;
-            uint32_t ch[LIST_AHEAD];
+    uint32_t use = 0;
+    auto units = [&](auto kind) {
+        constexpr bool staged = decltype(kind)::value;
+        for (;; ++use) {
+            if (!unit_wait(S, use, err)) return UNITS_GAVE_UP;
+            const BrickUnit& U = S.unit[use & 1u];
+            if (U.ncell == 0) return units_end(S, use);
+            const float4* s_pos = s_buf + (use & 1u) * 2u * FORCE_CAP;
+            const float4* s_vel = s_pos + FORCE_CAP;
+            const float cvisc = U.cvisc;
+            const int tasks = (int)((U.npair + TASK_PAIRS - 1u) / TASK_PAIRS);
+            for (; turn < tasks; turn += consumers) {
+                const PairTask t = pair_task<R, RC>(U, (uint32_t)turn * TASK_PAIRS + (lane >> 2));
+                const uint32_t two = t.two ? 1u : 0u;
+                if constexpr (staged) {
+                    // everything from global memory at once: the list's length and first chunks (whatever
+                    // its length), the targets' particles and, with those known, the lane's part of their state
+                    const uint32_t meta = ld_phase<COH>(nbr_meta + t.gi);
+                    const PairState st = pair_state<FUSED, COH>(t, l, index, pos, vel, force);
+                    const uint32_t* list = reinterpret_cast<const uint32_t*>(nbr) + (size_t)t.gi * (NBR_CAP / 2) + l;
+                    uint32_t ch[LIST_AHEAD];
 #pragma unroll
-            for (uint32_t k = 0; k < LIST_AHEAD; ++k) ch[k] = ld_phase<COH>(list + 4u * k);
-            const float4 pA = s_pos[t.self], pB = s_pos[t.self + two], vA = s_vel[t.self], vB = s_vel[t.self + two];
-            const float aA = rcp_approx(pA.w), aB = rcp_approx(pB.w);
-            float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            auto both = [&](const float4& pj, const float4& vj) {
-                const float aj = rcp_approx(pj.w);
-                force_pair<DIMS>(pA, vA, aA, pj, vj, aj, kp.h, thr, accA);
-                force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
-            };
-            const bool scan = meta == NBR_SCAN;
-            const uint32_t n = scan ? 0u : meta, win = smem_addr(s_pos + t.lo);
-            auto entry = [&](uint32_t v) { both(lds_f4(win + v), lds_f4(win + v + FORCE_CAP * 16u)); };
-            for (uint32_t k0 = 2u * l; k0 < n; k0 += 8u * LIST_AHEAD) {
-                if (k0 >= 8u * LIST_AHEAD) {
+                    for (uint32_t k = 0; k < LIST_AHEAD; ++k) ch[k] = ld_phase<COH>(list + 4u * k);
+                    const float4 pA = s_pos[t.self], pB = s_pos[t.self + two], vA = s_vel[t.self], vB = s_vel[t.self + two];
+                    const float aA = rcp_approx(pA.w), aB = rcp_approx(pB.w);
+                    float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    auto both = [&](const float4& pj, const float4& vj) {
+                        const float aj = rcp_approx(pj.w);
+                        force_pair<DIMS>(pA, vA, aA, pj, vj, aj, kp.h, thr, accA);
+                        force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
+                    };
+                    const bool scan = meta == NBR_SCAN;
+                    const uint32_t n = scan ? 0u : meta, win = smem_addr(s_pos + t.lo);
+                    auto entry = [&](uint32_t v) { both(lds_f4(win + v), lds_f4(win + v + FORCE_CAP * 16u)); };
+                    for (uint32_t k0 = 2u * l; k0 < n; k0 += 8u * LIST_AHEAD) {
+                        if (k0 >= 8u * LIST_AHEAD) {
 #pragma unroll
-                    for (uint32_t k = 0; k < LIST_AHEAD; ++k)
-                        if (k0 + 8u * k < n) ch[k] = ld_phase<COH>(list + 4u * k + ((k0 >> 3) << 2));
-                }
+                            for (uint32_t k = 0; k < LIST_AHEAD; ++k)
+                                if (k0 + 8u * k < n) ch[k] = ld_phase<COH>(list + 4u * k + ((k0 >> 3) << 2));
+                        }
 #pragma unroll
-                for (uint32_t k = 0; k < LIST_AHEAD; ++k) {
-                    if (k0 + 8u * k >= n) break;
-                    entry(ch[k] & 0xFFFFu);
-                    if (k0 + 8u * k + 1u < n) entry(ch[k] >> 16);
-                }
-            }
-            float f[2][3];
-            pair_sums(kp, cvisc, accA, accB, f);
-            // pairs without a list: the whole warp scans each one's window in turn
-            uint32_t pend = __ballot_sync(0xffffffffu, t.live && scan && l == 0u);
-            while (pend) {
-                const int src = __ffs((int)pend) - 1;
-                pend &= pend - 1u;
-                const uint32_t self = __shfl_sync(0xffffffffu, t.self, src), lo = __shfl_sync(0xffffffffu, t.lo, src),
-                               len = __shfl_sync(0xffffffffu, t.len, src), more = __shfl_sync(0xffffffffu, two, src);
-#pragma unroll 1
-                for (uint32_t w = 0; w <= more; ++w) {
-                    const float4 ps = s_pos[self + w], vs = s_vel[self + w];
-                    const float as = rcp_approx(ps.w);
-                    float a[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                    for (uint32_t j = lo + lane; j < lo + len; j += 32u)
-                        force_pair<DIMS>(ps, vs, as, s_pos[j], s_vel[j], rcp_approx(s_pos[j].w), kp.h, thr, a);
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        float x = fmaf(kp.cpress, a[k], cvisc * a[3 + k]);
-                        for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
-                        if ((lane >> 2) == (uint32_t)src >> 2) {
-                            if (w) f[1][k] = x;
-                            else f[0][k] = x;
+                        for (uint32_t k = 0; k < LIST_AHEAD; ++k) {
+                            if (k0 + 8u * k >= n) break;
+                            entry(ch[k] & 0xFFFFu);
+                            if (k0 + 8u * k + 1u < n) entry(ch[k] >> 16);
                         }
                     }
+                    float f[2][3];
+                    pair_sums(kp, cvisc, accA, accB, f);
+                    // pairs without a list: the whole warp scans each one's window in turn
+                    uint32_t pend = __ballot_sync(0xffffffffu, t.live && scan && l == 0u);
+                    while (pend) {
+                        const int src = __ffs((int)pend) - 1;
+                        pend &= pend - 1u;
+                        const uint32_t self = __shfl_sync(0xffffffffu, t.self, src), lo = __shfl_sync(0xffffffffu, t.lo, src),
+                                       len = __shfl_sync(0xffffffffu, t.len, src), more = __shfl_sync(0xffffffffu, two, src);
+#pragma unroll 1
+                        for (uint32_t w = 0; w <= more; ++w) {
+                            const float4 ps = s_pos[self + w], vs = s_vel[self + w];
+                            const float as = rcp_approx(ps.w);
+                            float a[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                            for (uint32_t j = lo + lane; j < lo + len; j += 32u)
+                                force_pair<DIMS>(ps, vs, as, s_pos[j], s_vel[j], rcp_approx(s_pos[j].w), kp.h, thr, a);
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) {
+                                float x = fmaf(kp.cpress, a[k], cvisc * a[3 + k]);
+                                for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+                                if ((lane >> 2) == (uint32_t)src >> 2) {
+                                    if (w) f[1][k] = x;
+                                    else f[0][k] = x;
+                                }
+                            }
+                        }
+                    }
+                    pair_finish<DIMS, FUSED>(kp, U, t, l, st, f, pA, pB, vA, vB, pos, vel, force);
+                } else {
+                    // with correctly rounded reciprocals of the densities (the staged targets take the
+                    // hardware's, one unit in the last place off for one density in eight)
+                    const PairState st = pair_state<FUSED, COH>(t, l, index, pos, vel, force);
+                    const float4 pA = ld_phase<COH>(spos + t.gi), pB = ld_phase<COH>(spos + t.gi + two);
+                    const float4 vA = ld_phase<COH>(svel + t.gi), vB = ld_phase<COH>(svel + t.gi + two);
+                    const float aA = __frcp_rn(pA.w), aB = __frcp_rn(pB.w);
+                    float accA[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, accB[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    for (int i = t.c * R; i < (t.c + 3) * R; ++i) {
+                        if (lane == 0u) atomicAdd(&S.progress, 1u);
+                        const uint32_t cnt = U.off[i + 1] - U.off[i], first = U.cell[i].x;
+                        if (l >= cnt) continue;
+                        float4 pn = ld_phase<COH>(spos + first + l), vn = ld_phase<COH>(svel + first + l);  // loaded a candidate ahead
+                        for (uint32_t j = l; j < cnt; j += 4u) {
+                            const float4 pj = pn, vj = vn;
+                            if (j + 4u < cnt) {
+                                pn = ld_phase<COH>(spos + first + j + 4u);
+                                vn = ld_phase<COH>(svel + first + j + 4u);
+                            }
+                            const float aj = __frcp_rn(pj.w);
+                            force_pair<DIMS>(pA, vA, aA, pj, vj, aj, kp.h, thr, accA);
+                            force_pair<DIMS>(pB, vB, aB, pj, vj, aj, kp.h, thr, accB);
+                        }
+                    }
+                    __syncwarp();
+                    float f[2][3];
+                    pair_sums(kp, cvisc, accA, accB, f);
+                    pair_finish<DIMS, FUSED>(kp, U, t, l, st, f, pA, pB, vA, vB, pos, vel, force);
                 }
             }
-            pair_finish<DIMS, FUSED>(kp, U, t, l, st, f, pA, pB, vA, vB, pos, vel, force);
+            turn -= tasks;
+            unit_release(S, use);
         }
-        turn -= tasks;
-        unit_release(S, use);
-    }
-    return true;
+    };
+    return both_kinds(units);
 }
 
 template <int DIMS, bool FUSED, bool BATCH>
@@ -1723,7 +1749,7 @@ __global__ void __launch_bounds__(32 * FORCE_CONSUMERS + 32, FORCE_CTAS) k_force
                                                                float4* __restrict__ force,
                                                                const uint2* __restrict__ table,
                                                                const uint32_t* __restrict__ bricks,
-                                                               uint32_t* counters, const __grid_constant__ KParams kp,
+                                                               uint32_t* counters, KParams kp,
                                                                const uint16_t* __restrict__ nbr,
                                                                const uint32_t* __restrict__ nbr_meta,
                                                                uint32_t* err) {
