@@ -945,7 +945,7 @@ static __global__ void k_emitter(float4* __restrict__ pos, float4* __restrict__ 
 // lists appended per candidate), forces 149 us (184 us with two lanes per target and the lists
 // staged). Density is bound by instruction issue (77% of cycles; 63 of the 137 us are the
 // candidate loop at 21 instructions for 64 pairs, 20 the lists, 16 the staging), forces by issue
-// and the LSU pipe's wavefronts (57% and 66%).
+// and the LSU pipe's wavefronts (59% and 68%).
 // Tried: a bulk copy per cell instead of the 16-byte asynchronous copies (170 / 260 us: the
 // small copies queue), two producers, one per buffer (139 / 178), 3 to 7 consumers at 3 to 6
 // CTAs per SM (density 133-137, forces 150-172).
