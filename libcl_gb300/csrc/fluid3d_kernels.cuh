@@ -930,7 +930,7 @@ static __global__ void k_emitter(float4* __restrict__ pos, float4* __restrict__ 
 // and the row loop around them cost as many instructions as the candidates themselves.
 //
 // A consumer waits for copies and for a task at most; the producer waits for whole units, and a unit
-// that is not staged may take long (8,000 particles in one cell: 64 ms for both passes; 60,000:
+// that is not staged may take long (8,000 particles in one cell: 57 ms for both passes; 60,000:
 // seconds). So consumers count the cells that they read from global memory in S.progress, and
 // the producer gives up only after a second in which nothing moved.
 //
